@@ -6,6 +6,7 @@
     run(state)        one pass through the public entry points; returns its outputs
     work(case)        bytes and flops one pass cannot do without
     tolerance(case)   how far another correct implementation may be off
+    exact(case, s)    the same outputs in plain torch and 64 bits
 
 Five kinds of work, each through the entry point a program calls:
 
@@ -23,6 +24,8 @@ router logits N(0, 1), router weights N(0, 0.02): the distributions of the bench
 from __future__ import annotations
 
 import ctypes as C
+import re
+from pathlib import Path
 
 import numpy as np
 import torch
@@ -169,21 +172,28 @@ def _experts(c, gen):
     return t
 
 
+def _table_inputs(c, gen):
+    """The resident arrays of one layer (with its envelope when there are several streams) and the input rows."""
+    t, S, H = _experts(c, gen), c["streams"], c["hidden"]
+    randn = lambda *shape: torch.randn(shape, device="cuda", generator=gen)  # noqa: E731
+    if S > 1:
+        t["mhc_fn"] = randn((S + 2) * S, S * H) * 0.05
+        t["mhc_scale"] = torch.tensor([0.7, 1.3, 0.9], device="cuda")
+        t["mhc_base"] = randn((S + 2) * S) * 0.3
+        t["ffn_norm"] = 1.0 + 0.1 * randn(H)
+    return t, randn(c["tokens"], S * H)
+
+
 class _Table:
     """A backend session as a runtime holds it: resident arena, attached workspace, one layer job, page-locked host rows."""
 
     def __init__(self, c, gen):
         from yvex_b200 import backend as B
         self.B, T, H, S, k = B, c["tokens"], c["hidden"], c["streams"], c["topk"]
-        arrays = {n: v.cpu().numpy() for n, v in _experts(c, gen).items()}
-        if S > 1:
-            rows = (S + 2) * S
-            arrays["mhc_fn"] = (torch.randn((rows, S * H), device="cuda", generator=gen) * 0.05).cpu().numpy()
-            arrays["mhc_scale"] = np.array([0.7, 1.3, 0.9], np.float32)
-            arrays["mhc_base"] = (torch.randn(rows, device="cuda", generator=gen) * 0.3).cpu().numpy()
-            arrays["ffn_norm"] = (1.0 + 0.1 * torch.randn(H, device="cuda", generator=gen)).cpu().numpy()
+        tensors, rows = _table_inputs(c, gen)
+        arrays = {n: v.cpu().numpy() for n, v in tensors.items()}
         self.rows_in = torch.empty((T, S * H), dtype=torch.float32).pin_memory()
-        self.rows_in.copy_(torch.randn((T, S * H), device="cuda", generator=gen))
+        self.rows_in.copy_(rows)
         self.rows_out = torch.empty((T, S * H), dtype=torch.float32).pin_memory()
         self.selected, self.weights = np.zeros((T, k), np.uint64), np.zeros((T, k), np.float32)
         self.be = B.Backend()
@@ -299,3 +309,140 @@ def tolerance(case):
     if case["kind"] == "attention":
         return {"rel": 8e-6, "max": 4e-5}
     return {"rel": 1e-3, "max": 0.05}
+
+
+# ---- the same outputs in 64 bits ------------------------------------------------------------------------------------------
+# Plain torch over the block layouts of the GGUF format; sums and products in 64 bits, rounded where the layer is specified
+# to round (bf16 of the ingress rows, of the SwiGLU products, of each expert's result and of the layer's; f32 of a projection).
+
+def _codebook():
+    """The IQ2_XXS magnitudes [256, 8], from the table of nibbles (digit 0, 1, 2 = 8, 25, 43) that the format fixes."""
+    text = (Path(__file__).resolve().parent.parent / "yvex_b200" / "csrc" / "iq2xxs_grid_nibbles.inc").read_text()
+    words = [int(v, 16) for v in re.findall(r"0x([0-9a-f]{8})u", text)]
+    digits = torch.tensor([[(w >> (4 * i)) & 3 for i in range(8)] for w in words], device="cuda")
+    return torch.tensor([8.0, 25.0, 43.0], dtype=torch.float64, device="cuda")[digits]
+
+
+def _f16(b):
+    return b.contiguous().view(torch.float16).double()
+
+
+def _decoded(name, raw, rows, width):
+    """Encoded rows as [rows, width] in 64 bits."""
+    raw = raw.reshape(rows, -1)
+    if name in ("F32", "F16", "BF16"):
+        return raw.view({"F32": torch.float32, "F16": torch.float16, "BF16": torch.bfloat16}[name]).double()
+    b = raw.reshape(-1, {"IQ2_XXS": 66, "Q2_K": 84, "Q4_K": 144, "Q8_0": 34, "MXFP4": 17}[name])
+    if name == "Q8_0":
+        w = _f16(b[:, :2]) * b[:, 2:].contiguous().view(torch.int8).double()
+    elif name == "MXFP4":
+        levels = torch.tensor([0, 1, 2, 3, 4, 6, 8, 12, 0, -1, -2, -3, -4, -6, -8, -12], dtype=torch.float64, device=b.device)
+        codes = torch.cat((b[:, 1:] & 15, b[:, 1:] >> 4), 1).long()
+        w = levels[codes] * torch.exp2(b[:, :1].double() - 128.0)
+    elif name == "IQ2_XXS":
+        groups = b[:, 2:].reshape(-1, 8, 8)
+        bits = groups[:, :, 4:].contiguous().view(torch.int32).long().squeeze(-1) & 0xffffffff              # [n, 8]
+        low = (bits[:, :, None] >> (7 * torch.arange(4, device=b.device))) & 127                            # [n, 8, 4]
+        sign = (low[..., None] >> torch.arange(7, device=b.device)) & 1
+        sign = torch.cat((sign, sign.sum(-1, keepdim=True) & 1), -1)                                        # the eighth makes the parity even
+        scale = _f16(b[:, :2]) * 0.25 * (0.5 + (bits >> 28).double())                                       # [n, 8]
+        w = scale[:, :, None, None] * _codebook()[groups[:, :, :4].long()] * (1.0 - 2.0 * sign)
+    elif name == "Q2_K":
+        planes = b[:, 16:80].reshape(-1, 2, 1, 32) >> (2 * torch.arange(4, device=b.device, dtype=torch.uint8))[:, None]
+        code = (planes & 3).reshape(-1, 16, 16).double()
+        w = _f16(b[:, 80:82])[..., None] * (b[:, :16] & 15).double()[..., None] * code - _f16(b[:, 82:])[..., None] * (b[:, :16] >> 4).double()[..., None]
+    else:
+        s = b[:, 4:16].long()
+        scale = torch.cat((s[:, :4] & 63, (s[:, 8:] & 15) | (s[:, :4] >> 6 << 4)), 1).double()[..., None]
+        least = torch.cat((s[:, 4:8] & 63, (s[:, 8:] >> 4) | (s[:, 4:8] >> 6 << 4)), 1).double()[..., None]
+        q = b[:, 16:].reshape(-1, 4, 32)
+        w = _f16(b[:, :2])[..., None] * scale * torch.stack((q & 15, q >> 4), 2).reshape(-1, 8, 32).double() - _f16(b[:, 2:4])[..., None] * least
+    return w.reshape(rows, width)
+
+
+def _bf16(v):
+    return v.float().to(torch.bfloat16).double()
+
+
+def _exact_layer(c, t, x, logits):
+    """The layer on 64-bit rows: (result rows, selections, their weights)."""
+    H, I, k = c["hidden"], c["inter"], c["topk"]
+    spec = _spec(c)
+    x = _bf16(x)
+    logits = (x @ t["router"].double().T).float().double() if logits is None else logits.double()
+    score = torch.nn.functional.softplus(logits, threshold=700.0).sqrt().float()
+    selected = torch.sort(score, dim=1, descending=True, stable=True)[1][:, :k]
+    weight = score.gather(1, selected).double()
+    weight = weight / weight.sum(1, keepdim=True) * spec.scaling
+
+    def expert(parts, rows, w):
+        gate, up, down = (_decoded(c[q], p, n, m) for q, p, n, m in zip(("gate", "gate", "down"), parts, (I, I, H), (H, H, I)))
+        g, u = (x[rows] @ gate.T).clamp(max=spec.limit), (x[rows] @ up.T).clamp(-spec.limit, spec.limit)
+        return _bf16(_bf16(g * torch.sigmoid(g) * u * w[:, None]) @ down.T).float()
+
+    every = torch.arange(x.shape[0], device=x.device)
+    pairs = torch.zeros((x.shape[0], k, H), device=x.device)
+    packs = [t[n].reshape(c["experts"], -1) for n in ("gate", "up", "down")]
+    for e in selected.unique().tolist():
+        row, rank = (selected == e).nonzero(as_tuple=True)
+        pairs[row, rank] = expert([p[e] for p in packs], row, weight[row, rank])
+    shared = expert([t["shared_gate"], t["shared_up"], t["shared_down"]], every, torch.ones_like(weight[:, 0]))
+    out = shared.double()
+    for r in range(k):
+        out += pairs[:, r]
+    return _bf16(out), selected, weight
+
+
+def _exact_table(c, gen):
+    t, rows = _table_inputs(c, gen)
+    S, H, eps = c["streams"], c["hidden"], 1e-6
+    x = rows.double()
+    if S == 1:
+        return _exact_layer(c, t, x, None)
+    scale, base = t["mhc_scale"].double(), t["mhc_base"].double()
+    mix = (x @ t["mhc_fn"].double().T) / (x.square().mean(1, keepdim=True) + eps).sqrt()
+    pre = torch.sigmoid(mix[:, :S] * scale[0] + base[:S]) + eps
+    post = 2.0 * torch.sigmoid(mix[:, S:2 * S] * scale[1] + base[S:2 * S])
+    comb = torch.softmax((mix[:, 2 * S:] * scale[2] + base[2 * S:]).reshape(-1, S, S), 2) + eps
+    for n in range(20):
+        if n:
+            comb = comb / (comb.sum(2, keepdim=True) + eps)
+        comb = comb / (comb.sum(1, keepdim=True) + eps)
+    streams = x.reshape(-1, S, H)
+    flat = _bf16((pre[..., None] * streams).sum(1))
+    normed = _bf16(flat / (flat.square().mean(1, keepdim=True) + eps).sqrt() * t["ffn_norm"].double())
+    core, selected, weight = _exact_layer(c, t, normed, None)
+    out = _bf16(post[..., None] * core[:, None] + torch.einsum("nst,nsh->nth", comb, streams))
+    return out.reshape(-1, S * H), selected, weight
+
+
+def exact(case, seed):
+    c = case
+    if c["kind"] == "matvec":
+        s = prepare(c, seed)
+        step = max(1, (1 << 27) // c["width"])                          # rows at a time: a decoded head is several GB
+        cuts = [(a, min(a + step, c["rows"])) for a in range(0, c["rows"], step)]
+        raw = s["weights"].reshape(c["rows"], -1)
+        return torch.cat([s["x"].double() @ _decoded(c["qtype"], raw[a:b].contiguous(), b - a, c["width"]).T for a, b in cuts], 1)
+    if c["kind"] == "batch":
+        s = prepare(c, seed)
+        raw = s["weights"].reshape(c["count"], -1)
+        return torch.stack([_decoded(c["qtype"], raw[m], c["rows"], c["width"]) @ s["x"][m].double() for m in range(c["count"])])
+    if c["kind"] == "table":
+        out, selected, weight = _exact_table(c, _generator(seed))
+        return dict(rows=out.cpu(), selected=selected.cpu().numpy().astype(np.uint64), weights=weight.cpu().numpy())
+    if c["kind"] == "attention":
+        s, V, group = prepare(c, seed), c["visible"], c["q_heads"] // c["kv_heads"]
+        out = torch.empty((c["sessions"], c["q_heads"], c["dim"]), dtype=torch.float64, device="cuda")
+        for n in range(c["sessions"]):
+            for h in range(c["kv_heads"]):
+                q = s["q"][n, h * group:(h + 1) * group].double()
+                p = torch.softmax(q @ s["k"][n, h, :V].double().T * c["dim"] ** -0.5, 1)
+                out[n, h * group:(h + 1) * group] = p @ s["v"][n, h, :V].double()
+        return out
+    gen = _generator(seed)
+    t, T = _experts(c, gen), c["tokens"]
+    x = torch.randn((T, c["hidden"]), device="cuda", generator=gen)
+    logits = torch.randn((T, c["experts"]), device="cuda", generator=gen) if c["router"] == "logits" else None
+    out, selected, weight = _exact_layer(c, t, x.double(), logits)
+    return out, selected.int(), weight
