@@ -111,3 +111,25 @@ def test_envelope_refusals(L):
     L.mhc_prepare(ok, dev(bad), st)
     torch.cuda.synchronize()
     assert st.read() == 1
+
+
+@pytest.mark.parametrize("streams", [2, 3, 5, 6])
+def test_mhc_gates_and_combination_at_every_stream_count(L, streams):
+    """One lane per stream pair: 4 to 25 pairs fit a warp once, 36 take a second turn. Gates and combination are doubles
+    rounded to f32 in the same order on both sides: 1e-6, as above."""
+    from oracle_lib import Port
+    port, rng = Port(), np.random.default_rng(streams)
+    H, T, rows = 256, 3, (streams + 2) * streams
+    fn = rng.normal(0, 0.05, (rows, streams * H)).astype(np.float32)
+    scale, base = np.array([0.7, 1.3, 0.9], np.float32), rng.normal(0, 0.3, rows).astype(np.float32)
+    norm, x = rng.normal(1, 0.1, H).astype(np.float32), rng.normal(0, 1, (T, streams * H)).astype(np.float32)
+    m, st = L.mhc_of(H, streams, dev(fn), dev(scale), dev(base), dev(norm), **ENVELOPE_POLICY), L.Status()
+    normalized, post, comb = L.mhc_prepare(m, dev(x), st)
+    assert st.read() == 0
+    oracle = port.mhc(H, streams, fn, scale, base, norm, **ENVELOPE_POLICY)
+    for t in range(T):
+        rc, want_norm, want_post, want_comb = port.mhc_prepare(oracle, x[t])
+        assert rc == 0
+        assert np.allclose(post[t].cpu().numpy().ravel(), np.ravel(want_post), rtol=1e-6, atol=0)
+        assert np.allclose(comb[t].cpu().numpy().ravel(), np.ravel(want_comb), rtol=1e-6, atol=0)
+        assert bf16_close(normalized[t].cpu().numpy(), want_norm)

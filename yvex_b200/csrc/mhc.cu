@@ -10,16 +10,17 @@
 //   collapsed = sum_s (float)((pre[s]+eps) * x[s]) in stream order (f32 adds), bf16 round   :810-815
 //   normalized = bf16( collapsed * 1/sqrt(mean(collapsed^2)+rms_eps) * norm )   numeric.c:630-659, moe.c:487-489
 //   post:  out[t] = bf16( (float)(post[t]*core + sum_s comb[s][t]*x[s]) ), double   numeric.c:855-868
-// Launches: one CTA per (mix row, token row) for the dots (plus one per token row for the sum of
+// Launches: one CTA (512 threads: two rounds of loads at 4 x 4096; 128 took 14.5 us, this 7.5) per (mix row, token row) for the dots (plus one per token row for the sum of
 // squares), one CTA per token row for gates + Sinkhorn + collapse + RMSNorm, an elementwise kernel
 // for post.
 #include "common.cuh"
 
 namespace yb {
 
-constexpr int kMhcThreads = 128;
+constexpr int kMhcThreads = 512;
 constexpr int kMhcRowThreads = 1024;
 constexpr int kMhcMaxStreams = 6;            // (streams + 2) * streams <= 64 mixing rows (src/graph/moe.c:455)
+constexpr int kMhcPerLane = (kMhcMaxStreams * kMhcMaxStreams + 31) / 32;      // stream pairs a lane normalises
 constexpr int kMhcMaxPerThread = 16;         // hidden <= 16384 (src/graph/moe.c:456)
 
 __device__ __forceinline__ double block_sum(double v, double *scratch) {
@@ -85,58 +86,84 @@ __device__ __forceinline__ double sigmoid_d(double v) {
 __global__ void __launch_bounds__(kMhcRowThreads)
 mhc_collapse_kernel(yvex_b200_mhc m, const float *expanded, const float *mix, const double *squares, float *normalized,
                     float *post, float *combination, int *status) {
-    __shared__ double scratch[kMhcRowThreads / 32];
+    __shared__ double scratch[kMhcMaxStreams * kMhcMaxStreams];      // block sums (one per warp) and the softmax terms
     __shared__ double pre[kMhcMaxStreams];
+    __shared__ float c[kMhcMaxStreams * kMhcMaxStreams];
     __shared__ int failed;
     const uint64_t r = blockIdx.x, H = m.hidden, S = m.streams, W = S * H;
     const int rows = (int)((S + 2) * S);
     const float *x = expanded + r * W;
-    if (threadIdx.x == 0) {
-        failed = 0;
+    if (threadIdx.x < 32) {
+        // One lane per gate or mixing element: the chain of the 20 Sinkhorn rounds is 39 normalisations long whatever the
+        // width, and each is one shared-memory read, S additions and one division deep when every element has its lane
+        // (S = 6: two elements on four of them). Totals run in the same order as a serial loop, so no value changes.
+        // One thread doing all S * S elements in turn measured 125 us, this form 34 us (S = 4, one row of 4 x 4096).
+        const int lane = threadIdx.x, s_count = (int)S, elements = s_count * s_count;
         const float *mx = mix + r * rows;
         const double inv = 1.0 / sqrt(squares[r] / (double)W + m.rms_epsilon);
         bool ok = isfinite(inv);
-        for (int i = 0; i < 3; ++i) ok &= isfinite(m.scale[i]);
-        for (int i = 0; i < rows; ++i) ok &= isfinite(m.base[i]);
-        float c[kMhcMaxStreams * kMhcMaxStreams];
-        for (uint64_t s = 0; s < S; ++s) {
-            pre[s] = sigmoid_d((double)mx[s] * inv * (double)m.scale[0] + (double)m.base[s]);
-            post[r * S + s] = (float)(m.post_multiplier * sigmoid_d((double)mx[S + s] * inv * (double)m.scale[1] + (double)m.base[S + s]));
-            for (uint64_t t = 0; t < S; ++t) {
-                const uint64_t idx = 2 * S + s * S + t;
-                c[s * S + t] = (float)((double)mx[idx] * inv * (double)m.scale[2] + (double)m.base[idx]);
+        if (lane < 3) ok &= isfinite(m.scale[lane]) != 0;
+        for (int i = lane; i < rows; i += 32) {
+            ok &= isfinite(m.base[i]) != 0;
+            const double z = (double)mx[i] * inv * (double)m.scale[i < s_count ? 0 : i < 2 * s_count ? 1 : 2] + (double)m.base[i];
+            if (i < s_count) pre[i] = sigmoid_d(z);
+            else if (i < 2 * s_count) post[r * S + i - s_count] = (float)(m.post_multiplier * sigmoid_d(z));
+            else c[i - 2 * s_count] = (float)z;
+        }
+        __syncwarp();
+        // Sinkhorn normalisation of the stream combination (src/graph/numeric.c:706-750): row softmax + eps first, then
+        // rounds of columns and rows. Every lane reads its row or column total before any lane overwrites an element.
+        float mine[kMhcPerLane];
+        double denominator[kMhcPerLane];
+#pragma unroll
+        for (int j = 0; j < kMhcPerLane; ++j) {
+            const int e = lane + 32 * j, row = e / s_count;
+            mine[j] = 0.0f; denominator[j] = 1.0;
+            if (e < elements) {
+                double mxv = -(double)INFINITY;
+                for (int col = 0; col < s_count; ++col) mxv = fmax(mxv, (double)c[row * s_count + col]);
+                denominator[j] = exp((double)c[e] - mxv);
+                mine[j] = (float)denominator[j];
             }
         }
-        // Sinkhorn normalisation of the stream combination (src/graph/numeric.c:706-750)
-        for (uint64_t row = 0; row < S && ok; ++row) {
-            double mxv = -(double)INFINITY, total = 0.0;
-            for (uint64_t col = 0; col < S; ++col) mxv = fmax(mxv, (double)c[row * S + col]);
-            for (uint64_t col = 0; col < S; ++col) {
-                const double v = exp((double)c[row * S + col] - mxv);
-                c[row * S + col] = (float)v;
-                total += v;
-            }
+        __syncwarp();
+        double *terms = scratch;                                 // the row's unrounded exponentials, S * S <= 36 of them
+#pragma unroll
+        for (int j = 0; j < kMhcPerLane; ++j) if (lane + 32 * j < elements) terms[lane + 32 * j] = denominator[j];
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < kMhcPerLane; ++j) {
+            const int e = lane + 32 * j, row = e / s_count;
+            if (e >= elements) continue;
+            double total = 0.0;
+            for (int col = 0; col < s_count; ++col) total += terms[row * s_count + col];
             ok &= isfinite(total) && total > 0.0;
-            for (uint64_t col = 0; col < S; ++col) c[row * S + col] = (float)((double)c[row * S + col] / total + m.mhc_epsilon);
+            c[e] = (float)((double)mine[j] / total + m.mhc_epsilon);
         }
-        for (uint64_t it = 0; it < m.sinkhorn_iterations && ok; ++it) {
-            if (it != 0) {
-                for (uint64_t row = 0; row < S; ++row) {
-                    double total = 0.0;
-                    for (uint64_t col = 0; col < S; ++col) total += c[row * S + col];
-                    ok &= isfinite(total);
-                    for (uint64_t col = 0; col < S; ++col) c[row * S + col] = (float)((double)c[row * S + col] / (total + m.mhc_epsilon));
-                }
-            }
-            for (uint64_t col = 0; col < S; ++col) {
+        __syncwarp();
+        auto normalise = [&](bool by_row) {
+#pragma unroll
+            for (int j = 0; j < kMhcPerLane; ++j) {
+                const int e = lane + 32 * j, at = by_row ? (e / s_count) * s_count : e % s_count, step = by_row ? 1 : s_count;
+                if (e >= elements) continue;
                 double total = 0.0;
-                for (uint64_t row = 0; row < S; ++row) total += c[row * S + col];
-                ok &= isfinite(total);
-                for (uint64_t row = 0; row < S; ++row) c[row * S + col] = (float)((double)c[row * S + col] / (total + m.mhc_epsilon));
+                for (int i = 0; i < s_count; ++i) total += c[at + i * step];
+                ok &= isfinite(total) != 0;
+                mine[j] = (float)((double)c[e] / (total + m.mhc_epsilon));
             }
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < kMhcPerLane; ++j) if (lane + 32 * j < elements) c[lane + 32 * j] = mine[j];
+            __syncwarp();
+        };
+        // (a row that has failed leaves the rounds: its launch is refused)
+        for (uint64_t it = 0; it < m.sinkhorn_iterations && __all_sync(0xffffffffu, ok); ++it) {
+            if (it != 0) normalise(true);
+            normalise(false);
         }
-        for (uint64_t i = 0; i < S * S; ++i) combination[r * S * S + i] = c[i];
-        if (!ok) failed = 1;
+        for (int e = lane; e < elements; e += 32) combination[r * S * S + e] = c[e];
+        ok = __all_sync(0xffffffffu, ok) != 0;
+        if (lane == 0) failed = !ok;
     }
     __syncthreads();
     if (failed) { if (threadIdx.x == 0) raise(status, YVEX_B200_STATUS_NUMERIC); return; }
