@@ -491,3 +491,27 @@ def test_sink_attention_reducer_vs_restatement(L, heads, n, D):
         bad[0, 1] = np.inf
         L.attention_sink(dev(bad), dev(rows), dev(sinks), scale, st)
         assert st.read() == 1
+
+
+@pytest.mark.parametrize("dim,group,sessions,kv,visible,context", [(64, 1, 1, 1, 1, 16), (64, 4, 3, 2, 63, 64), (128, 2, 2, 2, 65, 300),
+                                                                   (128, 4, 1, 8, 1500, 4096), (256, 4, 1, 1, 4097, 4100),
+                                                                   (256, 1, 2, 3, 129, 129), (128, 1, 40, 16, 700, 701)])
+def test_gqa_decode_slices_and_block_edges(L, dim, group, sessions, kv, visible, context):
+    """One key, slices shorter than a block, slices that stay empty, every group and width: against the
+    same contraction in 64 bits. Probabilities carry 16 bits (hi + lo bf16) and sums are f32: 1e-5. The context is larger
+    than what is visible, what lies behind it is NaN, and a workspace made for the context serves the prefix."""
+    import torch
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(dim + visible)
+    q = torch.randn((sessions, kv * group, dim), device="cuda", generator=gen).to(torch.bfloat16)
+    k, v = (torch.randn((sessions, kv, context, dim), device="cuda", generator=gen).to(torch.bfloat16) for _ in range(2))
+    k[:, :, visible:], v[:, :, visible:] = float("nan"), float("nan")
+    ws = torch.empty(int(L.lib.yvex_b200_attention_workspace_bytes(sessions, kv * group, kv, dim, context)), dtype=torch.uint8, device="cuda")
+    st = L.Status()
+    out = L.attention_gqa_decode(q, k, v, visible - 1, dim ** -0.5, st, workspace=ws)
+    assert st.read() == 0
+    scores = torch.einsum("skgd,skcd->skgc", q.double().reshape(sessions, kv, group, dim), k[:, :, :visible].double()) * dim ** -0.5
+    want = torch.einsum("skgc,skcd->skgd", torch.softmax(scores, -1), v[:, :, :visible].double()).reshape(out.shape)
+    assert rel_l2(out.cpu().numpy(), want.cpu().numpy()) <= 1e-5
+    need = [int(L.lib.yvex_b200_attention_workspace_bytes(sessions, kv * group, kv, dim, c)) for c in range(1, context + 1)]
+    assert all(a <= b for a, b in zip(need, need[1:]))
