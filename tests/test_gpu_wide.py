@@ -295,3 +295,18 @@ def test_ep_dispatch_matches_the_tensor_formulation(L, world, tokens, topk, expe
     L.ep_dispatch(xh, bad, wts, per_rank, world, st)
     torch.cuda.synchronize()
     assert st.read() == 2
+
+
+@pytest.mark.parametrize("rows,experts,hidden", [(1, 4, 256), (7, 9, 260), (9, 8, 1024), (17, 256, 512), (333, 64, 4096), (1201, 72, 256),
+                                                 (5, 6, 258)])
+def test_router_projection_tiles(L, rows, experts, hidden):
+    """8 x 8 tiles with ragged ends, rows split over four warps or not (from 1184 tiles on), and the width that takes the
+    dot-by-dot kernel. Sums are doubles in another order than numpy's and rounded once: one f32 step."""
+    rng = np.random.default_rng(rows)
+    x, router = rng.normal(size=(rows, hidden)).astype(np.float32), rng.normal(0, 0.02, (experts, hidden)).astype(np.float32)
+    spec = synth.MoELayerSpec(hidden, experts, min(4, experts), 256)
+    st = L.Status()
+    sel, w, logits = L.moe_route(L.geometry_of(spec), L.weights_of({"router": dev(router)}), st, rows_f32=dev(x))
+    assert st.read() == 0
+    want = x.astype(np.float64) @ router.astype(np.float64).T
+    assert np.allclose(logits.cpu().numpy(), want, rtol=2.0 ** -23, atol=1e-12)

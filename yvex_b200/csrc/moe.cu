@@ -42,6 +42,75 @@ __global__ void router_logits_kernel(const float *router, const float *xr, uint6
     }
 }
 
+// ---- router projection over a prompt: 8 x 8 (row, expert) tiles per warp -----------------------------
+// Bound by the doubles: every product is one DFMA, and the f32 operands of a dot taken on its own would need two
+// conversions per product on a pipe with a quarter of the DFMA rate (router_logits_kernel: 62 us for 333 rows x 64 experts x
+// 4096). A lane converts 8 + 8 values and uses each eight times; lanes run along the row in 16-byte loads, and the 64
+// sums of the 32 lanes are folded by halves (lane l keeps sums 2 l and 2 l + 1). ksplit = 4: the four warps of a CTA take a
+// quarter of the row each - short prompts have too few tiles for the chip - else four neighbouring tiles of the
+// same rows, which then come from L1.
+constexpr int kRouterTile = 8, kRouterTileWarps = 4;
+__global__ void __launch_bounds__(32 * kRouterTileWarps)
+router_tile_kernel(const float *router, const float *xr, uint64_t rows, uint64_t experts, uint64_t hidden, int ksplit, float *logits, int *status) {
+    constexpr int R = kRouterTile;
+    __shared__ double part[kRouterTileWarps][R * R];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t row0 = (uint64_t)blockIdx.x * R, e0 = ((uint64_t)blockIdx.y * (uint64_t)(kRouterTileWarps / ksplit) + (uint64_t)(warp / ksplit)) * R;
+    double acc[R * R];
+#pragma unroll
+    for (int i = 0; i < R * R; ++i) acc[i] = 0.0;
+    const uint64_t vec = hidden / 4, share = (vec + ksplit - 1) / ksplit, v0 = share * (uint64_t)(warp % ksplit), v1 = v0 + share < vec ? v0 + share : vec;
+    if (e0 < experts) {
+        // rows and experts past the end repeat the last one; their sums are not stored
+        const float4 *xb = reinterpret_cast<const float4 *>(xr + row0 * hidden), *wb = reinterpret_cast<const float4 *>(router + e0 * hidden);
+        const uint32_t pitch = (uint32_t)vec, xn = (uint32_t)(rows - row0 < R ? rows - row0 : R) - 1u, wn = (uint32_t)(experts - e0 < R ? experts - e0 : R) - 1u;
+        for (uint64_t v = v0 + lane; v < v1; v += 32) {
+            float4 x4[R], w4[R];
+#pragma unroll
+            for (uint32_t i = 0; i < R; ++i) { x4[i] = __ldg(xb + v + min(i, xn) * pitch); w4[i] = __ldg(wb + v + min(i, wn) * pitch); }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                double w[R];
+#pragma unroll
+                for (int j = 0; j < R; ++j) w[j] = (double)(k == 0 ? w4[j].x : k == 1 ? w4[j].y : k == 2 ? w4[j].z : w4[j].w);
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    const double x = (double)(k == 0 ? x4[i].x : k == 1 ? x4[i].y : k == 2 ? x4[i].z : x4[i].w);
+#pragma unroll
+                    for (int j = 0; j < R; ++j) acc[i * R + j] = fma(x, w[j], acc[i * R + j]);
+                }
+            }
+        }
+    }
+    // fold: after the step over lane bit o a lane holds half as many sums, those whose index has that bit like the lane
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const int half = 2 * o;
+#pragma unroll
+        for (int i = 0; i < half; ++i) {
+            const bool up = (lane & o) != 0;
+            const double give = up ? acc[i] : acc[i + half], keep = up ? acc[i + half] : acc[i];
+            acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    // lane l: sums 2 l and 2 l + 1 (bit 16 chose between the halves of 64, ..., bit 1 between the halves of 4)
+    part[warp][2 * lane] = acc[0];
+    part[warp][2 * lane + 1] = acc[1];
+    __syncthreads();
+    if (warp % ksplit) return;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int idx = 2 * lane + h;
+        double total = part[warp][idx];
+        for (int q = 1; q < ksplit; ++q) total += part[warp + q][idx];
+        const uint64_t row = row0 + idx / R, e = e0 + idx % R;
+        if (row >= rows || e >= experts) continue;
+        const float v = (float)total;
+        if (!isfinite(v)) raise(status, YVEX_B200_STATUS_NUMERIC);
+        logits[row * experts + e] = v;
+    }
+}
+
 // ---- decode-width router: ingress rounding + projection + score in one launch ---------------------
 // One CTA per (expert, row): dot of the expert's router row with the bf16-rounded input in double
 // (same arithmetic as router_logits_kernel), then score = sqrt(softplus(logit)) in double
@@ -308,9 +377,16 @@ static int route_into(const MoeGeom &g, const yvex_b200_moe_weights *w, const fl
     const float *logits = logits_in;
     int launches = 1;
     if (w->router) {
-        uint64_t jobs = rows * g.experts;
-        unsigned grid = grid_for(jobs, 8, 8);
-        router_logits_kernel<<<grid, 256, 0, s>>>(w->router, xr, rows, g.experts, g.hidden, logits_ws, status);
+        if (g.hidden % 4 == 0 && ((reinterpret_cast<uintptr_t>(w->router) | reinterpret_cast<uintptr_t>(xr)) & 15u) == 0) {
+            // (16-byte loads; other widths and addresses take the dot-by-dot kernel)
+            const uint64_t rt = (rows + kRouterTile - 1) / kRouterTile, et = (g.experts + kRouterTile - 1) / kRouterTile;
+            const int ksplit = rt * et < (uint64_t)kSmCount * 8 ? kRouterTileWarps : 1;      // one warp per tile is at least 8 warps per SM
+            const uint64_t per = (uint64_t)(kRouterTileWarps / ksplit);
+            router_tile_kernel<<<dim3((unsigned)rt, (unsigned)((et + per - 1) / per)), 32 * kRouterTileWarps, 0, s>>>(
+                w->router, xr, rows, g.experts, g.hidden, ksplit, logits_ws, status);
+        } else {
+            router_logits_kernel<<<grid_for(rows * g.experts, 8, 8), 256, 0, s>>>(w->router, xr, rows, g.experts, g.hidden, logits_ws, status);
+        }
         logits = logits_ws;
         ++launches;
     } else if (!logits_in) {
