@@ -310,3 +310,43 @@ def test_router_projection_tiles(L, rows, experts, hidden):
     assert st.read() == 0
     want = x.astype(np.float64) @ router.astype(np.float64).T
     assert np.allclose(logits.cpu().numpy(), want, rtol=2.0 ** -23, atol=1e-12)
+
+
+@pytest.mark.parametrize("gate,down,hidden,inter", [(synth.IQ2_XXS, synth.Q4_K, 512, 256), (synth.IQ2_XXS, synth.Q2_K, 1280, 768),
+                                                    (synth.Q4_K, synth.IQ2_XXS, 256, 512), (synth.Q2_K, synth.Q2_K, 768, 1280)])
+def test_grouped_gemm_tile_edges(L, gate, down, hidden, inter):
+    """Group sizes around every edge of a tile - the 16 columns of an MMA, the 32- and 64-row boxes, one, two and three column
+    blocks of equal width - with one to five superblocks along K (rows that start on every 16-byte phase), against 64 bits over
+    the decoded weights with the layer's two bf16 roundings: 1e-3, the bound of the layer outputs."""
+    import torch
+    counts = [0, 1, 15, 16, 17, 31, 33, 64, 65, 97, 128, 129, 192, 193, 224, 225, 256, 257, 448, 449, 700]
+    E = len(counts)
+    spec = synth.MoELayerSpec(hidden, E, 2, inter, gate_qtype=gate, down_qtype=down)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(hidden)
+    from yvex_b200.workloads import device_blocks
+    t = {n: device_blocks(torch, q, r, w, gen, "cuda") for n, q, r, w in (
+        ("gate", gate, E * inter, hidden), ("up", gate, E * inter, hidden), ("down", down, E * hidden, inter),
+        ("shared_gate", gate, inter, hidden), ("shared_up", gate, inter, hidden), ("shared_down", down, hidden, inter))}
+    ids = torch.cat([torch.full((n,), e, dtype=torch.int32) for e, n in enumerate(counts)] + [torch.full((130,), -1, dtype=torch.int32)])
+    ids = ids[torch.randperm(ids.numel(), generator=torch.Generator().manual_seed(1))].cuda()
+    P = ids.numel()
+    x = torch.randn((P, hidden), device="cuda", generator=gen).to(torch.bfloat16)
+    w = torch.rand(P, device="cuda", generator=gen) + 0.5
+    st = L.Status()
+    y = L.moe_expert_rows(L.geometry_of(spec), L.weights_of(t), x.half(), ids, w, st)
+    assert st.read() == 0
+    want = torch.empty((P, hidden), dtype=torch.float64, device="cuda")
+    for e in list(range(E)) + [-1]:
+        rows = (ids == e).nonzero()[:, 0]
+        if not rows.numel():
+            continue
+        part = lambda n, q, r, c: L.dequant_rows(q, (t["shared_" + n] if e < 0 else t[n].reshape(E, -1)[e]).contiguous(), r, c, st).double()  # noqa: E731
+        g, u = x[rows].double() @ part("gate", gate, inter, hidden).T, x[rows].double() @ part("up", gate, inter, hidden).T
+        g, u = g.clamp(max=spec.limit), u.clamp(-spec.limit, spec.limit)
+        mid = (g * torch.sigmoid(g) * u * w[rows].double()[:, None]).to(torch.bfloat16).double()
+        want[rows] = (mid @ part("down", down, hidden, inter).T).to(torch.bfloat16).double()
+    for e in list(range(E)) + [-1]:
+        rows = (ids == e).nonzero()[:, 0]
+        if rows.numel():
+            assert rel_l2(y[rows].float().cpu().numpy(), want[rows].cpu().numpy()) <= 1e-3, (e, rows.numel())

@@ -1,11 +1,9 @@
 // Grouped dequant GEMM on the 5th-generation tensor cores (tcgen05 + TMEM) for the wide MoE path.
 //
 // Problem: for every expert group g with n_g token rows, OUT[row][m] = sum_k W_g[m][k] * X[row][k],
-// W_g stored as GGUF superblocks. Weights sit on the MMA M side (128-row tiles), tokens on N
-// (<=256 per tile for qtypes without a min term, <=128 for the affine ones whose second
-// accumulator needs the other half of TMEM; ragged tails padded to 16), so a small group wastes
-// at most 15 columns. A wider N halves the shared-memory traffic per flop of everything on the
-// weight side (decode stores, table lookups, A operand reads), which is what bounds this kernel.
+// W_g stored as GGUF superblocks. Weights sit on the MMA M side (128-row tiles), tokens on N; a group's
+// rows are cut into column blocks of equal width (a multiple of 16), because tensor time follows the
+// width while every block decodes the same weights again.
 //
 // Exactness: the A operand carries EXACT small integers in fp16 (IQ2_XXS: +-{8,25,43}*(2*sub+1);
 // Q4_K / Q2_K: code * sub-scale), the B operand the fp16 image of bf16-exact activations, so
@@ -15,20 +13,28 @@
 // being filled. Affine qtypes add one more K=16/32 MMA per superblock: A' = integer mins,
 // B' = per-sub-block activation sums (hi/lo fp16 split), drained as acc -= dmin * tmem'.
 //
+// Where the operands live, and why. Shared memory is the unit this kernel runs out of: with A in shared
+// memory a 64-K chunk cost 16 KiB of tile stores, 16 KiB of A and up to 32 KiB of B operand reads,
+// 32 KiB of TMA writes and the bank conflicts of 64 table lookups per row - about 930 cycles of
+// its 128 bytes per cycle against 512 cycles of MMA. So the decoded A operand goes to TENSOR memory
+// (tcgen05.st from the decoding warps, tcgen05.mma with A in TMEM): neither its stores nor its reads
+// touch shared memory any more, and the room it leaves holds the IQ2_XXS tables replicated per lane
+// (64 KiB, no conflicts). The price is the columns: 224 instead of 256 per IQ2_XXS tile, and one
+// min-term accumulator instead of two.
+//
 // CTA = 28 warps, persistent over a device-built tile list:
-//   warp 0      TMA producer: activation tiles [N x 64] fp16, 128-byte swizzle, mbarrier tx; and the raw
-//               weight superblocks of the tile's 128 rows (u8 boxes, three superblocks in flight)
-//   warps 1-2   MMA issuers (one elected lane each, alternating superblocks / TMEM buffers):
-//               4 x tcgen05.mma (K=16) per 64-K chunk
-//   warp 3      B' tiles of the min term (copies the activation sums into the swizzled tile)
-//   warps 4-11  dequant producers. Each warp owns 16 weight rows of the tile; thread = (row, half of a
-//               64-K chunk) decodes 32 weights of the staged superblock to fp16 and stores 16-byte
-//               chunks into the swizzled A tile. The same warps write the A' rows and the
-//               per-row block scales for the epilogue. (Staging the raw bytes through these warps'
-//               registers cost them about as many instructions as the decode itself.)
-//   warps 12-27 epilogue, one warp per (32 TMEM lanes, 64 or 32 columns): TMEM -> registers
-//               (tcgen05.ld), scale, accumulate, final store
-// Every mbarrier wait is bounded; on expiry the CTA sets status 3, unwinds and frees its TMEM.
+//   warp 0      TMA producer: activation tiles [N x 64] fp16, 128-byte swizzle, mbarrier tx; B' tiles of the
+//               min term (the sub-block sums, 64-byte swizzle); the lookup tables once
+//   warp 1      MMA issuer: per 64-K chunk 4 x tcgen05.mma (K=16), superblocks alternating between two accumulators
+//   warp 2      TMA producer: the raw weight superblocks of the tile's 128 rows (u8 boxes, four or five in flight)
+//   warp 3      looks the tiles up ahead of the other roles
+//   then the dequant producers: thread = (row, half of a 64-K chunk) decodes 32 weights of the staged
+//               superblock to fp16 and stores them into its row's lane of the A ring; the same warps write the A'
+//               rows and the per-row block scales for the epilogue
+//   and the epilogue warps, one per (32 TMEM lanes, 32 or 64 columns): TMEM -> registers (tcgen05.ld), scale,
+//               accumulate, final store
+// Single-lane roles are chosen with elect.sync. Every mbarrier wait is bounded; on expiry the CTA sets
+// status 3, unwinds and frees its TMEM.
 //
 // Two forms. The plain one multiplies by ONE matrix and stores bf16 rows (down projection). The
 // fused one computes gate and up together: a tile's 128 A rows are 64 gate rows and the 64 up rows
@@ -41,18 +47,17 @@
 #pragma once
 #include <type_traits>
 
-#include "gemv_mma.cuh"
+#include "gemv_stream.cuh"
 #include "moe_common.cuh"
 #include "tcgen05.cuh"
 
 namespace yb {
 
-constexpr int kTileM = 128, kBoxN = 128, kMaxTileN = 256, kChunkK = 64;
-constexpr int kStages = 4;                                  // {A, B} 64-K chunk stages: two rings of two
-constexpr uint32_t kTileBytes = kTileM * kChunkK * 2;        // 16 KiB: an A chunk, or one 128-row box of a B chunk
+constexpr int kTileM = 128, kBoxN = 64, kMinTileN = 128, kChunkK = 64;
+constexpr uint32_t kBoxBytes = kBoxN * kChunkK * 2;          // activations arrive in boxes of 64 rows: a ragged tile fetches what it needs
+constexpr uint32_t kMinTileBytes = kTileM * 64;               // 8 KiB: A' or B' of the min term, 32 fp16 per row, 64-byte swizzle
 constexpr uint32_t kTmemCols = 512;
 constexpr int kScaleRing = 4;                               // superblocks of per-row scales kept for the epilogue
-constexpr int kRawStages = 3;                               // raw weight superblocks in flight
 
 // <= kTileN token rows of one expert (expert < 0: the shared expert). Column blocks of the same expert
 // form groups of consecutive entries [first, first + count) covering <= kGroupRows rows: the tiles of a
@@ -65,14 +70,15 @@ constexpr int kGroupRows = 1024;
 // `fuse` consecutive rows joined into one tensor row, so that the row pitch is a multiple of 16
 // bytes whatever the block size (66-byte IQ2_XXS blocks give pitches that are only multiples of 2).
 struct GemmMaps {
-    CUtensorMap act;
+    CUtensorMap act, act_tail;                  // activation rows in boxes of 64 and of 32 rows
+    CUtensorMap sums;                           // affine qtypes: [rows][K/256][32] hi/lo sub-block sums
     CUtensorMap w_routed[2], w_shared[2];
 };
 
 struct GemmParams {
     uint32_t row_bytes;
     int fuse;                                   // rows per tensor row of the weight maps: 1, 2, 4 or 8
-    int M, K, nmat;
+    int M, K;
     const ColBlock *colblocks;
     const int *num_colblocks;
     uint16_t *out_bf16;                         // [rows][M] bf16 bits (plain kernel: down results) ...
@@ -84,25 +90,26 @@ struct GemmParams {
     __half *mid;                                // ... or [rows][M] SwiGLU intermediates as fp16 (fused gate/up kernel)
     const float *col_weight;                    // route weight of sorted row r (fused kernel)
     float limit;                                // SwiGLU clamp (fused kernel)
-    const __half *sums;                         // [rows][K/256][32] hi/lo sub-block sums (affine qtypes)
     int *status;
 };
 
+constexpr int kTileRing = 4;                                // tiles looked up ahead of the roles
+
 struct GemmSmem {
-    uint64_t full[kStages], empty[kStages];
-    uint64_t raw_full[kRawStages], raw_empty[kRawStages];
+    uint64_t a_full[4], a_empty[4], b_full[5], b_empty[5], tab_full;
+    uint64_t raw_full[5], raw_empty[5];
     uint64_t acc_full[2], acc_empty[2], min_full[2], min_empty[2];
+    uint64_t tile_full[kTileRing], tile_empty[kTileRing];
+    int4 tile[kTileRing];                                   // {first row, columns, expert, m tile} of the tiles ahead
     uint32_t tmem_base;
     int abort;
 };
 
-// Chunk `it` (four per superblock, counted over the CTA's whole tile sequence) -> stage and phase.
-// Even superblocks cycle through stages 0-1, odd ones through stages 2-3, so each MMA issuer
-// only ever waits on stages whose fills it consumes itself, in order. (With one shared ring an
-// issuer that skips the other's superblock could test a barrier that is still a whole phase
-// behind, and a parity wait cannot tell "one phase behind" from "done".)
-__device__ __forceinline__ uint32_t stage_of(uint32_t it) { return ((it >> 1) & 2u) | (it & 1u); }
-__device__ __forceinline__ uint32_t phase_of(uint32_t it) { return (it >> 1) & 1u; }     // fills per stage: 2 per own superblock
+// A ring position: stage and the parity of its current use.
+struct RingAt {
+    uint32_t s = 0, ph = 0;
+    template <int kDepth> __device__ __forceinline__ void next() { if (++s == (uint32_t)kDepth) { s = 0; ph ^= 1u; } }
+};
 
 // ---- per-qtype decoders -----------------------------------------------------------------------------
 // A decoder sees one superblock of one weight row as 32-bit words in shared memory, starting at the
@@ -113,15 +120,32 @@ __device__ __forceinline__ uint32_t phase_of(uint32_t it) { return (it >> 1) & 1
 //   store      weights k = 64*c + (64/kParts)*part .. -> 16-byte fp16 chunks of the A tile row
 //   scales     {d, dmin} of the block, and whether they are acceptable
 //   mins       this thread's share of the A' row (affine qtypes)
-__device__ __forceinline__ void store_scaled8(uint8_t *tile, uint32_t row, uint32_t chunk, uint32_t bytes_lo,
-                                              uint32_t bytes_hi, __half2 sc2, __half2 nb2) {
-    uint32_t a = __byte_perm(bytes_lo, 0x64646464u, 0x4140), b = __byte_perm(bytes_lo, 0x64646464u, 0x4342);
-    uint32_t c = __byte_perm(bytes_hi, 0x64646464u, 0x4140), d = __byte_perm(bytes_hi, 0x64646464u, 0x4342);
-    __half2 va = __hfma2(*reinterpret_cast<__half2 *>(&a), sc2, nb2), vb = __hfma2(*reinterpret_cast<__half2 *>(&b), sc2, nb2);
-    __half2 vc = __hfma2(*reinterpret_cast<__half2 *>(&c), sc2, nb2), vd = __hfma2(*reinterpret_cast<__half2 *>(&d), sc2, nb2);
-    uint4 v = make_uint4(*reinterpret_cast<uint32_t *>(&va), *reinterpret_cast<uint32_t *>(&vb),
-                         *reinterpret_cast<uint32_t *>(&vc), *reinterpret_cast<uint32_t *>(&vd));
-    *reinterpret_cast<uint4 *>(tile + sm100::sw128_offset(row, chunk)) = v;
+// prmt.b32 with a run-time selector. (__byte_perm masks the selector with 0x7777 first; the decoders'
+// selectors never have bit 3 of a nibble set, and the instruction reads only the low 16 bits.)
+__device__ __forceinline__ uint32_t prmt_raw(uint32_t a, uint32_t b, uint32_t sel) {
+    uint32_t d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+    return d;
+}
+
+// Eight codes (bytes) -> eight fp16 (code + bias - bias) * scale in K order, exact: 0x6400 | b is 1024 + b, and the product with
+// the integer scale and the subtraction round once.
+__device__ __forceinline__ void scaled8(uint32_t bytes_lo, uint32_t bytes_hi, uint32_t sc2, uint32_t nb2, uint32_t *v) {
+    v[0] = prmt_raw(bytes_lo, 0x64646464u, 0x4140); v[1] = prmt_raw(bytes_lo, 0x64646464u, 0x4342);
+    v[2] = prmt_raw(bytes_hi, 0x64646464u, 0x4140); v[3] = prmt_raw(bytes_hi, 0x64646464u, 0x4342);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const __half2 h = __hfma2(*reinterpret_cast<__half2 *>(&v[i]), *reinterpret_cast<const __half2 *>(&sc2), *reinterpret_cast<const __half2 *>(&nb2));
+        v[i] = *reinterpret_cast<const uint32_t *>(&h);
+    }
+}
+// An integer scale s < 64 as half2(s, s), and half2(-bias * s) (exact: bias is 1024 or 1152).
+__device__ __forceinline__ void scale_pair(uint32_t s, float bias, uint32_t &sc2, uint32_t &nb2) {
+    const uint32_t dup = prmt_raw(s, 0x64646464u, 0x4040);
+    const __half2 v = __hsub2(*reinterpret_cast<const __half2 *>(&dup), __float2half2_rn(1024.0f));
+    const __half2 n = __hmul2(v, __float2half2_rn(-bias));
+    sc2 = *reinterpret_cast<const uint32_t *>(&v);
+    nb2 = *reinterpret_cast<const uint32_t *>(&n);
 }
 
 // Four bytes (each < 1024) -> four exact fp16 values: 0x6400 | b is 1024 + b, minus 1024.
@@ -138,137 +162,139 @@ __device__ __forceinline__ float2 checked_scales(uint32_t d_bits, uint32_t dmin_
     return make_float2(d * d_mul, dmin);
 }
 
-// prmt.b32 with a run-time selector. (__byte_perm masks the selector with 0x7777 first; the decoders'
-// selectors never have bit 3 of a nibble set, and the instruction reads only the low 16 bits.)
-__device__ __forceinline__ uint32_t prmt_raw(uint32_t a, uint32_t b, uint32_t sel) {
-    uint32_t d;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
-    return d;
-}
-
 struct GemmIq2 {
     static constexpr int kBlockBytes = 66, kMinSlots = 0, kBoxBytes = 80;     // 66 bytes from a 2-byte aligned start
-    static constexpr int kParts = 2;
-    static constexpr float kBias = 1152.0f;
-    __device__ static void store(const uint32_t *raw, uint32_t mis, int c, int h, uint8_t *tile, uint32_t row,
-                                 const MmaTables *tab) {
-        const uint32_t o = mis + 2u + 8u * (2 * c + h), sh = 8u * (o & 3u);
-        const uint32_t *w = raw + (o >> 2);
+    static constexpr uint32_t kTableBytes = gs::kTableBytes;
+    struct Block { const uint32_t *raw; uint32_t mis; };
+    struct Half { uint32_t sel[4], sc2, nb2; };
+    __device__ static void open(const uint8_t *slot, uint32_t off, Block &b) { b.raw = reinterpret_cast<const uint32_t *>(slot + (off & ~3u)); b.mis = off & 3u; }
+    __device__ static void fetch(const Block &b, int c, int h, const uint8_t *tab, uint32_t lane4, Half &p) {
+        const uint32_t o = b.mis + 2u + 8u * (2 * c + h), sh = 8u * (o & 3u);
+        const uint32_t *w = b.raw + (o >> 2);
         const uint32_t w1 = w[1];
         const uint32_t grids = __funnelshift_r(w[0], w1, sh), ss = __funnelshift_r(w1, w[2], sh);
-        const uint2 sc = tab->scale[2u * (ss >> 28) + 1u];
-        const __half2 sc2 = *reinterpret_cast<const __half2 *>(&sc.x), nb2 = *reinterpret_cast<const __half2 *>(&sc.y);
+        // index byte into byte 1 of the table offset, the lane's column into byte 0 (each lane has its own bank)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            p.sel[j] = *reinterpret_cast<const uint32_t *>(tab + prmt_raw(grids, lane4, 0x5504u | ((uint32_t)j << 4))) |
+                       *reinterpret_cast<const uint32_t *>(tab + 128 + prmt_raw(ss >> (7 * j), lane4, 0x5504u));
+        scale_pair((ss >> 27) | 1u, 1152.0f, p.sc2, p.nb2);                                      // 2 * sub + 1
+    }
+    // weights 64 c + 32 h + 16 q .. + 15 as eight words of two fp16
+    __device__ static void convert(const Half &p, int q, uint32_t (&v)[8]) {
         constexpr uint32_t kLo = (8u + 128u) | ((25u + 128u) << 8) | ((43u + 128u) << 16);
         constexpr uint32_t kHi = (128u - 8u) | ((128u - 25u) << 8) | ((128u - 43u) << 16);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint32_t sel = tab->nib[(grids >> (8 * j)) & 255u] | tab->sign[(ss >> (7 * j)) & 127u];
-            store_scaled8(tile, row, 4 * h + j, prmt_raw(kLo, kHi, sel), prmt_raw(kLo, kHi, sel >> 16), sc2, nb2);
-        }
+        for (int j = 0; j < 2; ++j)
+            scaled8(prmt_raw(kLo, kHi, p.sel[2 * q + j]), prmt_raw(kLo, kHi, p.sel[2 * q + j] >> 16), p.sc2, p.nb2, v + 4 * j);
     }
-    __device__ static float2 scales(const uint32_t *raw, uint32_t mis, bool &bad) {
-        return checked_scales(raw[0] >> (8u * mis), 0u, 0.125f, bad);
-    }
-    __device__ static void mins(const uint32_t *, int, uint8_t *, uint32_t) {}
+    __device__ static float2 scales(const Block &b, bool &bad) { return checked_scales(b.raw[0] >> (8u * b.mis), 0u, 0.125f, bad); }
+    __device__ static void mins(const Block &, int, uint8_t *, uint32_t) {}
 };
 
 struct GemmQ4k {
     static constexpr int kBlockBytes = 144, kMinSlots = 16, kBoxBytes = 144;   // 8 mins x (hi, lo); blocks are 16-byte aligned
-    static constexpr int kParts = 4;
-    static constexpr float kBias = 1024.0f;
-    // 6-bit (scale, min) of sub-block j from the 12 packed bytes held as three little-endian words
-    __device__ static void scale_min_words(uint32_t s0, uint32_t s1, uint32_t s2, int j, uint32_t &sc, uint32_t &m) {
-        const uint32_t w[3] = {s0, s1, s2};
-        auto byte = [&](int i) { return (w[i >> 2] >> (8 * (i & 3))) & 255u; };
-        if (j < 4) { sc = byte(j) & 63u; m = byte(j + 4) & 63u; }
-        else { sc = (byte(j + 4) & 15u) | ((byte(j - 4) >> 6) << 4); m = (byte(j + 4) >> 4) | ((byte(j) >> 6) << 4); }
+    static constexpr uint32_t kTableBytes = 0;
+    struct Block { const uint4 *raw; uint4 head; };
+    struct Half { uint4 q[2]; uint32_t sc2, nb2, shift; };
+    __device__ static void open(const uint8_t *slot, uint32_t, Block &b) { b.raw = reinterpret_cast<const uint4 *>(slot); b.head = b.raw[0]; }   // d, dmin and the 12 scale bytes
+    // sub-block 2c + h: the low (h = 0) or high nibbles of the chunk's 32 bytes. Its 6-bit scale: byte k of the first four
+    // scale bytes, or (c >= 2) the low nibble of byte k of the last four under the top two bits of the first's.
+    __device__ static void fetch(const Block &b, int c, int h, const uint8_t *, uint32_t, Half &p) {
+        p.q[0] = b.raw[1 + 2 * c];
+        p.q[1] = b.raw[2 + 2 * c];
+        const uint32_t k8 = 8u * (uint32_t)(2 * (c & 1) + h);
+        const uint32_t sc = c < 2 ? (b.head.y >> k8) & 63u : ((b.head.w >> k8) & 15u) | (((b.head.y >> (k8 + 6u)) & 3u) << 4);
+        p.shift = 4u * (uint32_t)h;
+        scale_pair(sc, 1024.0f, p.sc2, p.nb2);
     }
-    // part = 2 * h + half: sub-block 2c + h (low or high nibbles of the chunk's 32 bytes), bytes 16*half .. +15
-    __device__ static void store(const uint32_t *raw, uint32_t, int c, int part, uint8_t *tile, uint32_t row, const MmaTables *tab) {
-        const int h = part >> 1;
-        uint32_t sc, m;
-        scale_min_words(raw[1], raw[2], raw[3], 2 * c + h, sc, m);
-        const uint2 s = tab->scale[sc];
-        const __half2 sc2 = *reinterpret_cast<const __half2 *>(&s.x), nb2 = *reinterpret_cast<const __half2 *>(&s.y);
-        const uint4 q = *reinterpret_cast<const uint4 *>(raw + 4 + 8 * c + 4 * (part & 1));
-        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const uint32_t a = h ? (w[2 * j] >> 4) & 0x0f0f0f0fu : w[2 * j] & 0x0f0f0f0fu;
-            const uint32_t b = h ? (w[2 * j + 1] >> 4) & 0x0f0f0f0fu : w[2 * j + 1] & 0x0f0f0f0fu;
-            store_scaled8(tile, row, 2 * part + j, a, b, sc2, nb2);
-        }
+    __device__ static void convert(const Half &p, int q, uint32_t (&v)[8]) {
+        scaled8((p.q[q].x >> p.shift) & 0x0f0f0f0fu, (p.q[q].y >> p.shift) & 0x0f0f0f0fu, p.sc2, p.nb2, v);
+        scaled8((p.q[q].z >> p.shift) & 0x0f0f0f0fu, (p.q[q].w >> p.shift) & 0x0f0f0f0fu, p.sc2, p.nb2, v + 4);
     }
-    __device__ static float2 scales(const uint32_t *raw, uint32_t, bool &bad) {
-        return checked_scales(raw[0], raw[0] >> 16, 1.0f, bad);
-    }
-    // A' row: slots 0..7 = the eight mins (paired with the hi sums), 8..15 = the same mins (lo sums);
-    // thread h writes 16-byte part h.
-    // (the eight 6-bit mins, four bytes at a time: mins 0..3 are bytes 4..7 & 63, mins 4..7 the high
-    // nibbles of bytes 8..11 with the top two bits of bytes 4..7 above them)
-    __device__ static void mins(const uint32_t *raw, int h, uint8_t *tile, uint32_t row) {
-        const uint32_t s1 = raw[2], s2 = raw[3];
-        const uint2 a = bytes_to_half4(s1 & 0x3f3f3f3fu);
-        const uint2 b = bytes_to_half4(((s2 >> 4) & 0x0f0f0f0fu) | (((s1 >> 6) & 0x03030303u) << 4));
-        *reinterpret_cast<uint4 *>(tile + sm100::sw128_offset(row, h)) = make_uint4(a.x, a.y, b.x, b.y);
+    __device__ static float2 scales(const Block &b, bool &bad) { return checked_scales(b.head.x, b.head.x >> 16, 1.0f, bad); }
+    // A' row: slots 0..7 = the eight mins (paired with the hi sums), 8..15 = the same mins (lo sums); thread h writes
+    // 16-byte part h. (four bytes at a time: mins 0..3 are bytes 4..7 & 63, mins 4..7 the high nibbles of bytes 8..11 with
+    // the top two bits of bytes 4..7 above them)
+    __device__ static void mins(const Block &b, int h, uint8_t *tile, uint32_t row) {
+        const uint32_t s1 = b.head.z, s2 = b.head.w;
+        const uint2 lo = bytes_to_half4(s1 & 0x3f3f3f3fu);
+        const uint2 hi = bytes_to_half4(((s2 >> 4) & 0x0f0f0f0fu) | (((s1 >> 6) & 0x03030303u) << 4));
+        *reinterpret_cast<uint4 *>(tile + sm100::sw64_offset(row, h)) = make_uint4(lo.x, lo.y, hi.x, hi.y);
     }
 };
 
 struct GemmQ2k {
-    static constexpr int kBlockBytes = 84, kMinSlots = 32, kBoxBytes = 96;     // 16 mins x (hi, lo); 4-byte aligned start
-    static constexpr int kParts = 4;
-    static constexpr float kBias = 1024.0f;
-    // part = 2 * h + half: 2-bit plane 2*(c&1) + h of the 32 bytes, bytes 16*half .. +15 (one 16-weight sub-block)
-    __device__ static void store(const uint32_t *raw, uint32_t, int c, int part, uint8_t *tile, uint32_t row, const MmaTables *tab) {
-        const int hf = c >> 1, plane = 2 * (c & 1) + (part >> 1), half = part & 1;
-        const uint32_t *q = raw + 4 + 8 * hf + 4 * half;
-        const uint32_t sbytes = raw[2 * hf + (plane >> 1)] >> (16 * (plane & 1) + 8 * half);   // scale byte 8*hf + 2*plane + half
-        const uint2 s = tab->scale[sbytes & 15u];
+    // 16 mins x (hi, lo); 4-byte aligned start. The box is 112 bytes, not the 96 that hold a block: rows seven 16-byte units
+    // apart meet no two on the same banks in 16-byte reads.
+    static constexpr int kBlockBytes = 84, kMinSlots = 32, kBoxBytes = 112;
+    static constexpr uint32_t kTableBytes = 0;
+    struct Block { uint32_t w[24]; };           // w[0..3] scales and mins, w[4..19] codes, w[20] d and dmin
+    struct Half { uint32_t q[8], s, plane2; };
+    // The whole block in six 16-byte reads, then moved down to word 0 by the start's offset (word reads at a 112-byte pitch
+    // would be four to a bank, and a thread needs every word of the block).
+    __device__ static void open(const uint8_t *slot, uint32_t off, Block &b) {
+        const uint4 *raw = reinterpret_cast<const uint4 *>(slot);
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const uint32_t a = (q[2 * j] >> (2 * plane)) & 0x03030303u, b = (q[2 * j + 1] >> (2 * plane)) & 0x03030303u;
-            store_scaled8(tile, row, 2 * part + j, a, b, *reinterpret_cast<const __half2 *>(&s.x), *reinterpret_cast<const __half2 *>(&s.y));
-        }
+        for (int i = 0; i < 6; ++i) { const uint4 v = raw[i]; b.w[4 * i] = v.x; b.w[4 * i + 1] = v.y; b.w[4 * i + 2] = v.z; b.w[4 * i + 3] = v.w; }
+#pragma unroll
+        for (int i = 0; i < 23; ++i) b.w[i] = (off & 4u) ? b.w[i + 1] : b.w[i];
+#pragma unroll
+        for (int i = 0; i < 21; ++i) b.w[i] = (off & 8u) ? b.w[i + 2] : b.w[i];
     }
-    __device__ static float2 scales(const uint32_t *raw, uint32_t, bool &bad) {
-        return checked_scales(raw[20], raw[20] >> 16, 1.0f, bad);
+    // plane 2 (c & 1) + h of the 32 bytes of half c >> 1: two 16-weight sub-blocks, scale bytes 8 (c >> 1) + 2 plane + (0, 1)
+    __device__ static void fetch(const Block &b, int c, int h, const uint8_t *, uint32_t, Half &p) {
+        p.plane2 = 2u * (uint32_t)(2 * (c & 1) + h);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) p.q[i] = b.w[4 + 8 * (c >> 1) + i];
+        p.s = b.w[2 * (c >> 1) + (c & 1)] >> (16 * h);
     }
-    // A' row: slots 0..15 = the sixteen mins (hi sums), 16..31 = the same mins (lo sums); thread h
-    // converts mins 8h..8h+7 and writes them to parts h and h + 2.
-    __device__ static void mins(const uint32_t *raw, int h, uint8_t *tile, uint32_t row) {
-        const uint2 a = bytes_to_half4((raw[2 * h] >> 4) & 0x0f0f0f0fu), b = bytes_to_half4((raw[2 * h + 1] >> 4) & 0x0f0f0f0fu);
-        const uint4 v = make_uint4(a.x, a.y, b.x, b.y);
-        *reinterpret_cast<uint4 *>(tile + sm100::sw128_offset(row, h)) = v;
-        *reinterpret_cast<uint4 *>(tile + sm100::sw128_offset(row, h + 2)) = v;
+    __device__ static void convert(const Half &p, int q, uint32_t (&v)[8]) {
+        uint32_t sc2, nb2;
+        scale_pair((p.s >> (8 * q)) & 15u, 1024.0f, sc2, nb2);
+        scaled8((p.q[4 * q] >> p.plane2) & 0x03030303u, (p.q[4 * q + 1] >> p.plane2) & 0x03030303u, sc2, nb2, v);
+        scaled8((p.q[4 * q + 2] >> p.plane2) & 0x03030303u, (p.q[4 * q + 3] >> p.plane2) & 0x03030303u, sc2, nb2, v + 4);
+    }
+    __device__ static float2 scales(const Block &b, bool &bad) { return checked_scales(b.w[20], b.w[20] >> 16, 1.0f, bad); }
+    // A' row: slots 0..15 = the sixteen mins (hi sums), 16..31 = the same mins (lo sums); thread h converts mins 8h..8h+7
+    // and writes them to parts h and h + 2.
+    __device__ static void mins(const Block &b, int h, uint8_t *tile, uint32_t row) {
+        const uint2 lo = bytes_to_half4(((h ? b.w[2] : b.w[0]) >> 4) & 0x0f0f0f0fu), hi = bytes_to_half4(((h ? b.w[3] : b.w[1]) >> 4) & 0x0f0f0f0fu);
+        const uint4 v = make_uint4(lo.x, lo.y, hi.x, hi.y);
+        *reinterpret_cast<uint4 *>(tile + sm100::sw64_offset(row, h)) = v;
+        *reinterpret_cast<uint4 *>(tile + sm100::sw64_offset(row, h + 2)) = v;
     }
 };
 
 // ---- shared-memory plan -----------------------------------------------------------------------------
 // tiles (1024-byte aligned; the kernel refuses to run if the dynamic shared memory does not start on
-// such a boundary): A ring, B ring, [min tiles: A' in 16-byte parts 0..3 of each row, B' in parts
-// 4..7], then the raw superblock ring (kRawStages x 128 rows x kBoxBytes, plus a pad: the decoders'
-// funnel reads run one word over), the scale ring, the decode tables and the barriers.
+// such a boundary): B ring, [min tiles: two A', two B'], then the raw superblock ring (kRawStages x 128 rows x
+// kBoxBytes, plus a pad: the decoders' funnel reads run one word over), the scale ring, the lookup tables and the barriers.
 template <class Dec> struct GemmPlan {
     static constexpr bool kHasMin = Dec::kMinSlots > 0;
-    static constexpr int kTileN = kHasMin ? 128 : 256;                              // columns per tile
+    // Tensor memory: two accumulators of kTileN columns that alternate by superblock, one min-term accumulator (affine), and
+    // the A ring: 32 columns (two fp16 each) per 64-K chunk. 224 + 224 + 2 x 32, or 128 + 128 + 128 + 4 x 32.
+    static constexpr int kTileN = kHasMin ? 128 : 224;                              // columns per tile
+    static constexpr int kAStages = kHasMin ? 4 : 2, kBStages = kHasMin ? 5 : 4;
+    static constexpr int kRawStages = kHasMin ? 5 : 4;                      // raw weight superblocks in flight
+    static constexpr uint32_t kMinCol = 2 * kTileN, kACol = kTmemCols - kAStages * (kChunkK / 2);
+    static_assert(kMinCol + (kHasMin ? kTileN : 0) <= kACol, "tensor memory columns");
     // 8 producer and 16 epilogue warps: an epilogue warp owns 32 TMEM lanes x kColsPerWarp columns
-    // (64 with 256-column tiles, 32 with 128-column ones, where the shorter tile-end store matters
-    // more than more producers: with K of 1536..2048 a tile ends every six to eight superblocks)
-    static constexpr int kEpilogueWarps = 16, kColsPerWarp = kTileN / (kEpilogueWarps / 4);
-    static constexpr int kProducerWarps = 8, kRowsPerWarp = kTileM / kProducerWarps;
-    static constexpr int kPartsPerThread = Dec::kParts / (32 / kRowsPerWarp);       // chunk parts a producer thread decodes
+    static constexpr int kEpilogueWarps = 16, kColsPerWarp = kHasMin ? 32 : 64;
+    static constexpr int kProducerWarps = 8;
     static constexpr int kThreads = 32 * (4 + kProducerWarps + kEpilogueWarps);
-    // registers per thread of each role (setmaxnreg); the B' warp of the affine qtypes holds a tile of sums
-    static constexpr int kCtlRegs = kHasMin ? 72 : 48;                               // the B' warp holds eight uint4
-    static constexpr int kProdRegs = kHasMin ? 56 : 48, kEpiRegs = kHasMin ? 80 : 88;
-    static constexpr uint32_t kBTileBytes = (kTileN / kBoxN) * kTileBytes;
+    // registers per thread of each role (setmaxnreg)
+    static constexpr int kCtlRegs = kHasMin ? 48 : 40;
+    static constexpr int kProdRegs = kHasMin ? 72 : 56, kEpiRegs = kHasMin ? 72 : 88;
+    static constexpr uint32_t kBTileBytes = kTileN * kChunkK * 2;
     static constexpr uint32_t kRawStageBytes = kTileM * Dec::kBoxBytes;
     using Scale = typename std::conditional<kHasMin, float2, float>::type;          // {d, dmin} or d per row and superblock
-    static constexpr size_t kTilesBytes = (size_t)kStages * (kTileBytes + kBTileBytes) + (kHasMin ? 2 : 0) * (size_t)kTileBytes;
+    static constexpr size_t kTilesBytes = (size_t)kBStages * kBTileBytes + (kHasMin ? 4 : 0) * (size_t)kMinTileBytes;
     static constexpr size_t kRawBytes = (size_t)kRawStages * kRawStageBytes + 128;
     static constexpr size_t kScaleBytes = (size_t)kScaleRing * kTileM * sizeof(Scale);
-    static constexpr size_t kBytes = kTilesBytes + kRawBytes + kScaleBytes + sizeof(MmaTables) + sizeof(GemmSmem);
+    static constexpr size_t kBytes = kTilesBytes + kRawBytes + kScaleBytes + Dec::kTableBytes + sizeof(GemmSmem);
     static_assert(kBytes <= 227 * 1024, "shared memory plan exceeds the 227 KiB a CTA can have");
+    static_assert(kBTileBytes % 1024 == 0 && kTilesBytes % 1024 == 0, "swizzled tiles start on 1024-byte boundaries");
     static_assert(kRawStageBytes % 128 == 0 && (kTileM / 16) * Dec::kBoxBytes % 128 == 0,
                   "TMA destinations are 128-byte aligned (boxes of 64 rows, up to 8 rows fused)");
 };
@@ -280,6 +306,13 @@ template <int N, int kLaunched> __device__ __forceinline__ void set_registers() 
     else if constexpr (N < kLaunched) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
+// a0 = d * v0 + a0, a1 = d * v1 + a1 in one instruction (each rounded like fmaf)
+__device__ __forceinline__ void fma2(float &a0, float &a1, float d, uint32_t v0, uint32_t v1) {
+    asm("{\n\t.reg .b64 a, v, s;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 v, {%2, %3};\n\tmov.b64 s, {%4, %4};\n\t"
+        "fma.rn.f32x2 a, s, v, a;\n\tmov.b64 {%0, %1}, a;\n\t}"
+        : "+f"(a0), "+f"(a1) : "r"(v0), "r"(v1), "f"(d));
+}
+
 template <class Dec, bool kFused>
 __global__ void __launch_bounds__(GemmPlan<Dec>::kThreads, 1)
 moe_grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, GemmParams p) {
@@ -288,35 +321,35 @@ moe_grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, GemmParams p) {
     constexpr bool kHasMin = Plan::kHasMin;
     constexpr int kTileN = Plan::kTileN;
     constexpr uint32_t kBTileBytes = Plan::kBTileBytes;
-    constexpr int kProducerWarps = Plan::kProducerWarps, kRowsPerWarp = Plan::kRowsPerWarp;
+    constexpr int kProducerWarps = Plan::kProducerWarps, kAStages = Plan::kAStages, kBStages = Plan::kBStages, kRawStages = Plan::kRawStages;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     if (smem_u32(smem_raw) & 1023u) {                           // uniform: nothing has been set up yet
         if (threadIdx.x == 0) raise(p.status, YVEX_B200_STATUS_TIMEOUT);
         return;
     }
     uint8_t *tiles = smem_raw;
-    uint8_t *a_tiles = tiles;                                   // [kStages][16 KiB]
-    uint8_t *b_tiles = tiles + kStages * kTileBytes;            // [kStages][16 or 32 KiB]
-    uint8_t *min_tiles = b_tiles + kStages * kBTileBytes;       // [2][16 KiB] when the qtype has mins
+    uint8_t *b_tiles = tiles;                                   // [kBStages][kTileN rows x 128 bytes]
+    uint8_t *min_a = b_tiles + kBStages * kBTileBytes, *min_b = min_a + 2 * kMinTileBytes;      // [2][8 KiB] each when the qtype has mins
     uint8_t *raw_stage = tiles + Plan::kTilesBytes;             // [kRawStages][fuse][128 / fuse rows][kBoxBytes]
     typename Plan::Scale *dscale = reinterpret_cast<typename Plan::Scale *>(raw_stage + Plan::kRawBytes);
-    MmaTables *tab = reinterpret_cast<MmaTables *>(reinterpret_cast<uint8_t *>(dscale) + Plan::kScaleBytes);
-    GemmSmem *sm = reinterpret_cast<GemmSmem *>(reinterpret_cast<uint8_t *>(tab) + sizeof(MmaTables));
+    uint8_t *tab = reinterpret_cast<uint8_t *>(dscale) + Plan::kScaleBytes;
+    GemmSmem *sm = reinterpret_cast<GemmSmem *>(tab + Dec::kTableBytes);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        // full[s]: 8 producer warps + the TMA thread's expect_tx arrival (and its bytes) complete a stage,
-        // so an MMA issuer pays for one wait per 64-K chunk, not two.
-        for (int s = 0; s < kStages; ++s) { mbar_init(&sm->full[s], kProducerWarps + 1); mbar_init(&sm->empty[s], 1); }
+        for (int s = 0; s < kAStages; ++s) { mbar_init(&sm->a_full[s], kProducerWarps); mbar_init(&sm->a_empty[s], 1); }
+        for (int s = 0; s < kBStages; ++s) { mbar_init(&sm->b_full[s], 1); mbar_init(&sm->b_empty[s], 1); }
+        mbar_init(&sm->tab_full, 1);
         for (int s = 0; s < kRawStages; ++s) { mbar_init(&sm->raw_full[s], 1); mbar_init(&sm->raw_empty[s], kProducerWarps); }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&sm->acc_full[b], 1); mbar_init(&sm->acc_empty[b], Plan::kEpilogueWarps);
             mbar_init(&sm->min_full[b], kProducerWarps + 1); mbar_init(&sm->min_empty[b], 1);
         }
+        // readers of a tile's entry: the three single-lane roles and every epilogue warp
+        for (int i = 0; i < kTileRing; ++i) { mbar_init(&sm->tile_full[i], 1); mbar_init(&sm->tile_empty[i], 3 + Plan::kEpilogueWarps); }
         sm->abort = 0;
         fence_barrier_init();
     }
-    load_tables(tab, Dec::kBias);
     if (warp == 0) tmem_alloc(&sm->tmem_base, kTmemCols);
     tc_fence_before();
     __syncthreads();
@@ -327,207 +360,220 @@ moe_grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, GemmParams p) {
     const int ncb = *p.num_colblocks;
     constexpr int kRowsPerMat = kFused ? kTileM / 2 : kTileM;      // weight rows of one matrix in a tile
     const int mtiles = p.M / kRowsPerMat, nsb = p.K / 256;
-    const long long tiles_total = (long long)ncb * mtiles * p.nmat;
+    const uint32_t tiles_total = (uint32_t)ncb * (uint32_t)mtiles;
 
-    // Every role walks the same tile sequence: group of column blocks -> (matrix, m tile) -> column block.
-    auto tile_of = [&](long long t, ColBlock &cb, int &mat, int &mt) {
-        const int per_cb = mtiles * p.nmat;
-        const ColBlock g0 = p.colblocks[t / per_cb];            // any block of the group names the group
-        const int local = (int)(t - (long long)g0.first * per_cb);
-        const int r = local / g0.count;
-        cb = p.colblocks[g0.first + local % g0.count];
-        mat = r / mtiles;
-        mt = r % mtiles;
+    // Every role walks the same tile sequence: group of column blocks -> m tile -> column block. Warp 3 looks the tiles up
+    // ahead of the roles (two dependent loads and a few divisions are about a microsecond, which every role used to spend at
+    // each tile's start with the pipeline standing still) and leaves them in a ring. Tile counts fit 32 bits: 2^31 tiles
+    // would need activations of more than 2^43 bytes.
+    struct Tile { int row0, ncols, expert, mt; };
+    auto next_tile = [&](uint32_t n, Tile &tl) -> bool {            // single-lane roles: entry n of this CTA's sequence
+        const uint32_t i = n % kTileRing;
+        if (!mbar_wait(&sm->tile_full[i], (n / kTileRing) & 1u, abort)) return false;
+        const int4 v = sm->tile[i];
+        tl.row0 = v.x; tl.ncols = v.y; tl.expert = v.z; tl.mt = v.w;
+        mbar_arrive(&sm->tile_empty[i]);
+        return true;
     };
-    // Weight map and first tensor row of a tile. (Selects, not maps.w_routed[mat]: a dynamically
+    // Weight map of matrix `mat` and first tensor row of a tile. (Selects, not maps.w_routed[mat]: a dynamically
     // indexed parameter array makes the compiler copy the parameter block to local memory.)
-    auto weights_of = [&](const ColBlock &cb, int mat, int mt, int &y) {
-        const CUtensorMap *shared = mat ? &maps.w_shared[1] : &maps.w_shared[0], *routed = mat ? &maps.w_routed[1] : &maps.w_routed[0];
-        y = ((cb.expert < 0 ? 0 : cb.expert * p.M) + mt * kRowsPerMat) / p.fuse;
-        return cb.expert < 0 ? shared : routed;
+    auto weights_of = [&](const Tile &tl, int mat, int &y) {
+        y = ((tl.expert < 0 ? 0 : tl.expert * p.M) + tl.mt * kRowsPerMat) / p.fuse;
+        return mat ? (tl.expert < 0 ? &maps.w_shared[1] : &maps.w_routed[1]) : (tl.expert < 0 ? &maps.w_shared[0] : &maps.w_routed[0]);
     };
 
-    // Register budget per role (256-column tiles only: 28 warps leave 72 registers per thread, and the
-    // epilogue's 64 partial sums per thread do not fit in that): the control warps hand registers back
-    // and the epilogue warpgroups take them. Warps 0-3, 4-11 and 12+ are whole warpgroups.
-    {
-        static_assert(4 * Plan::kCtlRegs + kProducerWarps * Plan::kProdRegs + Plan::kEpilogueWarps * Plan::kEpiRegs <=
-                                           ((65536 / Plan::kThreads) & ~7) * (Plan::kThreads / 32),
-                      "the role budgets must fit in the registers the CTA was launched with, or the increase never returns");
-        constexpr int kLaunched = (65536 / Plan::kThreads) & ~7;
-        if (warp < 4) set_registers<Plan::kCtlRegs, kLaunched>();
-        else if (warp < 4 + kProducerWarps) set_registers<Plan::kProdRegs, kLaunched>();
-        else set_registers<Plan::kEpiRegs, kLaunched>();
-    }
+    const uint32_t my_tiles = tiles_total > blockIdx.x ? (tiles_total - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+
+    // Register budget per role: 28 warps leave 72 registers per thread, and the epilogue's 64 partial sums per thread
+    // do not fit in that: the control warps and producers hand registers back and the epilogue warpgroups take them.
+    // Warps 0-3, 4-11 and 12+ are whole warpgroups, and each sets its count as the first thing on its own branch, where
+    // the compiler can hold the role to it (behind a common if/else it allocated all roles for the launch's 72 and spilled).
+    constexpr int kLaunched = (65536 / Plan::kThreads) & ~7;
+    static_assert(4 * Plan::kCtlRegs + kProducerWarps * Plan::kProdRegs + Plan::kEpilogueWarps * Plan::kEpiRegs <= kLaunched * (Plan::kThreads / 32),
+                  "the role budgets must fit in the registers the CTA was launched with, or the increase never returns");
+    if (warp < 4) {
+    set_registers<Plan::kCtlRegs, kLaunched>();
     if (warp == 0) {
-        // ---------------- TMA producer: activation tiles ----------------
-        if (lane == 0) {
+        // ---------------- TMA producer: activation tiles (and the B' tiles of the min term) ----------------
+        if (elect_one()) {
             prefetch_tensormap(&maps.act);
-            // Raw weight superblocks run kRawStages - 1 ahead of the producers: one box per fused row
-            // r, [128 / fuse tensor rows] x [kBoxBytes from the 16-byte boundary at or below the block].
-            // (the fused form: the same from each of the two matrices, 64 / fuse tensor rows per box)
-            struct { long long t; int sb, y; uint32_t n; const CUtensorMap *map, *map2; } raw{(long long)blockIdx.x, 0, 0, 0u, nullptr, nullptr};
-            auto issue_raw = [&]() -> bool {
-                if (raw.t >= tiles_total) return true;
-                if (raw.sb == 0) {
-                    ColBlock cb; int mat, mt;
-                    tile_of(raw.t, cb, mat, mt);
-                    raw.map = weights_of(cb, mat, mt, raw.y);
-                    if constexpr (kFused) raw.map2 = weights_of(cb, 1, mt, raw.y);
-                }
-                const uint32_t s = raw.n % kRawStages, ph = (raw.n / kRawStages) & 1u;
-                if (!mbar_wait(&sm->raw_empty[s], ph ^ 1u, abort)) return false;
-                mbar_expect_tx(&sm->raw_full[s], Plan::kRawStageBytes);
-                const int rows = kRowsPerMat / p.fuse;
-                for (int r = 0; r < p.fuse; ++r) {
-                    const int x = (int)(r * p.row_bytes + raw.sb * Dec::kBlockBytes) & ~15;
-                    uint8_t *dst = raw_stage + s * Plan::kRawStageBytes + r * rows * Dec::kBoxBytes;
-                    tma_load_2d(dst, raw.map, x, raw.y, &sm->raw_full[s]);
-                    if constexpr (kFused) tma_load_2d(dst + kRowsPerMat * Dec::kBoxBytes, raw.map2, x, raw.y, &sm->raw_full[s]);
-                }
-                ++raw.n;
-                if (++raw.sb == nsb) { raw.sb = 0; raw.t += gridDim.x; }
-                return true;
-            };
+            if (kHasMin) prefetch_tensormap(&maps.sums);
+            if (Dec::kTableBytes && my_tiles) {
+                mbar_expect_tx(&sm->tab_full, Dec::kTableBytes);
+                bulk_load(tab, &gs::kIq2StreamTable, Dec::kTableBytes, &sm->tab_full);
+            }
+            RingAt b;
+            uint32_t sb_it = 0;
             bool ok = true;
-            for (int i = 0; i < kRawStages - 1 && ok; ++i) ok = issue_raw();
-            uint32_t it = 0;
-            for (long long t = blockIdx.x; t < tiles_total && !*abort && ok; t += gridDim.x) {
-                ColBlock cb; int mat, mt;
-                tile_of(t, cb, mat, mt);
-                const bool two = cb.ncols > kBoxN;             // a second 128-row box (only when kTileN = 256)
-                for (int kc = 0; kc < p.K / kChunkK; ++kc, ++it) {
-                    const uint32_t s = stage_of(it), ph = phase_of(it);
-                    if (!mbar_wait(&sm->empty[s], ph ^ 1u, abort)) { ok = false; break; }
-                    mbar_expect_tx(&sm->full[s], two ? 2 * kTileBytes : kTileBytes);
-                    tma_load_2d(b_tiles + s * kBTileBytes, &maps.act, kc * kChunkK, cb.row0, &sm->full[s]);
-                    if (two) tma_load_2d(b_tiles + s * kBTileBytes + kTileBytes, &maps.act, kc * kChunkK, cb.row0 + kBoxN, &sm->full[s]);
-                    // after the second chunk of a superblock: by then the producers have finished the
-                    // superblock before it, whose stage the next raw load reuses, so this wait is short
-                    if ((kc & 3) == 1 && !issue_raw()) { ok = false; break; }
-                }
-            }
-        }
-    } else if (warp < 3) {
-        // ---------------- MMA issuers ----------------
-        // Issuing is latency-bound in the issuing thread (barrier wait + four tcgen05.mma + commit cost
-        // more cycles than the MMAs execute), so two threads alternate superblocks: warp 1 fills TMEM
-        // buffer 0 with the even ones, warp 2 buffer 1 with the odd ones. The buffers are independent
-        // accumulators, so no ordering between the two instruction streams is needed.
-        if (lane == 0) {
-            const uint32_t mine = (uint32_t)(warp - 1);
-            const uint64_t adesc0 = smem_desc_sw128(smem_u32(a_tiles)), bdesc0 = smem_desc_sw128(smem_u32(b_tiles));
-            const uint64_t amin0 = smem_desc_sw128(smem_u32(min_tiles + mine * kTileBytes));
-            const uint64_t bmin0 = amin0 + 4;                  // parts 4..7 of the same rows (64 bytes along K)
-            uint32_t sb_it = 0;
-            for (long long t = blockIdx.x; t < tiles_total && !*abort; t += gridDim.x) {
-                ColBlock cb; int mat, mt;
-                tile_of(t, cb, mat, mt);
-                const uint32_t n = (uint32_t)((cb.ncols + 15) & ~15);
-                const uint32_t idesc = idesc_f16(n);
-                for (int sb = 0; sb < nsb; ++sb, ++sb_it) {
-                    if ((sb_it & 1u) != mine) continue;
-                    const uint32_t bph = (sb_it >> 1) & 1u;
-                    if (!mbar_wait(&sm->acc_empty[mine], bph ^ 1u, abort)) break;
-                    tc_fence_after();
+            uint32_t tn = 0;
+            Tile tl;
+            for (; tn < my_tiles && ok; ++tn) {
+                if (!next_tile(tn, tl)) break;
+                // boxes of 64 rows, the last one of 32 where that is enough: a ragged tile fetches what it needs
+                const int rem = tl.ncols & 63;
+                const uint32_t boxes = (uint32_t)(tl.ncols >> 6) + (rem > 32 ? 1u : 0u);
+                const bool tail = rem > 0 && rem <= 32;
+                for (int sb = 0; sb < nsb && ok; ++sb, ++sb_it) {
+#pragma unroll 1
                     for (int c = 0; c < 4; ++c) {
-                        const uint32_t it = 4u * sb_it + c, s = stage_of(it), ph = phase_of(it);
-                        if (!mbar_wait(&sm->full[s], ph, abort)) break;
-                        tc_fence_after();
-                        // descriptors differ from the stage-0 ones only in the start-address field (16-byte units)
-                        const uint64_t ad = adesc0 + (uint64_t)(s * (kTileBytes >> 4)), bd = bdesc0 + (uint64_t)(s * (kBTileBytes >> 4));
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            umma_f16(tmem + mine * kTileN, ad + 2 * k, bd + 2 * k, idesc, (c | k) ? 1u : 0u);
-                        umma_commit(&sm->empty[s]);
+                        if (!mbar_wait(&sm->b_empty[b.s], b.ph ^ 1u, abort)) { ok = false; break; }
+                        mbar_expect_tx(&sm->b_full[b.s], boxes * kBoxBytes + (tail ? kBoxBytes / 2 : 0u));
+                        const int x = (4 * sb + c) * kChunkK;
+                        uint8_t *dst = b_tiles + b.s * kBTileBytes;
+                        for (uint32_t i = 0; i < boxes; ++i) tma_load_2d(dst + i * kBoxBytes, &maps.act, x, tl.row0 + (int)(i * kBoxN), &sm->b_full[b.s]);
+                        if (tail) tma_load_2d(dst + boxes * kBoxBytes, &maps.act_tail, x, tl.row0 + (int)(boxes * kBoxN), &sm->b_full[b.s]);
+                        b.next<kBStages>();
                     }
-                    if (kHasMin) {
-                        if (!mbar_wait(&sm->min_full[mine], bph, abort)) break;
-                        tc_fence_after();
-#pragma unroll
-                        for (int k = 0; k < Dec::kMinSlots / 16; ++k)
-                            umma_f16(tmem + 2 * kTileN + mine * kTileN, amin0 + 2 * k, bmin0 + 2 * k, idesc, k ? 1u : 0u);
-                        umma_commit(&sm->min_empty[mine]);
+                    if (kHasMin && ok) {
+                        // (rows past the block's last one bring a neighbour's sums, past the last row of all zeros: columns never stored)
+                        const uint32_t buf = sb_it & 1u, bph = (sb_it >> 1) & 1u;
+                        if (!mbar_wait(&sm->min_empty[buf], bph ^ 1u, abort)) { ok = false; break; }
+                        mbar_expect_tx(&sm->min_full[buf], kMinTileBytes);
+                        tma_load_2d(min_b + buf * kMinTileBytes, &maps.sums, 32 * sb, tl.row0, &sm->min_full[buf]);
                     }
-                    umma_commit(&sm->acc_full[mine]);
                 }
             }
         }
-    } else if (warp < 4) {
-        // ---------------- B' tiles of the min term (affine qtypes only) ----------------
-        if (kHasMin) {
-            constexpr int kParts = kHasMin ? Dec::kMinSlots / 8 : 1, kRowsPerPass = 32 / kParts;
-            const int part = lane % kParts, rsub = lane / kParts;
+    } else if (warp == 1) {
+        // ---------------- MMA issuer ----------------
+        // One thread issues every MMA in chunk order; superblocks alternate between two TMEM accumulators.
+        if (elect_one()) {
+            const uint64_t bdesc0 = smem_desc_sw128(smem_u32(b_tiles));
+            const uint64_t amin0 = smem_desc_sw64(smem_u32(min_a)), bmin0 = smem_desc_sw64(smem_u32(min_b));
+            RingAt a, b;
             uint32_t sb_it = 0;
-            for (long long t = blockIdx.x; t < tiles_total && !*abort; t += gridDim.x) {
-                ColBlock cb; int mat, mt;
-                tile_of(t, cb, mat, mt);
-                for (int sb = 0; sb < nsb; ++sb, ++sb_it) {
-                    const uint32_t buf = sb_it & 1u, bph = (sb_it >> 1) & 1u;
-                    // this token row's sums for the superblock (zero rows past the block's tail), eight rows
-                    // per lane in flight together; the first eight are loaded before the wait for the tile
-                    constexpr int kPasses = kTileM / kRowsPerPass, kBatch = 8;
-                    uint8_t *tile = min_tiles + buf * kTileBytes;
+            bool ok = true;
+            uint32_t tn = 0;
+            Tile tl;
+            for (; tn < my_tiles && ok; ++tn) {
+                if (!next_tile(tn, tl)) break;
+                const uint32_t idesc = idesc_f16((uint32_t)((tl.ncols + 15) & ~15));
+                for (int sb = 0; sb < nsb && ok; ++sb, ++sb_it) {
+                    const uint32_t buf = sb_it & 1u, bph = (sb_it >> 1) & 1u, acc = tmem + buf * kTileN;
+                    if (!mbar_wait(&sm->acc_empty[buf], bph ^ 1u, abort)) { ok = false; break; }
+                    tc_fence_after();
+#pragma unroll 1
+                    for (int c = 0; c < 4; ++c) {
+                        if (!mbar_wait(&sm->b_full[b.s], b.ph, abort) || !mbar_wait(&sm->a_full[a.s], a.ph, abort)) { ok = false; break; }
+                        tc_fence_after();
+                        // descriptors differ from the stage-0 one only in the start-address field (16-byte units)
+                        const uint64_t bd = bdesc0 + (uint64_t)(b.s * (kBTileBytes >> 4));
+                        const uint32_t at = tmem + Plan::kACol + a.s * (kChunkK / 2);
 #pragma unroll
-                    for (int base = 0; base < kPasses; base += kBatch) {
-                        uint4 v[kBatch];
-#pragma unroll
-                        for (int i = 0; i < kBatch; ++i) {
-                            const int r = rsub + (base + i) * kRowsPerPass;
-                            const uint4 *src = reinterpret_cast<const uint4 *>(p.sums + ((uint64_t)(cb.row0 + r) * nsb + sb) * 32);
-                            v[i] = r < cb.ncols ? __ldg(src + part) : make_uint4(0, 0, 0, 0);
-                        }
-                        if (base == 0 && !mbar_wait_warp(&sm->min_empty[buf], bph ^ 1u, abort)) goto done;
-#pragma unroll
-                        for (int i = 0; i < kBatch; ++i)
-                            *reinterpret_cast<uint4 *>(tile + sw128_offset(rsub + (base + i) * kRowsPerPass, 4 + part)) = v[i];
+                        for (int k = 0; k < 4; ++k) umma_f16_ts(acc, at + 8 * k, bd + 2 * k, idesc, (c | k) ? 1u : 0u);
+                        umma_commit(&sm->a_empty[a.s]);
+                        umma_commit(&sm->b_empty[b.s]);
+                        a.next<kAStages>();
+                        b.next<kBStages>();
                     }
-                    fence_proxy_async();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&sm->min_full[buf]);
+                    if (!ok) break;
+                    if (kHasMin) {
+                        // there is one min-term accumulator: the superblock before must have been drained
+                        if (sb_it && !mbar_wait(&sm->acc_empty[buf ^ 1u], ((sb_it - 1u) >> 1) & 1u, abort)) { ok = false; break; }
+                        if (!mbar_wait(&sm->min_full[buf], bph, abort)) { ok = false; break; }
+                        tc_fence_after();
+                        const uint64_t ad = amin0 + (uint64_t)(buf * (kMinTileBytes >> 4)), bd = bmin0 + (uint64_t)(buf * (kMinTileBytes >> 4));
+#pragma unroll
+                        for (int k = 0; k < Dec::kMinSlots / 16; ++k) umma_f16(tmem + Plan::kMinCol, ad + 2 * k, bd + 2 * k, idesc, k ? 1u : 0u);
+                        umma_commit(&sm->min_empty[buf]);
+                    }
+                    umma_commit(&sm->acc_full[buf]);
                 }
             }
         }
+    } else if (warp == 2) {
+        // ---------------- TMA producer: raw weight superblocks ----------------
+        // One box per fused row r, [rows / fuse tensor rows] x [kBoxBytes from the 16-byte boundary at or below the block]
+        // (the fused form: the same from each of the two matrices), up to kRawStages superblocks ahead of the producers.
+        if (elect_one()) {
+            uint32_t n = 0;
+            bool ok = true;
+            uint32_t tn = 0;
+            Tile tl;
+            for (; tn < my_tiles && ok; ++tn) {
+                if (!next_tile(tn, tl)) break;
+                int y;
+                const CUtensorMap *map = weights_of(tl, 0, y), *map2 = kFused ? weights_of(tl, 1, y) : nullptr;
+                for (int sb = 0; sb < nsb && ok; ++sb, ++n) {
+                    const uint32_t s = n % kRawStages, ph = (n / kRawStages) & 1u;
+                    if (!mbar_wait(&sm->raw_empty[s], ph ^ 1u, abort)) { ok = false; break; }
+                    mbar_expect_tx(&sm->raw_full[s], Plan::kRawStageBytes);
+                    const int rows = kRowsPerMat / p.fuse;
+                    for (int r = 0; r < p.fuse; ++r) {
+                        const int x = (int)(r * p.row_bytes + sb * Dec::kBlockBytes) & ~15;
+                        uint8_t *dst = raw_stage + s * Plan::kRawStageBytes + r * rows * Dec::kBoxBytes;
+                        tma_load_2d(dst, map, x, y, &sm->raw_full[s]);
+                        if constexpr (kFused) tma_load_2d(dst + kRowsPerMat * Dec::kBoxBytes, map2, x, y, &sm->raw_full[s]);
+                    }
+                }
+            }
+        }
+    } else if (elect_one()) {
+        // ---------------- warp 3: tile look-ups ----------------
+        for (uint32_t n = 0; n < my_tiles; ++n) {
+            const uint32_t t = blockIdx.x + n * gridDim.x, i = n % kTileRing;
+            const ColBlock *g0 = p.colblocks + t / (uint32_t)mtiles;    // any block of the group names the group
+            const uint32_t first = (uint32_t)g0->first, count = (uint32_t)g0->count;
+            const uint32_t local = t - first * (uint32_t)mtiles, mt = local / count;
+            const ColBlock *cb = p.colblocks + first + (local - mt * count);
+            const int4 v = make_int4(cb->row0, cb->ncols, cb->expert, (int)mt);
+            if (!mbar_wait(&sm->tile_empty[i], ((n / kTileRing) & 1u) ^ 1u, abort)) break;
+            sm->tile[i] = v;
+            mbar_arrive(&sm->tile_full[i]);
+        }
+    }
     } else if (warp < 4 + kProducerWarps) {
+        set_registers<Plan::kProdRegs, kLaunched>();
+        if (Dec::kTableBytes && my_tiles && !mbar_wait_warp(&sm->tab_full, 0u, abort)) goto done;
         // ---------------- dequant producers ----------------
-        const int pw = warp - 4, rl = lane % kRowsPerWarp, h = lane / kRowsPerWarp;     // h: this thread's part of a chunk
-        const uint32_t row = (uint32_t)(kRowsPerWarp * pw + rl);
+        // warps w and w + 4 own the 32 TMEM lanes (A rows) of w % 4: thread = (row, 32-weight half of a 64-K chunk)
+        const int h = (warp - 4) >> 2;
+        const uint32_t row = (uint32_t)(32 * (warp & 3) + lane);
+        const uint32_t a_at = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + Plan::kACol + 16u * (uint32_t)h, lane4 = 4u * (uint32_t)lane;
+        RingAt a;
         // where the row's bytes land in a raw stage, and where its superblock 0 starts in the tensor row
         // (fused form: tile row 2i is row i of the first matrix, 2i + 1 row i of the second, whose boxes follow)
         const uint32_t wrow = kFused ? row >> 1 : row, wmat = kFused ? row & 1u : 0u;
         const uint32_t sub = wrow % (uint32_t)p.fuse;
         const uint32_t slot = ((wmat * (uint32_t)p.fuse + sub) * (uint32_t)(kRowsPerMat / p.fuse) + wrow / (uint32_t)p.fuse) * Dec::kBoxBytes;
         const uint32_t x_row = sub * p.row_bytes;
-        const long long my_tiles = tiles_total > blockIdx.x ? (tiles_total - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
         uint32_t sb_it = 0;
-        for (long long tile = 0; tile < my_tiles && !*abort; ++tile) {
+        for (uint32_t tile = 0; tile < my_tiles && !*abort; ++tile) {
             for (int sb = 0; sb < nsb; ++sb, ++sb_it) {
                 const uint32_t rs = sb_it % kRawStages, rph = (sb_it / kRawStages) & 1u;
                 if (!mbar_wait_warp(&sm->raw_full[rs], rph, abort)) goto done;
-                const uint32_t off = (x_row + (uint32_t)sb * Dec::kBlockBytes) & 15u, mis = off & 3u;
-                const uint32_t *raw = reinterpret_cast<const uint32_t *>(raw_stage + rs * Plan::kRawStageBytes + slot + (off & ~3u));
+                typename Dec::Block blk;
+                Dec::open(raw_stage + rs * Plan::kRawStageBytes + slot, (x_row + (uint32_t)sb * Dec::kBlockBytes) & 15u, blk);
                 if (h == 0) {
                     bool bad;
-                    const float2 dd = Dec::scales(raw, mis, bad);
+                    const float2 dd = Dec::scales(blk, bad);
                     if constexpr (kHasMin) dscale[(sb_it % kScaleRing) * kTileM + row] = dd;
                     else dscale[(sb_it % kScaleRing) * kTileM + row] = dd.x;
                     if (bad) raise(p.status, YVEX_B200_STATUS_NUMERIC);
                 }
+                // a chunk's words and table entries are read before the wait for its stage
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    const uint32_t it = 4u * sb_it + c, s = stage_of(it), ph = phase_of(it);
-                    if (!mbar_wait_warp(&sm->empty[s], ph ^ 1u, abort)) goto done;
+                    typename Dec::Half half;
+                    Dec::fetch(blk, c, h, tab, lane4, half);
+                    if (!mbar_wait_warp(&sm->a_empty[a.s], a.ph ^ 1u, abort)) goto done;
+                    tc_fence_after();
 #pragma unroll
-                    for (int q = 0; q < Plan::kPartsPerThread; ++q)
-                        Dec::store(raw, mis, c, h * Plan::kPartsPerThread + q, a_tiles + s * kTileBytes, row, tab);
-                    fence_proxy_async();
+                    for (int q = 0; q < 2; ++q) {
+                        uint32_t v[8];
+                        Dec::convert(half, q, v);
+                        tmem_st8(a_at + a.s * (kChunkK / 2) + 8u * (uint32_t)q, v);
+                    }
+                    tmem_st_wait();
+                    tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&sm->full[s]);
+                    if (lane == 0) mbar_arrive(&sm->a_full[a.s]);
+                    a.next<kAStages>();
                 }
                 if (kHasMin) {
                     const uint32_t buf = sb_it & 1u, bph = (sb_it >> 1) & 1u;
                     if (!mbar_wait_warp(&sm->min_empty[buf], bph ^ 1u, abort)) goto done;
-                    if (h < 2) Dec::mins(raw, h, min_tiles + buf * kTileBytes, row);
+                    Dec::mins(blk, h, min_a + buf * kMinTileBytes, row);
                     fence_proxy_async();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&sm->min_full[buf]);
@@ -538,14 +584,23 @@ moe_grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, GemmParams p) {
         }
     } else {
         // ---------------- epilogue ----------------
+        set_registers<Plan::kEpiRegs, kLaunched>();
         constexpr int kCols = Plan::kColsPerWarp;
         const int ew = warp - (4 + kProducerWarps), quarter = warp & 3, colhalf = ew >> 2;     // TMEM lanes 32*quarter.., columns kCols*colhalf..
         const int row = 32 * quarter + lane;
         const uint32_t lane_addr = (uint32_t)(32 * quarter) << 16;
         uint32_t sb_it = 0;
-        for (long long t = blockIdx.x; t < tiles_total && !*abort; t += gridDim.x) {
-            ColBlock cb; int mat, mt;
-            tile_of(t, cb, mat, mt);
+        for (uint32_t tn = 0; tn < my_tiles && !*abort; ++tn) {
+            Tile cb;
+            {
+                const uint32_t i = tn % kTileRing;
+                if (!mbar_wait_warp(&sm->tile_full[i], (tn / kTileRing) & 1u, abort)) goto done;
+                const int4 v = sm->tile[i];
+                cb.row0 = v.x; cb.ncols = v.y; cb.mt = v.w;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sm->tile_empty[i]);
+            }
+            const int mt = cb.mt;
             float acc[kCols];
 #pragma unroll
             for (int i = 0; i < kCols; ++i) acc[i] = 0.0f;
@@ -577,12 +632,12 @@ moe_grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, GemmParams p) {
                         tmem_ld16(tmem + lane_addr + buf * kTileN + kCols * colhalf + 16 * q, v);
                         tmem_ld_wait();
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) acc[16 * q + i] = fmaf(d, __uint_as_float(v[i]), acc[16 * q + i]);
+                        for (int i = 0; i < 16; i += 2) fma2(acc[16 * q + i], acc[16 * q + i + 1], d, v[i], v[i + 1]);
                         if (kHasMin) {
-                            tmem_ld16(tmem + lane_addr + 2 * kTileN + buf * kTileN + kCols * colhalf + 16 * q, v);
+                            tmem_ld16(tmem + lane_addr + Plan::kMinCol + kCols * colhalf + 16 * q, v);
                             tmem_ld_wait();
 #pragma unroll
-                            for (int i = 0; i < 16; ++i) acc[16 * q + i] = fmaf(-dmin, __uint_as_float(v[i]), acc[16 * q + i]);
+                            for (int i = 0; i < 16; i += 2) fma2(acc[16 * q + i], acc[16 * q + i + 1], -dmin, v[i], v[i + 1]);
                         }
                     }
                 }
@@ -590,11 +645,12 @@ moe_grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, GemmParams p) {
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&sm->acc_empty[buf]);
             }
+            if (ncols_here <= 0) continue;                      // no real column: nothing to store
             // non-finite sums are refused: x * 0 is zero for finite x and NaN otherwise
-            float poison = 0.0f;
+            float poison = 0.0f, poison2 = 0.0f;
 #pragma unroll
-            for (int i = 0; i < kCols; ++i) poison = fmaf(acc[i], 0.0f, poison);
-            if (poison != poison) raise(p.status, YVEX_B200_STATUS_NUMERIC);
+            for (int i = 0; i < kCols; i += 2) fma2(poison, poison2, 0.0f, __float_as_uint(acc[i]), __float_as_uint(acc[i + 1]));
+            if (poison != poison || poison2 != poison2) raise(p.status, YVEX_B200_STATUS_NUMERIC);
             if constexpr (kFused) {
                 // Even lanes hold the gate row of intermediate i = row / 2, odd lanes its up row. A pair of
                 // lanes swaps every other column, so the even lane ends up with gate and up of the even
@@ -610,47 +666,51 @@ moe_grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, GemmParams p) {
                 const bool odd = lane & 1, o2 = lane & 2, o4 = lane & 4;
                 const int rr = (lane >> 1) & 3;
                 const uint64_t m0 = (uint64_t)mt * kRowsPerMat + 16 * quarter + 4 * (lane >> 3);
+                bool bad = false;
+                // (32 columns, sixteen swaps, at a time: steps without a real column are left out)
 #pragma unroll
-                for (int m = 0; m < kCols / 2; ++m) {               // acc[2m] = gate, acc[2m + 1] = up of column 2m + parity
-                    const float keep = odd ? acc[2 * m + 1] : acc[2 * m];
-                    const float got = __shfl_xor_sync(0xffffffffu, odd ? acc[2 * m] : acc[2 * m + 1], 1);
-                    acc[2 * m] = odd ? got : keep;
-                    acc[2 * m + 1] = odd ? keep : got;
-                }
+                for (int c0 = 0; c0 < kCols; c0 += 32) {
+                    if (c0 >= ncols_here) break;
+                    float *g = acc + c0;
 #pragma unroll
-                for (int m = 0; m < kCols / 2; ++m)                 // acc[m] = silu(gate) * up
-                    acc[m] = swiglu_product(acc[2 * m], acc[2 * m + 1], 1.0f, p.limit);
-                float wv[kCols / 8];                                // route weight of column 8b + 2rr + parity
+                    for (int m = 0; m < 16; ++m) {                      // g[2m] = gate, g[2m + 1] = up of column c0 + 2m + parity
+                        const float keep = odd ? g[2 * m + 1] : g[2 * m];
+                        const float got = __shfl_xor_sync(0xffffffffu, odd ? g[2 * m] : g[2 * m + 1], 1);
+                        g[2 * m] = odd ? got : keep;
+                        g[2 * m + 1] = odd ? keep : got;
+                    }
+                    const float wl = c0 ? w_hi : w_lo;
+                    float wv[4];                                        // route weight of column c0 + 8b + 2rr + parity
 #pragma unroll
-                for (int b = 0; b < kCols / 8; ++b) wv[b] = __shfl_sync(0xffffffffu, b < 4 ? w_lo : w_hi, (8 * b + 2 * rr + (odd ? 1 : 0)) & 31);
+                    for (int b = 0; b < 4; ++b) wv[b] = __shfl_sync(0xffffffffu, wl, 8 * b + 2 * rr + (odd ? 1 : 0));
 #pragma unroll
-                for (int b0 = 0; b0 < kCols / 8; b0 += 4) {           // four blocks (eight shuffles) per round
+                    for (int m = 0; m < 16; ++m)                        // g[m] = silu(gate) * up
+                        g[m] = swiglu_product_bounded(g[2 * m], g[2 * m + 1], p.limit);
 #pragma unroll
-                    for (int b = b0; b < b0 + 4; ++b) {
-                        float *r = acc + 4 * b;
+                    for (int b = 0; b < 4; ++b) {
+                        float *r = g + 4 * b;
                         const float s0 = __shfl_xor_sync(0xffffffffu, o2 ? r[0] : r[1], 2), s1 = __shfl_xor_sync(0xffffffffu, o2 ? r[2] : r[3], 2);
                         if (o2) { r[0] = s0; r[2] = s1; } else { r[1] = s0; r[3] = s1; }
                     }
 #pragma unroll
-                    for (int b = b0; b < b0 + 4; ++b) {
-                        float *r = acc + 4 * b;
+                    for (int b = 0; b < 4; ++b) {
+                        float *r = g + 4 * b;
                         const float s0 = __shfl_xor_sync(0xffffffffu, o4 ? r[0] : r[2], 4), s1 = __shfl_xor_sync(0xffffffffu, o4 ? r[1] : r[3], 4);
                         if (o4) { r[0] = s0; r[1] = s1; } else { r[2] = s0; r[3] = s1; }
                     }
-                }
-                bool bad = false;
 #pragma unroll
-                for (int b = 0; b < kCols / 8; ++b) {
-                    const int col = 8 * b + 2 * rr + (odd ? 1 : 0);
-                    if (col < ncols_here) {
-                        const uint64_t srow = (uint64_t)cb.row0 + kCols * colhalf + col;
-                        const float r0 = acc[4 * b] * wv[b], r1 = acc[4 * b + 1] * wv[b], r2 = acc[4 * b + 2] * wv[b], r3 = acc[4 * b + 3] * wv[b];
-                        bad |= !isfinite(r0) || !isfinite(r1) || !isfinite(r2) || !isfinite(r3);
-                        // f32 -> bf16 (round to nearest even; the product is finite or the launch is refused) -> the same values as fp16
-                        const __nv_bfloat162 b01 = __floats2bfloat162_rn(r0, r1), b23 = __floats2bfloat162_rn(r2, r3);
-                        const __half2 h01 = __float22half2_rn(__bfloat1622float2(b01)), h23 = __float22half2_rn(__bfloat1622float2(b23));
-                        *reinterpret_cast<uint2 *>(p.mid + srow * p.M + m0) =
-                            make_uint2(*reinterpret_cast<const uint32_t *>(&h01), *reinterpret_cast<const uint32_t *>(&h23));
+                    for (int b = 0; b < 4; ++b) {
+                        const int col = c0 + 8 * b + 2 * rr + (odd ? 1 : 0);
+                        if (col < ncols_here) {
+                            const uint64_t srow = (uint64_t)cb.row0 + kCols * colhalf + col;
+                            const float r0 = g[4 * b] * wv[b], r1 = g[4 * b + 1] * wv[b], r2 = g[4 * b + 2] * wv[b], r3 = g[4 * b + 3] * wv[b];
+                            bad |= !isfinite(r0) || !isfinite(r1) || !isfinite(r2) || !isfinite(r3);
+                            // f32 -> bf16 (round to nearest even; the product is finite or the launch is refused) -> the same values as fp16
+                            const __nv_bfloat162 b01 = __floats2bfloat162_rn(r0, r1), b23 = __floats2bfloat162_rn(r2, r3);
+                            const __half2 h01 = __float22half2_rn(__bfloat1622float2(b01)), h23 = __float22half2_rn(__bfloat1622float2(b23));
+                            *reinterpret_cast<uint2 *>(p.mid + srow * p.M + m0) =
+                                make_uint2(*reinterpret_cast<const uint32_t *>(&h01), *reinterpret_cast<const uint32_t *>(&h23));
+                        }
                     }
                 }
                 if (bad) raise(p.status, YVEX_B200_STATUS_NUMERIC);
@@ -688,9 +748,10 @@ moe_grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, GemmParams p) {
                         else dst = p.out_bf16 + (p.out_rows ? (uint64_t)__ldg(p.out_rows + srow) : srow) * p.M;
                         // streaming stores: the results are not read again by this kernel and must not push the
                         // activation tiles and weight rows that other CTAs are about to reuse out of L2
-                        const uint2 v = make_uint2(bf16_bits(acc[4 * b]) | ((uint32_t)bf16_bits(acc[4 * b + 1]) << 16),
-                                                   bf16_bits(acc[4 * b + 2]) | ((uint32_t)bf16_bits(acc[4 * b + 3]) << 16));
-                        if (dst) __stcs(reinterpret_cast<uint2 *>(dst + m0), v);
+                        // (round to nearest even; a launch with a non-finite sum is refused)
+                        const __nv_bfloat162 lo = __floats2bfloat162_rn(acc[4 * b], acc[4 * b + 1]), hi2 = __floats2bfloat162_rn(acc[4 * b + 2], acc[4 * b + 3]);
+                        if (dst) __stcs(reinterpret_cast<uint2 *>(dst + m0),
+                                        make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi2)));
                     }
                 }
             }

@@ -76,11 +76,14 @@ __global__ void wide_plan_kernel(const int *counts, int experts, uint64_t pairs,
         const int row0 = off + row_end - count, blk0 = nb + blk_end - nblocks;
         if (e <= experts) {
             if (blockIdx.x == 0) offsets[e] = row0;
+            // an expert's rows in blocks of equal width (rounded up to the MMA's 16 columns): the tensor time follows the width,
+            // while a full block beside a nearly empty one would decode the same weights for both
+            const int width = nblocks ? ((count + nblocks - 1) / nblocks + 15) & ~15 : 0;
             for (int b = 0; b < nblocks; ++b) {
                 const int first = blk0 + b - b % per_group;
                 const int in_group = min(per_group, nblocks - (b - b % per_group));
                 if (blk0 + b < max_blocks)
-                    blocks[blk0 + b] = ColBlock{row0 + b * tile_n, min(tile_n, count - b * tile_n), e < experts ? e : -1, first, in_group, 0};
+                    blocks[blk0 + b] = ColBlock{row0 + b * width, min(width, count - b * width), e < experts ? e : -1, first, in_group, 0};
             }
         }
         off += __shfl_sync(0xffffffffu, row_end, 31);
@@ -298,7 +301,7 @@ static uint64_t pair_layout(const MoeGeom &g, uint64_t pairs, uint64_t base_off,
     uint64_t off = base_off;
     auto take = [&](uint64_t bytes) { uint64_t at = off; off = (off + bytes + 255) & ~255ull; return at; };
     PairWorkspace l{};
-    l.max_blocks = (int)(pairs / kBoxN + g.experts + 2);
+    l.max_blocks = (int)(pairs / kMinTileN + g.experts + 2);
     l.counts = reinterpret_cast<int *>(take((g.experts + 2) * 4));
     l.offsets = reinterpret_cast<int *>(take((g.experts + 3) * 4));
     l.num_blocks = reinterpret_cast<int *>(take(8));
@@ -336,15 +339,27 @@ static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
     return fn;
 }
 
-// Row-major fp16 [rows][width] -> boxes of [kBoxN rows][64 columns], 128-byte swizzle, zero fill.
+// Row-major fp16 [rows][width] -> boxes of [box_rows rows][64 columns], 128-byte swizzle, zero fill.
 // (pitch_bytes: distance between rows when they are not packed, a multiple of 16; 0 = packed)
-static int make_act_map(CUtensorMap *map, const __half *base, uint64_t rows, uint64_t width, uint64_t pitch_bytes = 0) {
+static int make_act_map(CUtensorMap *map, const __half *base, uint64_t rows, uint64_t width, int box_rows, uint64_t pitch_bytes = 0) {
     auto fn = encode_fn();
     if (!fn) return ERR_BACKEND;
     cuuint64_t dims[2] = {width, rows}, strides[1] = {pitch_bytes ? pitch_bytes : width * 2};
-    cuuint32_t box[2] = {kChunkK, kBoxN}, estr[2] = {1, 1};
+    cuuint32_t box[2] = {kChunkK, (cuuint32_t)box_rows}, estr[2] = {1, 1};
     CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half *>(base), dims, strides, box, estr,
                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? OK : ERR_BACKEND;
+}
+
+// Sub-block sums [rows][supers][32] fp16 -> boxes of one superblock's 32 sums of 128 rows, 64-byte swizzle, zero fill.
+static int make_sums_map(CUtensorMap *map, const __half *base, uint64_t rows, uint64_t supers) {
+    auto fn = encode_fn();
+    if (!fn) return ERR_BACKEND;
+    cuuint64_t dims[2] = {supers * 32, rows}, strides[1] = {supers * 64};
+    cuuint32_t box[2] = {32, kMinTileN}, estr[2] = {1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half *>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? OK : ERR_BACKEND;
 }
@@ -359,7 +374,7 @@ static int make_weight_map(CUtensorMap *map, const void *base, uint64_t rows, ui
     cuuint64_t dims[2] = {fuse * row_bytes, rows / fuse}, strides[1] = {fuse * row_bytes};
     cuuint32_t box[2] = {box_bytes, (cuuint32_t)(box_rows / fuse)}, estr[2] = {1, 1};
     CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(base), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? OK : ERR_BACKEND;
 }
@@ -414,7 +429,7 @@ static int run_gemm(unsigned qtype, bool fused, const GemmMaps &map, const GemmP
 }
 
 static bool gemm_qtype(unsigned q) { return q == Q_IQ2_XXS || q == Q_Q4_K || q == Q_Q2_K; }
-// Token columns per GEMM tile: 256 unless the qtype's min term needs the second accumulator.
+// Most token columns of a GEMM tile: what tensor memory has room for beside the A ring and the min term's accumulator.
 static int gemm_tile_n(unsigned q) { return q == Q_IQ2_XXS ? GemmPlan<GemmIq2>::kTileN : q == Q_Q4_K ? GemmPlan<GemmQ4k>::kTileN : GemmPlan<GemmQ2k>::kTileN; }
 
 bool moe_wide_gemm_eligible(const MoeGeom &g, const MoeWeights &w) {
@@ -470,19 +485,21 @@ static int run_sorted_gemms(const MoeGeom &g, const MoeWeights &w, const PairWor
     const auto sum_group = [](unsigned q) { return q == Q_Q4_K ? 32 : q == Q_Q2_K ? 16 : 0; };
     int rc;
     GemmMaps gu_maps, dn_maps;
-    if (make_act_map(&gu_maps.act, act, pairs, g.hidden, act_pitch) != OK || make_act_map(&dn_maps.act, pw.mid_h, pairs, g.inter) != OK)
+    if (make_act_map(&gu_maps.act, act, pairs, g.hidden, kBoxN, act_pitch) != OK || make_act_map(&gu_maps.act_tail, act, pairs, g.hidden, kBoxN / 2, act_pitch) != OK ||
+        make_act_map(&dn_maps.act, pw.mid_h, pairs, g.inter, kBoxN) != OK || make_act_map(&dn_maps.act_tail, pw.mid_h, pairs, g.inter, kBoxN / 2) != OK ||
+        make_sums_map(&gu_maps.sums, pw.act_sums, pairs, g.hidden / 256) != OK || make_sums_map(&dn_maps.sums, pw.sums, pairs, g.inter / 256) != OK)
         return ERR_BACKEND;
     GemmParams gu{};
     gu.row_bytes = (uint32_t)(g.hidden / gg.elems * gg.bytes);
     gu.fuse = fuse_of(gu.row_bytes);
-    gu.M = (int)g.inter; gu.K = (int)g.hidden; gu.nmat = 1;              // one fused pass over both matrices
+    gu.M = (int)g.inter; gu.K = (int)g.hidden;                            // one fused pass over both matrices
     {
         const void *routed[2] = {w.gate, w.up}, *shared[2] = {w.shared_gate, w.shared_up};
         rc = make_weight_maps(&gu_maps, g.gate_qtype, routed, shared, 2, (uint64_t)g.experts * g.inter, g.inter, gu);
         if (rc != OK) return rc;
     }
     gu.colblocks = pw.blocks; gu.num_colblocks = pw.num_blocks;
-    gu.mid = pw.mid_h; gu.col_weight = pw.weight_sorted; gu.limit = (float)g.limit; gu.out_bf16 = nullptr; gu.sums = pw.act_sums;
+    gu.mid = pw.mid_h; gu.col_weight = pw.weight_sorted; gu.limit = (float)g.limit; gu.out_bf16 = nullptr;
     gu.status = status;
     rc = run_gemm(g.gate_qtype, true, gu_maps, gu, s);
     if (rc != OK) return rc;
@@ -495,14 +512,14 @@ static int run_sorted_gemms(const MoeGeom &g, const MoeWeights &w, const PairWor
     GemmParams dn{};
     dn.row_bytes = (uint32_t)(g.inter / dg.elems * dg.bytes);
     dn.fuse = fuse_of(dn.row_bytes);
-    dn.M = (int)g.hidden; dn.K = (int)g.inter; dn.nmat = 1;
+    dn.M = (int)g.hidden; dn.K = (int)g.inter;
     {
         const void *routed[2] = {w.down, nullptr}, *shared[2] = {w.shared_down, nullptr};
         rc = make_weight_maps(&dn_maps, g.down_qtype, routed, shared, 1, (uint64_t)g.experts * g.hidden, g.hidden, dn);
         if (rc != OK) return rc;
     }
     dn.colblocks = pw.blocks_down; dn.num_colblocks = pw.num_blocks + 1;
-    dn.out_bf16 = y; dn.out_rows = out_rows; dn.sums = pw.sums; dn.status = status;
+    dn.out_bf16 = y; dn.out_rows = out_rows; dn.status = status;
     dn.out_addr = out_addr;
     rc = run_gemm(g.down_qtype, false, dn_maps, dn, s);
     if (rc != OK) return rc;
@@ -571,7 +588,10 @@ extern "C" int yvex_b200_moe_wide_uses_gemm(const yvex_b200_moe_geometry *g, con
     return g && w && moe_check_geometry(g, w) == OK && moe_wide_gemm_eligible(*g, *w) ? 1 : 0;
 }
 
-extern "C" uint64_t yvex_b200_moe_wide_tile_columns(unsigned int qtype) { return gemm_qtype(qtype) ? (uint64_t)gemm_tile_n(qtype) : 0; }
+extern "C" uint64_t yvex_b200_moe_wide_tile_columns(unsigned int qtype) {
+    // the width the worklist counts its tails in; a tile takes at most as many columns (224 or 128, in blocks of equal width)
+    return gemm_qtype(qtype) ? qtype == Q_IQ2_XXS ? 256 : 128 : 0;
+}
 
 extern "C" uint64_t yvex_b200_moe_wide_workspace_bytes(const yvex_b200_moe_geometry *g, uint64_t rows) {
     return g ? moe_wide_workspace_bytes(*g, rows) : 0;
