@@ -515,3 +515,21 @@ def test_gqa_decode_slices_and_block_edges(L, dim, group, sessions, kv, visible,
     assert rel_l2(out.cpu().numpy(), want.cpu().numpy()) <= 1e-5
     need = [int(L.lib.yvex_b200_attention_workspace_bytes(sessions, kv * group, kv, dim, c)) for c in range(1, context + 1)]
     assert all(a <= b for a, b in zip(need, need[1:]))
+
+
+@pytest.mark.parametrize("qtype", [synth.F32, synth.F16, synth.BF16])
+@pytest.mark.parametrize("rows,width,inputs", [(2048, 256, 2), (2051, 1000, 3), (2050, 512, 8), (9473, 264, 9), (2049, 8192, 17), (2048, 16, 4)])
+def test_gemv_scalar_qtypes_several_inputs(L, qtype, rows, width, inputs):
+    """Four matrix rows per warp and two, four or eight inputs per pass: ragged rows, widths below a warp's chunk and a width
+    whose eight rows do not fit beside each other, against 64 bits (f32 sums of `width` products: 1e-6), with an additive row."""
+    import torch
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(rows + inputs)
+    w = torch.randn((rows, width), device="cuda", generator=gen).to({synth.F32: torch.float32, synth.F16: torch.float16, synth.BF16: torch.bfloat16}[qtype])
+    x, st = torch.randn((inputs, width), device="cuda", generator=gen), L.Status()
+    y = L.gemv(qtype, w.view(torch.uint8).reshape(-1), rows, width, x, st)
+    assert st.read() == 0
+    assert rel_l2(y.cpu().numpy(), (x.double() @ w.double().T).cpu().numpy()) <= 1e-6
+    x[inputs - 1, width - 1] = float("inf")
+    L.gemv(qtype, w.view(torch.uint8).reshape(-1), rows, width, x, st)
+    assert st.read() == 1
