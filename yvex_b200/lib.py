@@ -127,11 +127,18 @@ EXPORTS = ["yvex_b200_version", "yvex_b200_qtype_supported", "yvex_b200_qtype_ge
            "yvex_b200_moe_expert_rows_sorted"]
 
 
+_module = None
+
+
 def _torch():
-    import torch
-    if not torch.cuda.is_available():
-        raise RuntimeError("yvex_b200 compute entry points need a CUDA device; there is no CPU fallback")
-    return torch
+    """torch, once a CUDA device has been seen (asking the driver again on every call costs as much as a kernel launch)."""
+    global _module
+    if _module is None:
+        import torch
+        if not torch.cuda.is_available():
+            raise RuntimeError("yvex_b200 compute entry points need a CUDA device; there is no CPU fallback")
+        _module = torch
+    return _module
 
 
 def _p(t):
@@ -139,8 +146,9 @@ def _p(t):
 
 
 def _stream():
-    import torch
-    return torch.cuda.current_stream().cuda_stream
+    """Raw handle of the current device's current stream (without the stream object that current_stream() builds: 3.3 us a call)."""
+    torch = _torch()
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _check(rc, where):
@@ -192,7 +200,7 @@ def dequant_rows(qtype, enc, rows, width, status):
 
 def gemv(qtype, enc, rows, width, x, status, additive=None, round_bf16=False, out=None, row_bytes=None):
     torch = _torch()
-    x2 = x.reshape(-1, width)
+    x2 = x if x.dim() == 2 and x.shape[1] == width else x.reshape(-1, width)
     if out is None:
         out = torch.empty((x2.shape[0], rows), dtype=torch.float32, device=x.device)
     rb = row_bytes if row_bytes is not None else enc.numel() // rows
