@@ -533,3 +533,18 @@ def test_gemv_scalar_qtypes_several_inputs(L, qtype, rows, width, inputs):
     x[inputs - 1, width - 1] = float("inf")
     L.gemv(qtype, w.view(torch.uint8).reshape(-1), rows, width, x, st)
     assert st.read() == 1
+
+
+@pytest.mark.parametrize("rows,width,inputs", [(2048, 7168, 1), (8, 8192, 1), (13, 6912, 2), (1, 7936, 5), (149 * 8 + 3, 8192, 1)])
+def test_gemv_q8_0_long_rows(L, rows, width, inputs):
+    """Rows of which sixteen leave no room for a second stage go in groups of eight: ragged tiles, padded and plain pitches,
+    several inputs, against 64 bits (the activation is held to 28 bits: 1e-6)."""
+    import torch
+    raw = synth.random_blocks(synth.Q8_0, rows, width, rows)
+    blocks = raw.reshape(rows, -1, 34)
+    w = blocks[:, :, :2].copy().view(np.float16).astype(np.float64) * blocks[:, :, 2:].copy().view(np.int8)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(width)
+    x, st = torch.randn((inputs, width), device="cuda", generator=gen), L.Status()
+    y = L.gemv(synth.Q8_0, dev(raw), rows, width, x, st)
+    assert st.read() == 0 and rel_l2(y.cpu().numpy(), x.cpu().numpy().astype(np.float64) @ w.reshape(rows, width).T) <= 1e-6

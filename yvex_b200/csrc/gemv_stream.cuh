@@ -499,7 +499,8 @@ struct TaskCursor {
 
 // kBReg: the warp's whole K-slice is one unit, so its B fragments live in registers from one matrix change to the next.
 // kGroupsPerWarp: 16-row groups a consumer warp decodes per stage.
-template <class Dec, bool kBReg, int kGroupsPerWarp>
+// kRows: matrix rows in one MMA group: 16, or 8 where sixteen rows are too long for a ring (row g + 8 of a fragment then repeats row g).
+template <class Dec, bool kBReg, int kGroupsPerWarp, int kRows>
 __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kernel(const StreamParams p) {
     using namespace sm100;
     extern __shared__ __align__(128) uint8_t dyn[];
@@ -507,7 +508,7 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int consumers = p.slices * p.row_warps;
     const int D = p.depth;
-    const uint32_t warp_rows = (uint32_t)(kTileRows * kGroupsPerWarp), tile_rows = warp_rows * (uint32_t)p.row_warps;
+    const uint32_t warp_rows = (uint32_t)(kRows * kGroupsPerWarp), tile_rows = warp_rows * (uint32_t)p.row_warps;
     const uint64_t tiles_m = (p.rows + tile_rows - 1) / tile_rows, Q = (uint64_t)p.count * tiles_m;
     const uint64_t q0 = Q * blockIdx.x / gridDim.x, q1 = Q * (blockIdx.x + 1) / gridDim.x;
     const uint32_t n_local = (uint32_t)(q1 - q0);
@@ -564,7 +565,7 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
         cj.init(q0, tiles_m);
         uint32_t issued = 0, i_slot = 0, i_phase = 0, j_buf = 0, j_phase = 0;      // i_phase = (issued / D) & 1, j_phase = (j / (D + 1)) & 1
         bool ok = true;
-        const int per_tile = consumers * kGroupsPerWarp * kTileRows;
+        const int per_tile = consumers * (int)warp_rows;
         for (uint32_t j = 0; j < n_local && ok; ++j, cj.next()) {
             while (issued < n_local && issued < j + (uint32_t)D && ok) {
                 const uint32_t slot = i_slot;               // issued % D; its previous use was one ring turn ago
@@ -647,6 +648,8 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
     constexpr int kSumsPerUnit = Dec::kSumGroup ? Dec::kBlockK / Dec::kSumGroup : 0;
     uint32_t sums = ctl.sums + (uint32_t)(unit0 * kSumsPerUnit * 4);
     const uint32_t row_bytes = p.pitch;                                    // stage rows, as the consumers see them
+    constexpr bool whole = kRows == kTileRows;
+    const uint32_t second = whole ? 8 * row_bytes : 0u;                    // from row g of a group to the row of the fragment's upper half
     float *red_all = reinterpret_cast<float *>(generic(ctl.red));
     const int cthreads = consumers * 32;
     if (threadIdx.x < 64 * p.units_per_slice + 4) reinterpret_cast<uint32_t *>(generic(ctl.zeros))[threadIdx.x] = 0u;
@@ -658,6 +661,9 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
             b.bl[hj] = lds64(b_lo + k);
         }
     };
+
+    // 8-value chunks of the input row per consumer thread: K / 8 over 32 x slices x row warps threads, at most the units per slice
+    constexpr int kXChunks = kBReg ? 1 : 2;
 
     // A warp whose wait ran out keeps walking the task list without touching data, so that it still
     // meets the other consumers at the named barriers of every matrix change and nobody waits for it.
@@ -685,23 +691,35 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
             asm volatile("bar.sync 1, %0;" ::"r"(cthreads) : "memory");
             cur_x = p.x_rows ? __ldg(p.x_rows + c.m) : c.m;
             const float *x = p.x + (uint64_t)cur_x * p.x_stride;
+            // The row is read (and SwiGLU evaluated) once: a thread keeps its eight values, or sixteen at widths where a warp
+            // owns two units of one row group, from the search for the largest magnitude to the digits.
             float mx = 0.0f;
             bool badx = false;
             const float *xu = p.x_up ? p.x_up + (uint64_t)cur_x * p.x_stride : nullptr;
             const float xw = p.x_up ? __ldg(p.x_weight + c.m) : 1.0f;
-            for (int k = threadIdx.x; k < p.K; k += cthreads) {
-                float v = __ldg(x + k);
-                if (xu) v = swiglu_mid(v, __ldg(xu + k), xw, p.x_limit, p.status);
-                badx |= !isfinite(v);
-                mx = fmaxf(mx, fabsf(v));
-            }
+            float xs[kXChunks][8];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            for (int q = 0; q < kXChunks; ++q) {
+                const int k8 = threadIdx.x + q * cthreads;
+                if (k8 < p.K / 8) {
+                    const float4 xa = __ldg(reinterpret_cast<const float4 *>(x + 8 * k8)), xb = __ldg(reinterpret_cast<const float4 *>(x + 8 * k8) + 1);
+                    xs[q][0] = xa.x; xs[q][1] = xa.y; xs[q][2] = xa.z; xs[q][3] = xa.w; xs[q][4] = xb.x; xs[q][5] = xb.y; xs[q][6] = xb.z; xs[q][7] = xb.w;
+                    if (xu) {
+                        const float4 ua = __ldg(reinterpret_cast<const float4 *>(xu + 8 * k8)), ub = __ldg(reinterpret_cast<const float4 *>(xu + 8 * k8) + 1);
+                        const float uv[8] = {ua.x, ua.y, ua.z, ua.w, ub.x, ub.y, ub.z, ub.w};
+#pragma unroll
+                        for (int i8 = 0; i8 < 8; ++i8) xs[q][i8] = swiglu_mid(xs[q][i8], uv[i8], xw, p.x_limit, p.status);
+                    }
+#pragma unroll
+                    for (int i8 = 0; i8 < 8; ++i8) { badx |= !isfinite(xs[q][i8]); mx = fmaxf(mx, fabsf(xs[q][i8])); }
+                }
+            }
+            // (magnitudes order like their bit patterns; fmaxf has dropped any NaN)
+            mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));
             if (lane == 0) ctl.warp_max[warp] = mx;
             if (badx) raise(p.status, YVEX_B200_STATUS_NUMERIC);
             asm volatile("bar.sync 1, %0;" ::"r"(cthreads) : "memory");
-            mx = 0.0f;
-            for (int w = 0; w < consumers; ++w) mx = fmaxf(mx, ctl.warp_max[w]);
+            mx = __uint_as_float(__reduce_max_sync(0xffffffffu, lane < consumers ? __float_as_uint(ctl.warp_max[lane]) : 0u));
             // S = the power of two above the largest magnitude; q = rint(x / S * 2^27), |q| <= 2^27
             int e = 0;
             if (mx > 0.0f && isfinite(mx)) frexpf(mx, &e);
@@ -709,17 +727,13 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
             if (threadIdx.x == 0) ctl.xscale[c.m & 7u] = ldexpf(1.0f, e - 27);
             int8_t *pl = reinterpret_cast<int8_t *>(generic(ctl.planes));
             float *sm = reinterpret_cast<float *>(generic(ctl.sums));
-            for (int k8 = threadIdx.x; k8 < p.K / 8; k8 += cthreads) {
+#pragma unroll
+            for (int c8 = 0; c8 < kXChunks; ++c8) {
+                const int k8 = threadIdx.x + c8 * cthreads;
+                if (k8 >= p.K / 8) continue;                                // (whole warps: K / 8 is a multiple of 32)
+                const float (&xv)[8] = xs[c8];
                 uint32_t d[4][2] = {{0u, 0u}, {0u, 0u}, {0u, 0u}, {0u, 0u}};
                 float s = 0.0f;
-                const float4 xa = __ldg(reinterpret_cast<const float4 *>(x + 8 * k8)), xb = __ldg(reinterpret_cast<const float4 *>(x + 8 * k8) + 1);
-                float xv[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
-                if (xu) {
-                    const float4 ua = __ldg(reinterpret_cast<const float4 *>(xu + 8 * k8)), ub = __ldg(reinterpret_cast<const float4 *>(xu + 8 * k8) + 1);
-                    const float uv[8] = {ua.x, ua.y, ua.z, ua.w, ub.x, ub.y, ub.z, ub.w};
-#pragma unroll
-                    for (int i8 = 0; i8 < 8; ++i8) xv[i8] = swiglu_mid(xv[i8], uv[i8], xw, p.x_limit, p.status);
-                }
 #pragma unroll
                 for (int i8 = 0; i8 < 8; ++i8) {
                     int q = isfinite(xv[i8]) ? __float2int_rn(xv[i8] * to_q) : 0;
@@ -784,8 +798,8 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
 #pragma unroll
                     for (int gi = 0; gi < kGroupsPerWarp; ++gi) {
                         // groups past a ragged tile's last row decode stale bytes; their results are never stored
-                        const uint32_t r0 = base + (uint32_t)(kTileRows * gi) * row_bytes + (uint32_t)(u * Dec::kBlockBytes);
-                        Dec::template unit<decltype(odd)::value>(r0, r0 + 8 * row_bytes, b, l, sums + (uint32_t)(u * kSumsPerUnit * 4), acc[gi],
+                        const uint32_t r0 = base + (uint32_t)(kRows * gi) * row_bytes + (uint32_t)(u * Dec::kBlockBytes);
+                        Dec::template unit<decltype(odd)::value>(r0, r0 + second, b, l, sums + (uint32_t)(u * kSumsPerUnit * 4), acc[gi],
                                                                  bad[gi]);
                     }
                 };
@@ -802,9 +816,10 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
             float a0 = acc[gi][0], a1 = acc[gi][1];
             a0 += __shfl_xor_sync(0xffffffffu, a0, 1); a0 += __shfl_xor_sync(0xffffffffu, a0, 2);
             a1 += __shfl_xor_sync(0xffffffffu, a1, 1); a1 += __shfl_xor_sync(0xffffffffu, a1, 2);
-            if (l.t == 0) { red[kTileRows * gi + l.g] = a0; red[kTileRows * gi + l.g + 8] = a1; }
+            float *to = red + (uint32_t)(kRows * gi) + (uint32_t)l.g;
+            if (l.t == 0) { to[0] = a0; if (whole) to[8] = a1; }
             // a malformed block scale only counts for rows that exist
-            const uint32_t r_lo = first + (uint32_t)(kTileRows * gi + l.g), r_hi = r_lo + 8;
+            const uint32_t r_lo = first + (uint32_t)(kRows * gi) + (uint32_t)l.g, r_hi = r_lo + (whole ? 8u : 0u);
             if (((bad[gi] & 1) && r_lo < nrows) || ((bad[gi] & 2) && r_hi < nrows)) raise(p.status, YVEX_B200_STATUS_NUMERIC);
         }
         __syncwarp();
@@ -813,7 +828,7 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
 }
 
 // ---- host side -----------------------------------------------------------------------------------------------
-struct StreamShape { int slices, units_per_slice, row_warps, consumers, depth, groups; uint32_t stage_bytes, smem_bytes, pitch; };
+struct StreamShape { int slices, units_per_slice, row_warps, consumers, depth, groups, group_rows; uint32_t stage_bytes, smem_bytes, pitch; };
 
 // K-slices (consumer warps along K), units per slice, warps along the rows of a stage and the deepest ring that fits.
 inline bool stream_shape(unsigned q, uint64_t width, uint64_t row_bytes, StreamShape &sh) {
@@ -834,8 +849,13 @@ inline bool stream_shape(unsigned q, uint64_t width, uint64_t row_bytes, StreamS
     }
     const uint32_t limit = 226u * 1024u;                   // the kernel also has a few hundred bytes of static shared memory
     // two row groups per warp when at least three such stages fit, else one
-    for (sh.groups = kMaxGroupsPerWarp; sh.groups >= 1; --sh.groups) {
-        sh.stage_bytes = (uint32_t)(kTileRows * sh.groups * sh.row_warps * sh.pitch);
+    // (last, groups of eight rows: Q8_0 rows of 7168 weights are 7616 bytes, and sixteen of them leave no room for a second stage.
+    // Half of every MMA is then idle, but the generic kernel such rows used to take measured 21.1 ms on 128 matrices of
+    // 2048 x 7168, this path 0.78 ms = 2.56 TB/s)
+    for (int step = 0; step < (q == Q_Q8_0 ? 3 : 2); ++step) {
+        sh.groups = step == 0 ? kMaxGroupsPerWarp : 1;
+        sh.group_rows = step < 2 ? kTileRows : kTileRows / 2;
+        sh.stage_bytes = (uint32_t)(sh.group_rows * sh.groups * sh.row_warps * sh.pitch);
         for (sh.depth = kMaxDepth; sh.depth >= (sh.groups > 1 ? 3 : 2); --sh.depth) {
             // every piece is rounded up to 128 bytes; with tables one piece may have to step over the table window,
             // which starts at most 64 KiB - 1 into the allocation (what lies before it stays usable)
@@ -859,20 +879,22 @@ inline bool stream_eligible(unsigned q, uint64_t rows, uint64_t width, uint64_t 
            stream_shape(q, width, row_bytes, sh);
 }
 
-template <class Dec, bool kBReg, int kG>
+template <class Dec, bool kBReg, int kG, int kRows = kTileRows>
 inline int stream_launch_v(StreamParams &p, const StreamShape &sh, cudaStream_t stream) {
     static SmemOptIn opt_in;
-    if (opt_in.ensure(gemv_stream_kernel<Dec, kBReg, kG>, 226 * 1024) != OK) return ERR_BACKEND;
-    const uint64_t tile_rows = (uint64_t)kTileRows * kG * sh.row_warps;
+    if (opt_in.ensure(gemv_stream_kernel<Dec, kBReg, kG, kRows>, 226 * 1024) != OK) return ERR_BACKEND;
+    const uint64_t tile_rows = (uint64_t)kRows * kG * sh.row_warps;
     const uint64_t tasks = (uint64_t)p.count * ((p.rows + tile_rows - 1) / tile_rows);
     const unsigned grid = (unsigned)(tasks < (uint64_t)kSmCount ? tasks : (uint64_t)kSmCount);
-    if (launch_pdl(gemv_stream_kernel<Dec, kBReg, kG>, dim3(grid), dim3(32 * (sh.consumers + 1)), sh.smem_bytes, stream, p) != cudaSuccess)
+    if (launch_pdl(gemv_stream_kernel<Dec, kBReg, kG, kRows>, dim3(grid), dim3(32 * (sh.consumers + 1)), sh.smem_bytes, stream, p) != cudaSuccess)
         return ERR_BACKEND;
     return launch_status(1);
 }
 
 template <class Dec>
 inline int stream_launch_t(StreamParams &p, const StreamShape &sh, cudaStream_t stream) {
+    if constexpr (Dec::kQtype == Q_Q8_0)
+        if (sh.group_rows == kTileRows / 2) return stream_launch_v<Dec, false, 1, kTileRows / 2>(p, sh, stream);
     const bool breg = sh.units_per_slice == 1;
     if (sh.groups == 2) return breg ? stream_launch_v<Dec, true, 2>(p, sh, stream) : stream_launch_v<Dec, false, 2>(p, sh, stream);
     return breg ? stream_launch_v<Dec, true, 1>(p, sh, stream) : stream_launch_v<Dec, false, 1>(p, sh, stream);
