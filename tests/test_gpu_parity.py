@@ -535,6 +535,30 @@ def test_gemv_scalar_qtypes_several_inputs(L, qtype, rows, width, inputs):
     assert st.read() == 1
 
 
+@pytest.mark.parametrize("qtype", [synth.IQ2_XXS, synth.Q4_K, synth.Q8_0, synth.Q2_K, synth.MXFP4])
+@pytest.mark.parametrize("rows,width,inputs", [(17, 512, 2), (33, 1536, 3), (300, 4096, 8), (5, 7168, 5), (64, 1024, 4), (40, 256, 6), (16, 8192, 9)])
+def test_gemv_block_qtypes_several_inputs(L, qtype, rows, width, inputs):
+    """Passes of four input rows against one call per row: full and ragged passes, ragged tiles, rows and planes of every
+    slicing, widths whose planes leave no room for four rows (those take one row per pass). Exact integer products and the
+    same f32 steps: 1e-6 covers another slicing of K. One non-finite value in the last row is refused."""
+    import torch
+    if qtype == synth.MXFP4 and width % 512:
+        pytest.skip("rows of an odd number of 256-weight units")
+    w = dev(synth.random_blocks(qtype, rows, width, rows + width))
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(inputs)
+    x, add, st = torch.randn((inputs, width), device="cuda", generator=gen), torch.randn((inputs, rows), device="cuda", generator=gen), L.Status()
+    x *= torch.logspace(-3, 3, inputs, device="cuda")[:, None]           # every row needs its own scale
+    y = L.gemv(qtype, w, rows, width, x, st, additive=add)
+    one = torch.stack([L.gemv(qtype, w, rows, width, x[i], st, additive=add[i])[0] for i in range(inputs)])
+    assert st.read() == 0
+    for i in range(inputs):
+        assert rel_l2(y[i].cpu().numpy(), one[i].cpu().numpy()) <= 1e-6
+    x[inputs - 1, width - 1] = float("nan")
+    L.gemv(qtype, w, rows, width, x, st)
+    assert st.read() == 1
+
+
 @pytest.mark.parametrize("rows,width,inputs", [(2048, 7168, 1), (8, 8192, 1), (13, 6912, 2), (1, 7936, 5), (149 * 8 + 3, 8192, 1)])
 def test_gemv_q8_0_long_rows(L, rows, width, inputs):
     """Rows of which sixteen leave no room for a second stage go in groups of eight: ragged tiles, padded and plain pitches,

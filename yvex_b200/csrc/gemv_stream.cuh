@@ -120,6 +120,24 @@ __device__ __forceinline__ float comb(int a_hi, int a_lo, int b_hi, int b_lo) {
     return fmaf((float)(a_hi * 128 + a_lo), 16384.0f, (float)(b_hi * 128 + b_lo));
 }
 
+// Several input rows per pass. A 32-weight group fills the K slots of one MMA (lane t of a quad holds weights 8t .. 8t + 7 of its
+// two rows), so all eight columns see every slot: columns 4 i + d are digit plane d of input i, two inputs per MMA, nothing
+// multiplied by zeros, and one decode serves every input. Lane t of a row ends up with the upper (t even) or lower digit
+// pair of input t >> 1; the group's scale is applied there, the halves meet once per tile. (With the single-row
+// arrangement - columns of zeros outside a lane's group - four rows in one pass were bound by 64 MMAs per 256 x 16 weights
+// and no faster than four passes.) 4096 x 4096, eight rows, a pass per row against this: Q8_0 30 / 17 us, Q4_K 27 / 17,
+// Q2_K 32 / 18, MXFP4 30 / 25; IQ2_XXS 65536 x 2048 148 / 66.
+struct DenseB { uint32_t at, pair, sums, sums_pair; bool low; };      // planes and sums of this lane's input (of pair 0), to the next pair
+
+template <int kIn> __device__ __forceinline__ void mma_dense(const uint32_t (&a)[4], const DenseB &b, int j, int (&c)[kIn / 2][4]) {
+#pragma unroll
+    for (int p = 0; p < kIn / 2; ++p) {
+        const uint2 w = lds64(b.at + p * b.pair + 32u * j);
+        mma_s8<true>(c[p], a, w.x, w.y);
+    }
+}
+__device__ __forceinline__ float digit_pair(int hi, int lo) { return (float)(hi * 128 + lo); }
+
 // What a decoder provides:
 //   kBlockBytes / kBlockK   bytes and weights of the unit a warp walks (IQ2_XXS, Q4_K: one 256-weight
 //                           superblock; Q8_0: eight 32-weight blocks, so that every qtype has 8 groups per unit)
@@ -189,6 +207,35 @@ struct StreamIq2 {
         acc[0] = fmaf(blk0, 0.125f * f0, acc[0]);
         acc[1] = fmaf(blk1, 0.125f * f1, acc[1]);
     }
+    __device__ __forceinline__ static void sub_of(uint32_t grids, uint32_t ss, const Lane &l, uint32_t &lo, uint32_t &hi) {
+        constexpr uint32_t kPos = 8u | (25u << 8) | (43u << 16), kNeg = 0xf8u | (0xe7u << 8) | (0xd5u << 16);
+        const uint32_t sel = lds32(prmt(grids, l.nib_base, 0x7604u | ((uint32_t)l.t << 4))) | lds32(prmt(ss >> (7 * l.t), l.sgn_base, 0x7604u));
+        lo = prmt(kPos, kNeg, sel);
+        hi = prmt(kPos, kNeg, sel >> 16);
+    }
+    template <int kIn, int> __device__ __forceinline__ static void dense(uint32_t row0, uint32_t row1, const DenseB &b, const Lane &l, float (&acc)[kIn / 2][2], int &bad) {
+        float blk[kIn / 2][2] = {};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            uint32_t g0, s0, g1, s1, a[4];
+            group(row0 + 2 + 8 * j, g0, s0);
+            group(row1 + 2 + 8 * j, g1, s1);
+            sub_of(g0, s0, l, a[0], a[2]);
+            sub_of(g1, s1, l, a[1], a[3]);
+            int c[kIn / 2][4];
+            mma_dense<kIn>(a, b, j, c);
+            const float f0 = (float)((s0 >> 27) | 1u), f1 = (float)((s1 >> 27) | 1u);
+#pragma unroll
+            for (int p = 0; p < kIn / 2; ++p) {
+                blk[p][0] = fmaf(digit_pair(c[p][0], c[p][1]), f0, blk[p][0]);
+                blk[p][1] = fmaf(digit_pair(c[p][2], c[p][3]), f1, blk[p][1]);
+            }
+        }
+        const float d0 = f16_bits_to_float((uint16_t)lds16(row0)), d1 = f16_bits_to_float((uint16_t)lds16(row1));
+        bad |= (scale_bad(d0) ? 1 : 0) | (scale_bad(d1) ? 2 : 0);
+#pragma unroll
+        for (int p = 0; p < kIn / 2; ++p) { acc[p][0] = fmaf(blk[p][0], 0.125f * d0, acc[p][0]); acc[p][1] = fmaf(blk[p][1], 0.125f * d1, acc[p][1]); }
+    }
 };
 
 // Q4_K (extension; no reference decoder): 144 bytes = f16 d, f16 dmin, 12 bytes of 6-bit (scale, min)
@@ -255,6 +302,36 @@ struct StreamQ4k {
         acc[0] += fmaf(d0, blk0, -n0 * min0);
         acc[1] += fmaf(d1, blk1, -n1 * min1);
     }
+    template <int kIn, int> __device__ __forceinline__ static void dense(uint32_t row0, uint32_t row1, const DenseB &b, const Lane &l, float (&acc)[kIn / 2][2], int &bad) {
+        float blk[kIn / 2][2] = {}, mn[kIn / 2][2] = {};
+        const uint4 head0 = lds128(row0), head1 = lds128(row1);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t at = 16 + 32 * (j >> 1) + 8 * l.t;
+            const uint2 w0 = lds64(row0 + at), w1 = lds64(row1 + at);
+            const uint32_t a[4] = {(w0.x >> (4 * (j & 1))) & 0x0f0f0f0fu, (w1.x >> (4 * (j & 1))) & 0x0f0f0f0fu,
+                                   (w0.y >> (4 * (j & 1))) & 0x0f0f0f0fu, (w1.y >> (4 * (j & 1))) & 0x0f0f0f0fu};
+            int c[kIn / 2][4];
+            mma_dense<kIn>(a, b, j, c);
+            uint32_t sc0, q0, sc1, q1;
+            scale_min(head0.y, head0.z, head0.w, j >> 2, j & 3, sc0, q0);
+            scale_min(head1.y, head1.z, head1.w, j >> 2, j & 3, sc1, q1);
+#pragma unroll
+            for (int p = 0; p < kIn / 2; ++p) {
+                const float xs = ldsf(b.sums + p * b.sums_pair + 4 * j);
+                blk[p][0] = fmaf(digit_pair(c[p][0], c[p][1]), (float)sc0, blk[p][0]);
+                blk[p][1] = fmaf(digit_pair(c[p][2], c[p][3]), (float)sc1, blk[p][1]);
+                mn[p][0] = fmaf((float)q0, xs, mn[p][0]);
+                mn[p][1] = fmaf((float)q1, xs, mn[p][1]);
+            }
+        }
+        const float d0 = f16_bits_to_float((uint16_t)head0.x), n0 = f16_bits_to_float((uint16_t)(head0.x >> 16));
+        const float d1 = f16_bits_to_float((uint16_t)head1.x), n1 = f16_bits_to_float((uint16_t)(head1.x >> 16));
+        bad |= (scale_bad(d0) || scale_bad(n0) ? 1 : 0) | (scale_bad(d1) || scale_bad(n1) ? 2 : 0);
+        const float m0 = b.low ? -n0 : 0.0f, m1 = b.low ? -n1 : 0.0f;           // the minimum term counts once, with the lower digits
+#pragma unroll
+        for (int p = 0; p < kIn / 2; ++p) { acc[p][0] += fmaf(d0, blk[p][0], m0 * mn[p][0]); acc[p][1] += fmaf(d1, blk[p][1], m1 * mn[p][1]); }
+    }
 };
 
 // Q2_K (src/gguf/quant_block.c:769-817): 84 bytes = 16 bytes of (4-bit scale | 4-bit min << 4) per 16-weight
@@ -313,6 +390,34 @@ struct StreamQ2k {
         acc[0] += fmaf(d0, blk0, -n0 * min0);
         acc[1] += fmaf(d1, blk1, -n1 * min1);
     }
+    template <int kIn, int> __device__ __forceinline__ static void dense(uint32_t row0, uint32_t row1, const DenseB &b, const Lane &l, float (&acc)[kIn / 2][2], int &bad) {
+        float blk[kIn / 2][2] = {}, mn[kIn / 2][2] = {};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t at = 16 + 32 * (j >> 2) + 8 * l.t;
+            const uint32_t s0 = lds16(row0 + 2 * j), s1 = lds16(row1 + 2 * j);                      // the group's two scale bytes
+            const uint32_t f0 = (s0 >> (8 * (l.t >> 1))) & 15u, f1 = (s1 >> (8 * (l.t >> 1))) & 15u;
+            const uint32_t a[4] = {((lds32(row0 + at) >> (2 * (j & 3))) & 0x03030303u) * f0, ((lds32(row1 + at) >> (2 * (j & 3))) & 0x03030303u) * f1,
+                                   ((lds32(row0 + at + 4) >> (2 * (j & 3))) & 0x03030303u) * f0, ((lds32(row1 + at + 4) >> (2 * (j & 3))) & 0x03030303u) * f1};
+            int c[kIn / 2][4];
+            mma_dense<kIn>(a, b, j, c);
+#pragma unroll
+            for (int p = 0; p < kIn / 2; ++p) {
+                const float xa = ldsf(b.sums + p * b.sums_pair + 8 * j), xb = ldsf(b.sums + p * b.sums_pair + 8 * j + 4);
+                blk[p][0] += digit_pair(c[p][0], c[p][1]);
+                blk[p][1] += digit_pair(c[p][2], c[p][3]);
+                mn[p][0] = fmaf((float)((s0 >> 4) & 15u), xa, fmaf((float)(s0 >> 12), xb, mn[p][0]));
+                mn[p][1] = fmaf((float)((s1 >> 4) & 15u), xa, fmaf((float)(s1 >> 12), xb, mn[p][1]));
+            }
+        }
+        const uint32_t h0 = lds32(row0 + 80), h1 = lds32(row1 + 80);                 // d, dmin
+        const float d0 = f16_bits_to_float((uint16_t)h0), n0 = f16_bits_to_float((uint16_t)(h0 >> 16));
+        const float d1 = f16_bits_to_float((uint16_t)h1), n1 = f16_bits_to_float((uint16_t)(h1 >> 16));
+        bad |= (scale_bad(d0) || scale_bad(n0) ? 1 : 0) | (scale_bad(d1) || scale_bad(n1) ? 2 : 0);
+        const float m0 = b.low ? -n0 : 0.0f, m1 = b.low ? -n1 : 0.0f;           // the minimum term counts once, with the lower digits
+#pragma unroll
+        for (int p = 0; p < kIn / 2; ++p) { acc[p][0] += fmaf(d0, blk[p][0], m0 * mn[p][0]); acc[p][1] += fmaf(d1, blk[p][1], m1 * mn[p][1]); }
+    }
 };
 
 // Q8_0 (src/gguf/quant_block.c:819-833): 34 bytes = f16 d + 32 int8. A unit is eight blocks (256 weights);
@@ -362,6 +467,31 @@ struct StreamQ80 {
                                                 float (&acc)[2], int &bad) {
         half<0>(row0, row1, b, l, acc, bad);
         half<1>(row0, row1, b, l, acc, bad);
+    }
+    // quants 8t .. 8t + 7 of a block that starts on a 2-byte boundary, and its scale
+    __device__ __forceinline__ static void eight(uint32_t block, int t, uint32_t &lo, uint32_t &hi, float &d, int &bad, int flag) {
+        const uint32_t at = block + 2 + 8 * t, sh = (at & 2u) * 8u, w = at & ~3u;
+        const uint32_t v0 = lds32(w), v1 = lds32(w + 4), v2 = lds32(w + 8);
+        lo = __funnelshift_r(v0, v1, sh);
+        hi = __funnelshift_r(v1, v2, sh);
+        d = f16_bits_to_float((uint16_t)lds16(block));
+        bad |= scale_bad(d) ? flag : 0;
+    }
+    template <int kIn, int> __device__ __forceinline__ static void dense(uint32_t row0, uint32_t row1, const DenseB &b, const Lane &l, float (&acc)[kIn / 2][2], int &bad) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            uint32_t a[4];
+            float d0, d1;
+            eight(row0 + 34 * j, l.t, a[0], a[2], d0, bad, 1);
+            eight(row1 + 34 * j, l.t, a[1], a[3], d1, bad, 2);
+            int c[kIn / 2][4];
+            mma_dense<kIn>(a, b, j, c);
+#pragma unroll
+            for (int p = 0; p < kIn / 2; ++p) {
+                acc[p][0] = fmaf(digit_pair(c[p][0], c[p][1]), d0, acc[p][0]);
+                acc[p][1] = fmaf(digit_pair(c[p][2], c[p][3]), d1, acc[p][1]);
+            }
+        }
     }
 };
 
@@ -445,6 +575,30 @@ struct StreamMxfp4 {
         half<0, kOdd>(row0, row1, b, l, sums, acc, bad);
         half<1, kOdd>(row0, row1, b, l, sums, acc, bad);
     }
+    // data word t of a block (codes of weights 4t .. and 16 + 4t ..), and its scale; a block starts on any byte
+    __device__ __forceinline__ static void word_of(uint32_t block, int t, uint32_t &lo, uint32_t &hi, float &scale, int &bad, int flag) {
+        const uint32_t at = block + 1 + 4 * t, w = at & ~3u, e = lds8(block);
+        codes(__funnelshift_r(lds32(w), lds32(w + 4), 8 * (at & 3u)), lo, hi);
+        bad |= e == 255u ? flag : 0;
+        scale = __uint_as_float(e ? e << 23 : 0x00400000u) * 0.5f;
+    }
+    template <int kIn, int> __device__ __forceinline__ static void dense(uint32_t row0, uint32_t row1, const DenseB &b, const Lane &l, float (&acc)[kIn / 2][2], int &bad) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            uint32_t a[4];
+            float s0, s1;
+            word_of(row0 + 17 * j, l.t, a[0], a[2], s0, bad, 1);
+            word_of(row1 + 17 * j, l.t, a[1], a[3], s1, bad, 2);
+            int c[kIn / 2][4];
+            mma_dense<kIn>(a, b, j, c);
+#pragma unroll
+            for (int p = 0; p < kIn / 2; ++p) {
+                const float off = b.low ? 16.0f * ldsf(b.sums + p * b.sums_pair + 4 * j) : 0.0f;        // 16 x the sum of the activation over this block
+                acc[p][0] = fmaf(digit_pair(c[p][0], c[p][1]) - off, s0, acc[p][0]);
+                acc[p][1] = fmaf(digit_pair(c[p][2], c[p][3]) - off, s1, acc[p][1]);
+            }
+        }
+    }
 };
 
 // ---- kernel ------------------------------------------------------------------------------------------------
@@ -463,6 +617,7 @@ struct StreamParams {
     uint32_t stage_bytes, smem_bytes;
     const float *x;                     // input vector of matrix m at x + m * x_stride
     uint64_t x_stride;
+    uint32_t inputs;                    // kIn > 1: matrix m multiplies input rows kIn m .. (of `inputs`), result i at out + (kIn m + i) * out_stride
     // optional: the input of matrix m is bf16(SwiGLU(x row, x_up row) * x_weight[m]) with the clamp x_limit
     // (src/graph/moe.c:605-613), x_up rows spaced like the x rows; formed while the planes are prepared
     const float *x_up;
@@ -477,16 +632,19 @@ struct StreamParams {
 
 constexpr int kMaxGroupsPerWarp = 2;    // 16-row groups one consumer warp decodes per stage (independent work in flight)
 
+constexpr int kMaxInputs = 4;            // input rows of one matrix a pass shares a decode between
+constexpr int kPlanePad = 32;            // bytes between their digit planes: the eight columns of a fragment on eight different bank groups
+
 struct StreamCtl {
     uint64_t full[kMaxDepth], empty[kMaxDepth], red_full[kMaxDepth + 1], tab_full;
     uint32_t stage[kMaxDepth];          // shared-window addresses
     uint32_t planes, zeros, sums, red, table;
-    float xscale[8], warp_max[kMaxConsumers];
+    float xscale[8][kMaxInputs], warp_max[kMaxConsumers];
     int abort, layout_bad;
 };
 
-__host__ __device__ inline uint32_t stream_small_bytes(int K, int consumers, int depth, int units_per_slice, int groups) {
-    return (uint32_t)(4 * K + 256 * units_per_slice + 128 + (K / 16) * 4 + 128 + (depth + 1) * consumers * groups * kTileRows * 4 + 256);
+__host__ __device__ inline uint32_t stream_small_bytes(int K, int consumers, int depth, int units_per_slice, int groups, int inputs) {
+    return (uint32_t)(inputs * 4 * (K + (inputs > 1 ? kPlanePad : 0)) + 256 * units_per_slice + 128 + inputs * (K / 16) * 4 + 128 + inputs * (depth + 1) * consumers * groups * kTileRows * 4 + 256);
 }
 
 // The task list of one CTA, walked without divisions: tile `tile` of matrix `m`.
@@ -500,14 +658,14 @@ struct TaskCursor {
 // kBReg: the warp's whole K-slice is one unit, so its B fragments live in registers from one matrix change to the next.
 // kGroupsPerWarp: 16-row groups a consumer warp decodes per stage.
 // kRows: matrix rows in one MMA group: 16, or 8 where sixteen rows are too long for a ring (row g + 8 of a fragment then repeats row g).
-template <class Dec, bool kBReg, int kGroupsPerWarp, int kRows>
+template <class Dec, bool kBReg, int kGroupsPerWarp, int kIn, int kRows>
 __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kernel(const StreamParams p) {
     using namespace sm100;
     extern __shared__ __align__(128) uint8_t dyn[];
     __shared__ StreamCtl ctl;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int consumers = p.slices * p.row_warps;
-    const int D = p.depth;
+    const int D = p.depth, plane = p.K + (kIn > 1 ? kPlanePad : 0);        // bytes from one digit plane to the next
     const uint32_t warp_rows = (uint32_t)(kRows * kGroupsPerWarp), tile_rows = warp_rows * (uint32_t)p.row_warps;
     const uint64_t tiles_m = (p.rows + tile_rows - 1) / tile_rows, Q = (uint64_t)p.count * tiles_m;
     const uint64_t q0 = Q * blockIdx.x / gridDim.x, q1 = Q * (blockIdx.x + 1) / gridDim.x;
@@ -530,10 +688,10 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
             return at;
         };
         for (int i = 0; i < D; ++i) ctl.stage[i] = take(p.stage_bytes + 16);
-        ctl.planes = take((uint32_t)(4 * p.K));
+        ctl.planes = take((uint32_t)(kIn * 4 * plane));
         ctl.zeros = take((uint32_t)(256 * p.units_per_slice + 16));
-        ctl.sums = take((uint32_t)(p.K / 16) * 4u);
-        ctl.red = take((uint32_t)((D + 1) * consumers * kGroupsPerWarp * kTileRows) * 4u);
+        ctl.sums = take((uint32_t)(kIn * (p.K / 16)) * 4u);
+        ctl.red = take((uint32_t)(kIn * (D + 1) * consumers * kGroupsPerWarp * kTileRows) * 4u);
         ctl.table = tab;
         ctl.layout_bad = cur > end || (Dec::kTables && tab + kTableBytes > end);
         ctl.abort = 0;
@@ -565,7 +723,7 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
         cj.init(q0, tiles_m);
         uint32_t issued = 0, i_slot = 0, i_phase = 0, j_buf = 0, j_phase = 0;      // i_phase = (issued / D) & 1, j_phase = (j / (D + 1)) & 1
         bool ok = true;
-        const int per_tile = consumers * (int)warp_rows;
+        const int per_tile = kIn * consumers * (int)warp_rows;
         for (uint32_t j = 0; j < n_local && ok; ++j, cj.next()) {
             while (issued < n_local && issued < j + (uint32_t)D && ok) {
                 const uint32_t slot = i_slot;               // issued % D; its previous use was one ring turn ago
@@ -607,18 +765,23 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
             if (!ok) break;
             uint64_t row0;
             const uint32_t nrows = rows_of(cj, row0);
-            // partial sums of the tile: [row warp][slice][group][16 rows]
+            // partial sums of the tile: [input][row warp][slice][group][16 rows]
             const float *red = reinterpret_cast<const float *>(generic(ctl.red)) + (size_t)buf * per_tile;
-            const float scale = ctl.xscale[cj.m & 7u];
-            for (uint32_t r = lane; r < nrows; r += 32) {
-                const uint32_t rw = r / warp_rows, in_warp = r % warp_rows;
-                float sum = 0.0f;
-                for (int s = 0; s < p.slices; ++s) sum += red[((size_t)rw * p.slices + s) * warp_rows + in_warp];        // fixed order
-                sum *= scale;
-                const uint64_t at = (uint64_t)cj.m * p.out_stride + row0 + r;
-                if (p.additive) sum += p.additive[at];
-                if (!isfinite(sum)) raise(p.status, YVEX_B200_STATUS_NUMERIC);
-                p.out[at] = p.round_bf16 ? bf16_round(sum) : sum;
+#pragma unroll
+            for (int in = 0; in < kIn; ++in, red += consumers * (int)warp_rows) {
+                const uint64_t result = (uint64_t)cj.m * kIn + in;
+                if (kIn > 1 && result >= p.inputs) break;
+                const float scale = ctl.xscale[cj.m & 7u][in];
+                for (uint32_t r = lane; r < nrows; r += 32) {
+                    const uint32_t rw = r / warp_rows, in_warp = r % warp_rows;
+                    float sum = 0.0f;
+                    for (int s = 0; s < p.slices; ++s) sum += red[((size_t)rw * p.slices + s) * warp_rows + in_warp];        // fixed order
+                    sum *= scale;
+                    const uint64_t at = result * p.out_stride + row0 + r;
+                    if (p.additive) sum += p.additive[at];
+                    if (!isfinite(sum)) raise(p.status, YVEX_B200_STATUS_NUMERIC);
+                    p.out[at] = p.round_bf16 ? bf16_round(sum) : sum;
+                }
             }
         }
         if (!ok && lane == 0) {
@@ -663,7 +826,7 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
     };
 
     // 8-value chunks of the input row per consumer thread: K / 8 over 32 x slices x row warps threads, at most the units per slice
-    constexpr int kXChunks = kBReg ? 1 : 2;
+    constexpr int kXChunks = kIn > 1 ? 4 : kBReg ? 1 : 2;
 
     // A warp whose wait ran out keeps walking the task list without touching data, so that it still
     // meets the other consumers at the named barriers of every matrix change and nobody waits for it.
@@ -682,7 +845,7 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
         const uint32_t nrows = rows_of(c, row0);
         if (c.m != cur_m && cur_m != 0xffffffffu && p.x_rows && __ldg(p.x_rows + c.m) == cur_x) {
             // the next matrix reads the same input row: the planes, sums and B registers stand as they are
-            if (threadIdx.x == 0) ctl.xscale[c.m & 7u] = ctl.xscale[cur_m & 7u];
+            if (threadIdx.x == 0) ctl.xscale[c.m & 7u][0] = ctl.xscale[cur_m & 7u][0];
             cur_m = c.m;
         }
         if (c.m != cur_m) {
@@ -690,48 +853,55 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
             // consumer has finished the previous matrix once it is past this barrier.
             asm volatile("bar.sync 1, %0;" ::"r"(cthreads) : "memory");
             cur_x = p.x_rows ? __ldg(p.x_rows + c.m) : c.m;
-            const float *x = p.x + (uint64_t)cur_x * p.x_stride;
-            // The row is read (and SwiGLU evaluated) once: a thread keeps its eight values, or sixteen at widths where a warp
-            // owns two units of one row group, from the search for the largest magnitude to the digits.
+            // kIn > 1: the warps are dealt to the pass's input rows (a remainder stays idle), rows past the last repeat it
+            const int xin = kIn == 1 ? 0 : warp % kIn, xthreads = kIn == 1 ? cthreads : 32 * (consumers / kIn);
+            const int x0 = kIn == 1 ? (int)threadIdx.x : warp / kIn < consumers / kIn ? 32 * (warp / kIn) + lane : p.K;
+            const uint32_t xrow = kIn == 1 ? cur_x : min(cur_x * kIn + (uint32_t)xin, p.inputs - 1u);
+            const float *x = p.x + (uint64_t)xrow * p.x_stride;
+            // One input row is read (and SwiGLU evaluated) once: a thread keeps its eight values, or sixteen at widths where a
+            // warp owns two units of one row group, from the search for the largest magnitude to the digits.
             float mx = 0.0f;
             bool badx = false;
-            const float *xu = p.x_up ? p.x_up + (uint64_t)cur_x * p.x_stride : nullptr;
-            const float xw = p.x_up ? __ldg(p.x_weight + c.m) : 1.0f;
+            const float *xu = kIn == 1 && p.x_up ? p.x_up + (uint64_t)cur_x * p.x_stride : nullptr;
+            const float xw = kIn == 1 && p.x_up ? __ldg(p.x_weight + c.m) : 1.0f;
             float xs[kXChunks][8];
+            auto load8 = [&](int k8, float (&v)[8]) {
+                const float4 xa = __ldg(reinterpret_cast<const float4 *>(x + 8 * k8)), xb = __ldg(reinterpret_cast<const float4 *>(x + 8 * k8) + 1);
+                v[0] = xa.x; v[1] = xa.y; v[2] = xa.z; v[3] = xa.w; v[4] = xb.x; v[5] = xb.y; v[6] = xb.z; v[7] = xb.w;
+                if (xu) {
+                    const float4 ua = __ldg(reinterpret_cast<const float4 *>(xu + 8 * k8)), ub = __ldg(reinterpret_cast<const float4 *>(xu + 8 * k8) + 1);
+                    const float uv[8] = {ua.x, ua.y, ua.z, ua.w, ub.x, ub.y, ub.z, ub.w};
 #pragma unroll
-            for (int q = 0; q < kXChunks; ++q) {
-                const int k8 = threadIdx.x + q * cthreads;
-                if (k8 < p.K / 8) {
-                    const float4 xa = __ldg(reinterpret_cast<const float4 *>(x + 8 * k8)), xb = __ldg(reinterpret_cast<const float4 *>(x + 8 * k8) + 1);
-                    xs[q][0] = xa.x; xs[q][1] = xa.y; xs[q][2] = xa.z; xs[q][3] = xa.w; xs[q][4] = xb.x; xs[q][5] = xb.y; xs[q][6] = xb.z; xs[q][7] = xb.w;
-                    if (xu) {
-                        const float4 ua = __ldg(reinterpret_cast<const float4 *>(xu + 8 * k8)), ub = __ldg(reinterpret_cast<const float4 *>(xu + 8 * k8) + 1);
-                        const float uv[8] = {ua.x, ua.y, ua.z, ua.w, ub.x, ub.y, ub.z, ub.w};
-#pragma unroll
-                        for (int i8 = 0; i8 < 8; ++i8) xs[q][i8] = swiglu_mid(xs[q][i8], uv[i8], xw, p.x_limit, p.status);
-                    }
-#pragma unroll
-                    for (int i8 = 0; i8 < 8; ++i8) { badx |= !isfinite(xs[q][i8]); mx = fmaxf(mx, fabsf(xs[q][i8])); }
+                    for (int i8 = 0; i8 < 8; ++i8) v[i8] = swiglu_mid(v[i8], uv[i8], xw, p.x_limit, p.status);
                 }
+            };
+            auto magnitude = [&](const float (&v)[8]) {
+#pragma unroll
+                for (int i8 = 0; i8 < 8; ++i8) { badx |= !isfinite(v[i8]); mx = fmaxf(mx, fabsf(v[i8])); }
+            };
+#pragma unroll
+            for (int q = 0; q < kXChunks; ++q)
+                if (x0 + q * xthreads < p.K / 8) load8(x0 + q * xthreads, xs[q]);
+#pragma unroll
+            for (int q = 0; q < kXChunks; ++q)
+                if (x0 + q * xthreads < p.K / 8) magnitude(xs[q]);
+            if constexpr (kIn > 1) {                                        // (a quarter of the threads per row: the rest is read twice)
+                for (int k8 = x0 + kXChunks * xthreads; k8 < p.K / 8; k8 += xthreads) { float v[8]; load8(k8, v); magnitude(v); }
             }
             // (magnitudes order like their bit patterns; fmaxf has dropped any NaN)
             mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));
             if (lane == 0) ctl.warp_max[warp] = mx;
             if (badx) raise(p.status, YVEX_B200_STATUS_NUMERIC);
             asm volatile("bar.sync 1, %0;" ::"r"(cthreads) : "memory");
-            mx = __uint_as_float(__reduce_max_sync(0xffffffffu, lane < consumers ? __float_as_uint(ctl.warp_max[lane]) : 0u));
+            mx = __uint_as_float(__reduce_max_sync(0xffffffffu, lane < consumers && (kIn == 1 || (lane % kIn == xin && lane / kIn < consumers / kIn)) ? __float_as_uint(ctl.warp_max[lane]) : 0u));
             // S = the power of two above the largest magnitude; q = rint(x / S * 2^27), |q| <= 2^27
             int e = 0;
             if (mx > 0.0f && isfinite(mx)) frexpf(mx, &e);
             const float to_q = ldexpf(1.0f, 27 - e);
-            if (threadIdx.x == 0) ctl.xscale[c.m & 7u] = ldexpf(1.0f, e - 27);
-            int8_t *pl = reinterpret_cast<int8_t *>(generic(ctl.planes));
-            float *sm = reinterpret_cast<float *>(generic(ctl.sums));
-#pragma unroll
-            for (int c8 = 0; c8 < kXChunks; ++c8) {
-                const int k8 = threadIdx.x + c8 * cthreads;
-                if (k8 >= p.K / 8) continue;                                // (whole warps: K / 8 is a multiple of 32)
-                const float (&xv)[8] = xs[c8];
+            if (kIn == 1 ? threadIdx.x == 0 : x0 == 0) ctl.xscale[c.m & 7u][xin] = ldexpf(1.0f, e - 27);
+            int8_t *pl = reinterpret_cast<int8_t *>(generic(ctl.planes)) + (size_t)xin * 4 * plane;
+            float *sm = reinterpret_cast<float *>(generic(ctl.sums)) + (size_t)xin * (p.K / 16);
+            auto digits = [&](int k8, const float (&xv)[8]) {               // (whole warps: K / 8 is a multiple of 32)
                 uint32_t d[4][2] = {{0u, 0u}, {0u, 0u}, {0u, 0u}, {0u, 0u}};
                 float s = 0.0f;
 #pragma unroll
@@ -755,13 +925,13 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
                         const uint32_t got = __shfl_xor_sync(0xffffffffu, sub < 2 ? d[pi][1] : d[pi][0], 2);
                         const uint32_t lo = sub < 2 ? d[pi][0] : got, hi = sub < 2 ? got : d[pi][1];
                         const int chunk = sub < 2 ? 2 * sub : 2 * (sub - 2) + 1;
-                        *reinterpret_cast<uint2 *>(pl + (size_t)pi * p.K + 32 * (k8 >> 2) + 8 * chunk) =
+                        *reinterpret_cast<uint2 *>(pl + (size_t)pi * plane + 32 * (k8 >> 2) + 8 * chunk) =
                             make_uint2(prmt(lo, hi, 0x5140u), prmt(lo, hi, 0x7362u));
                     }
                 } else {
 #pragma unroll
                     for (int pi = 0; pi < 4; ++pi)
-                        *reinterpret_cast<uint2 *>(pl + (size_t)pi * p.K + 8 * k8) = make_uint2(d[pi][0], d[pi][1]);
+                        *reinterpret_cast<uint2 *>(pl + (size_t)pi * plane + 8 * k8) = make_uint2(d[pi][0], d[pi][1]);
                 }
                 if (Dec::kSumGroup == 32) {
                     s += __shfl_xor_sync(0xffffffffu, s, 1);
@@ -771,6 +941,12 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
                     s += __shfl_xor_sync(0xffffffffu, s, 1);
                     if ((threadIdx.x & 1) == 0) sm[k8 >> 1] = s;
                 }
+            };
+#pragma unroll
+            for (int q = 0; q < kXChunks; ++q)
+                if (x0 + q * xthreads < p.K / 8) digits(x0 + q * xthreads, xs[q]);
+            if constexpr (kIn > 1) {
+                for (int k8 = x0 + kXChunks * xthreads; k8 < p.K / 8; k8 += xthreads) { float v[8]; load8(k8, v); digits(k8, v); }
             }
             asm volatile("bar.sync 1, %0;" ::"r"(cthreads) : "memory");
             asm volatile("" : "+r"(b_hi), "+r"(b_lo), "+r"(sums));      // reads of the new planes stay behind the barrier
@@ -782,25 +958,36 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
         if (!dead && !mbar_wait_warp<kTryWaitHintNs>(&ctl.full[slot], c_phase, &ctl.abort)) dead = true;
         if (++c_slot == (uint32_t)D) { c_slot = 0; c_phase ^= 1u; }
         if (++c_buf == (uint32_t)(D + 1)) c_buf = 0;
-        float acc[kGroupsPerWarp][2];
+        float acc[kGroupsPerWarp][kIn > 1 ? kIn / 2 : 1][2];               // [group][input pair][row]
         int bad[kGroupsPerWarp];
 #pragma unroll
-        for (int gi = 0; gi < kGroupsPerWarp; ++gi) { acc[gi][0] = acc[gi][1] = 0.0f; bad[gi] = 0; }
+        for (int gi = 0; gi < kGroupsPerWarp; ++gi) {
+            bad[gi] = 0;
+#pragma unroll
+            for (int pr = 0; pr < (kIn > 1 ? kIn / 2 : 1); ++pr) acc[gi][pr][0] = acc[gi][pr][1] = 0.0f;
+        }
         const uint32_t first = warp_rows * (uint32_t)rw;                     // this warp's first row within the tile
         if (!dead && first < nrows) {
             uint32_t base = ctl.stage[slot] + (first + (uint32_t)l.g) * row_bytes + (uint32_t)(unit0 * Dec::kBlockBytes);
             asm volatile("" : "+r"(base));                              // reads of the stage stay behind the wait above
             for (int u = 0; u < my_units; ++u) {
                 BUnit bmem;
-                if (!kBReg) load_b(bmem, u);
+                if (!kBReg && kIn == 1) load_b(bmem, u);
                 const BUnit &b = kBReg ? breg : bmem;
                 auto groups = [&](auto odd) {
 #pragma unroll
                     for (int gi = 0; gi < kGroupsPerWarp; ++gi) {
                         // groups past a ragged tile's last row decode stale bytes; their results are never stored
                         const uint32_t r0 = base + (uint32_t)(kRows * gi) * row_bytes + (uint32_t)(u * Dec::kBlockBytes);
-                        Dec::template unit<decltype(odd)::value>(r0, r0 + second, b, l, sums + (uint32_t)(u * kSumsPerUnit * 4), acc[gi],
-                                                                 bad[gi]);
+                        if constexpr (kIn == 1) {
+                            Dec::template unit<decltype(odd)::value>(r0, r0 + second, b, l, sums + (uint32_t)(u * kSumsPerUnit * 4), acc[gi][0], bad[gi]);
+                        } else {
+                            // column n = lane >> 2 of pair 0: digit plane n & 3 of input n >> 2; sums of the input this lane's results belong to
+                            const uint32_t n = (uint32_t)lane >> 2, k0 = (uint32_t)((unit0 + u) * Dec::kBlockK), per_input = (uint32_t)(p.K / 16) * 4u;
+                            const DenseB db{ctl.planes + n * (uint32_t)plane + k0 + 8u * (uint32_t)l.t, 8u * (uint32_t)plane,
+                                            sums + (uint32_t)(u * kSumsPerUnit * 4) + (uint32_t)(l.t >> 1) * per_input, 2u * per_input, (l.t & 1) != 0};
+                            Dec::template dense<kIn, 0>(r0, r0 + second, db, l, acc[gi], bad[gi]);
+                        }
                     }
                 };
                 if (Dec::kParity && ((unit0 + u) & 1)) groups(std::integral_constant<int, 1>{});
@@ -810,14 +997,24 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
         // this warp is done with the stage
         __syncwarp();
         if (lane == 0) mbar_arrive(&ctl.empty[slot]);
-        float *red = red_all + ((size_t)buf * consumers + warp) * warp_rows;
+        float *red = red_all + ((size_t)buf * kIn * consumers + warp) * warp_rows;           // [input][warp][rows]
 #pragma unroll
         for (int gi = 0; gi < kGroupsPerWarp; ++gi) {
-            float a0 = acc[gi][0], a1 = acc[gi][1];
-            a0 += __shfl_xor_sync(0xffffffffu, a0, 1); a0 += __shfl_xor_sync(0xffffffffu, a0, 2);
-            a1 += __shfl_xor_sync(0xffffffffu, a1, 1); a1 += __shfl_xor_sync(0xffffffffu, a1, 2);
-            float *to = red + (uint32_t)(kRows * gi) + (uint32_t)l.g;
-            if (l.t == 0) { to[0] = a0; if (whole) to[8] = a1; }
+            if constexpr (kIn == 1) {
+                float a0 = acc[gi][0][0], a1 = acc[gi][0][1];
+                a0 += __shfl_xor_sync(0xffffffffu, a0, 1); a0 += __shfl_xor_sync(0xffffffffu, a0, 2);
+                a1 += __shfl_xor_sync(0xffffffffu, a1, 1); a1 += __shfl_xor_sync(0xffffffffu, a1, 2);
+                float *to = red + (uint32_t)(kRows * gi) + (uint32_t)l.g;
+                if (l.t == 0) { to[0] = a0; if (whole) to[8] = a1; }
+            } else {
+#pragma unroll
+                for (int pr = 0; pr < kIn / 2; ++pr) {
+                    const float a0 = fmaf(acc[gi][pr][0], 16384.0f, __shfl_xor_sync(0xffffffffu, acc[gi][pr][0], 1));
+                    const float a1 = fmaf(acc[gi][pr][1], 16384.0f, __shfl_xor_sync(0xffffffffu, acc[gi][pr][1], 1));
+                    float *to = red + (size_t)(2 * pr + (l.t >> 1)) * consumers * warp_rows + (uint32_t)(kRows * gi) + (uint32_t)l.g;
+                    if ((l.t & 1) == 0) { to[0] = a0; if (whole) to[8] = a1; }
+                }
+            }
             // a malformed block scale only counts for rows that exist
             const uint32_t r_lo = first + (uint32_t)(kRows * gi) + (uint32_t)l.g, r_hi = r_lo + (whole ? 8u : 0u);
             if (((bad[gi] & 1) && r_lo < nrows) || ((bad[gi] & 2) && r_hi < nrows)) raise(p.status, YVEX_B200_STATUS_NUMERIC);
@@ -831,7 +1028,7 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
 struct StreamShape { int slices, units_per_slice, row_warps, consumers, depth, groups, group_rows; uint32_t stage_bytes, smem_bytes, pitch; };
 
 // K-slices (consumer warps along K), units per slice, warps along the rows of a stage and the deepest ring that fits.
-inline bool stream_shape(unsigned q, uint64_t width, uint64_t row_bytes, StreamShape &sh) {
+inline bool stream_shape(unsigned q, uint64_t width, uint64_t row_bytes, StreamShape &sh, int inputs = 1) {
     const bool tables = q == Q_IQ2_XXS;
     const int units = (int)(width / 256);
     if (!units || width % 256 || width > 8192) return false;
@@ -852,7 +1049,7 @@ inline bool stream_shape(unsigned q, uint64_t width, uint64_t row_bytes, StreamS
     // (last, groups of eight rows: Q8_0 rows of 7168 weights are 7616 bytes, and sixteen of them leave no room for a second stage.
     // Half of every MMA is then idle, but the generic kernel such rows used to take measured 21.1 ms on 128 matrices of
     // 2048 x 7168, this path 0.78 ms = 2.56 TB/s)
-    for (int step = 0; step < (q == Q_Q8_0 ? 3 : 2); ++step) {
+    for (int step = inputs > 1 ? 1 : 0; step < (q == Q_Q8_0 && inputs == 1 ? 3 : 2); ++step) {
         sh.groups = step == 0 ? kMaxGroupsPerWarp : 1;
         sh.group_rows = step < 2 ? kTileRows : kTileRows / 2;
         sh.stage_bytes = (uint32_t)(sh.group_rows * sh.groups * sh.row_warps * sh.pitch);
@@ -860,8 +1057,29 @@ inline bool stream_shape(unsigned q, uint64_t width, uint64_t row_bytes, StreamS
             // every piece is rounded up to 128 bytes; with tables one piece may have to step over the table window,
             // which starts at most 64 KiB - 1 into the allocation (what lies before it stays usable)
             const uint32_t pieces = (uint32_t)sh.depth * (sh.stage_bytes + 16 + 128) +
-                                    stream_small_bytes((int)width, sh.consumers, sh.depth, sh.units_per_slice, sh.groups) + 5 * 128;
-            sh.smem_bytes = tables ? pieces + kTableBytes + sh.stage_bytes + 16 + 128 : pieces;
+                                    stream_small_bytes((int)width, sh.consumers, sh.depth, sh.units_per_slice, sh.groups, inputs) + 5 * 128;
+            uint32_t largest = sh.stage_bytes + 16;         // the piece that steps over leaves a gap of up to its own size
+            for (uint32_t piece : {(uint32_t)(inputs * 4) * (uint32_t)(width + kPlanePad), (uint32_t)(inputs * (sh.depth + 1) * sh.consumers * sh.groups * kTileRows) * 4u})
+                largest = largest < piece ? piece : largest;
+            sh.smem_bytes = tables ? pieces + kTableBytes + largest + 128 : pieces;
+            // (four rows' planes are the largest piece by far, and that bound would leave the gap before the table unused: place the
+            // pieces as the kernel will, for every start the dynamic window may have)
+            if (tables && inputs > 1) {
+                sh.smem_bytes = 0;
+                for (uint32_t base = 1024; base <= 4096; base += 128) {
+                    const uint32_t tab = (base + 0xffffu) & ~0xffffu;
+                    uint32_t cur = base;
+                    auto take = [&](uint32_t bytes) { cur = (cur + 127u) & ~127u; if (cur < tab + kTableBytes && cur + bytes > tab) cur = tab + kTableBytes; cur += bytes; };
+                    for (int i = 0; i < sh.depth; ++i) take(sh.stage_bytes + 16);
+                    take((uint32_t)(inputs * 4) * (uint32_t)(width + kPlanePad));
+                    take((uint32_t)(256 * sh.units_per_slice + 16));
+                    take((uint32_t)(inputs * (int)(width / 16)) * 4u);
+                    take((uint32_t)(inputs * (sh.depth + 1) * sh.consumers * sh.groups * kTileRows) * 4u);
+                    const uint32_t end = cur > tab + kTableBytes ? cur : tab + kTableBytes;
+                    sh.smem_bytes = sh.smem_bytes > end - base ? sh.smem_bytes : end - base;
+                }
+                sh.smem_bytes += 128;
+            }
             if (tables && sh.smem_bytes < 2 * kTableBytes) sh.smem_bytes = 2 * kTableBytes;
             if (sh.smem_bytes <= limit) return true;
         }
@@ -879,25 +1097,26 @@ inline bool stream_eligible(unsigned q, uint64_t rows, uint64_t width, uint64_t 
            stream_shape(q, width, row_bytes, sh);
 }
 
-template <class Dec, bool kBReg, int kG, int kRows = kTileRows>
+template <class Dec, bool kBReg, int kG, int kIn, int kRows = kTileRows>
 inline int stream_launch_v(StreamParams &p, const StreamShape &sh, cudaStream_t stream) {
     static SmemOptIn opt_in;
-    if (opt_in.ensure(gemv_stream_kernel<Dec, kBReg, kG, kRows>, 226 * 1024) != OK) return ERR_BACKEND;
+    if (opt_in.ensure(gemv_stream_kernel<Dec, kBReg, kG, kIn, kRows>, 226 * 1024) != OK) return ERR_BACKEND;
     const uint64_t tile_rows = (uint64_t)kRows * kG * sh.row_warps;
     const uint64_t tasks = (uint64_t)p.count * ((p.rows + tile_rows - 1) / tile_rows);
     const unsigned grid = (unsigned)(tasks < (uint64_t)kSmCount ? tasks : (uint64_t)kSmCount);
-    if (launch_pdl(gemv_stream_kernel<Dec, kBReg, kG, kRows>, dim3(grid), dim3(32 * (sh.consumers + 1)), sh.smem_bytes, stream, p) != cudaSuccess)
+    if (launch_pdl(gemv_stream_kernel<Dec, kBReg, kG, kIn, kRows>, dim3(grid), dim3(32 * (sh.consumers + 1)), sh.smem_bytes, stream, p) != cudaSuccess)
         return ERR_BACKEND;
     return launch_status(1);
 }
 
 template <class Dec>
-inline int stream_launch_t(StreamParams &p, const StreamShape &sh, cudaStream_t stream) {
+inline int stream_launch_t(StreamParams &p, const StreamShape &sh, int inputs, cudaStream_t stream) {
+    if (inputs > 1) return stream_launch_v<Dec, false, 1, kMaxInputs>(p, sh, stream);
     if constexpr (Dec::kQtype == Q_Q8_0)
-        if (sh.group_rows == kTileRows / 2) return stream_launch_v<Dec, false, 1, kTileRows / 2>(p, sh, stream);
+        if (sh.group_rows == kTileRows / 2) return stream_launch_v<Dec, false, 1, 1, kTileRows / 2>(p, sh, stream);
     const bool breg = sh.units_per_slice == 1;
-    if (sh.groups == 2) return breg ? stream_launch_v<Dec, true, 2>(p, sh, stream) : stream_launch_v<Dec, false, 2>(p, sh, stream);
-    return breg ? stream_launch_v<Dec, true, 1>(p, sh, stream) : stream_launch_v<Dec, false, 1>(p, sh, stream);
+    if (sh.groups == 2) return breg ? stream_launch_v<Dec, true, 2, 1>(p, sh, stream) : stream_launch_v<Dec, false, 2, 1>(p, sh, stream);
+    return breg ? stream_launch_v<Dec, true, 1, 1>(p, sh, stream) : stream_launch_v<Dec, false, 1, 1>(p, sh, stream);
 }
 
 struct StreamActivation { const float *up; const float *weight; float limit; };
@@ -907,9 +1126,15 @@ inline int stream_launch(unsigned q, const uint8_t *enc, uint64_t matrix_stride,
                          uint64_t out_stride, int round_bf16, int *status, cudaStream_t stream,
                          const uint8_t *const *matrix_ptrs = nullptr, const uint32_t *x_rows = nullptr,
                          const StreamActivation *act = nullptr) {
+    // Several input rows of ONE matrix: passes of up to four rows that share each tile's decode, from two rows on (a pass
+    // costs 1.3 to 1.7 of a single row's) and where four rows' planes leave room for a ring.
     StreamShape sh;
-    if (!stream_shape(q, width, row_bytes, sh)) return ERR_BOUNDS;
+    const bool shared = count > 1 && matrix_stride == 0 && !matrix_ptrs && !act;
+    const int inputs = shared && stream_shape(q, width, row_bytes, sh, kMaxInputs) && sh.consumers >= kMaxInputs ? kMaxInputs : 1;
+    if (inputs == 1 && !stream_shape(q, width, row_bytes, sh)) return ERR_BOUNDS;
     StreamParams p{};
+    p.inputs = (uint32_t)count;
+    if (inputs > 1) count = (count + kMaxInputs - 1) / kMaxInputs;
     p.matrix_ptrs = matrix_ptrs; p.x_rows = x_rows;
     if (act) {
         if (x_rows || (reinterpret_cast<uintptr_t>(act->up) & 15u)) return ERR_INVALID_ARG;
@@ -921,11 +1146,11 @@ inline int stream_launch(unsigned q, const uint8_t *enc, uint64_t matrix_stride,
     p.x = x; p.x_stride = x_stride; p.additive = additive; p.out = out; p.out_stride = out_stride;
     p.round_bf16 = round_bf16; p.status = status;
     switch (q) {
-    case Q_IQ2_XXS: return stream_launch_t<StreamIq2>(p, sh, stream);
-    case Q_Q4_K: return stream_launch_t<StreamQ4k>(p, sh, stream);
-    case Q_Q8_0: return stream_launch_t<StreamQ80>(p, sh, stream);
-    case Q_Q2_K: return stream_launch_t<StreamQ2k>(p, sh, stream);
-    case Q_MXFP4: return stream_launch_t<StreamMxfp4>(p, sh, stream);
+    case Q_IQ2_XXS: return stream_launch_t<StreamIq2>(p, sh, inputs, stream);
+    case Q_Q4_K: return stream_launch_t<StreamQ4k>(p, sh, inputs, stream);
+    case Q_Q8_0: return stream_launch_t<StreamQ80>(p, sh, inputs, stream);
+    case Q_Q2_K: return stream_launch_t<StreamQ2k>(p, sh, inputs, stream);
+    case Q_MXFP4: return stream_launch_t<StreamMxfp4>(p, sh, inputs, stream);
     default: return ERR_UNSUPPORTED;
     }
 }
