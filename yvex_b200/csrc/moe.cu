@@ -12,6 +12,8 @@ namespace yb {
 
 // ---- ingress: x -> bf16-exact f32 rows ----------------------------------------------------------
 __global__ void ingress_round_kernel(const float *x, float *xr, __half *xr_h, uint64_t n, int *status) {
+    pdl_wait();
+    pdl_trigger();
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
         float v = x[i];
@@ -52,6 +54,8 @@ __global__ void router_logits_kernel(const float *router, const float *xr, uint6
 constexpr int kRouterTile = 8, kRouterTileWarps = 4;
 __global__ void __launch_bounds__(32 * kRouterTileWarps)
 router_tile_kernel(const float *router, const float *xr, uint64_t rows, uint64_t experts, uint64_t hidden, int ksplit, float *logits, int *status) {
+    pdl_wait();
+    pdl_trigger();
     constexpr int R = kRouterTile;
     __shared__ double part[kRouterTileWarps][R * R];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -382,8 +386,9 @@ static int route_into(const MoeGeom &g, const yvex_b200_moe_weights *w, const fl
             const uint64_t rt = (rows + kRouterTile - 1) / kRouterTile, et = (g.experts + kRouterTile - 1) / kRouterTile;
             const int ksplit = rt * et < (uint64_t)kSmCount * 8 ? kRouterTileWarps : 1;      // one warp per tile is at least 8 warps per SM
             const uint64_t per = (uint64_t)(kRouterTileWarps / ksplit);
-            router_tile_kernel<<<dim3((unsigned)rt, (unsigned)((et + per - 1) / per)), 32 * kRouterTileWarps, 0, s>>>(
-                w->router, xr, rows, g.experts, g.hidden, ksplit, logits_ws, status);
+            if (launch_pdl(router_tile_kernel, dim3((unsigned)rt, (unsigned)((et + per - 1) / per)), dim3(32 * kRouterTileWarps), 0, s, w->router, xr, rows,
+                           g.experts, g.hidden, ksplit, logits_ws, status) != cudaSuccess)
+                return ERR_BACKEND;
         } else {
             router_logits_kernel<<<grid_for(rows * g.experts, 8, 8), 256, 0, s>>>(w->router, xr, rows, g.experts, g.hidden, logits_ws, status);
         }
@@ -392,8 +397,9 @@ static int route_into(const MoeGeom &g, const yvex_b200_moe_weights *w, const fl
     } else if (!logits_in) {
         return ERR_INVALID_ARG;
     }
-    route_rows_kernel<<<(unsigned)((rows + 3) / 4), 128, 0, s>>>(g, logits, nullptr, w->bias, w->hash_table, token_ids, rows,
-                                                                selected, weights, status, RouteTables{});
+    if (launch_pdl(route_rows_kernel, dim3((unsigned)((rows + 3) / 4)), dim3(128), 0, s, g, logits, nullptr, w->bias, w->hash_table, token_ids, rows, selected,
+                   weights, status, RouteTables{}) != cudaSuccess)
+        return ERR_BACKEND;
     return launch_status(launches);
 }
 
@@ -414,7 +420,7 @@ int yb::moe_ingress_and_route(const MoeGeom &g, const MoeWeights &w, const MoeWo
         return launch_status(2);
     }
     if (tables) tables->enabled = 0;
-    ingress_round_kernel<<<grid_for(n, 256, 8), 256, 0, s>>>(x, ws.xr, ws.xr_h, n, status);
+    if (launch_pdl(ingress_round_kernel, dim3(grid_for(n, 256, 8)), dim3(256), 0, s, x, ws.xr, ws.xr_h, n, status) != cudaSuccess) return ERR_BACKEND;
     int rc = launch_status(1);
     if (rc != OK) return rc;
     return route_into(g, &w, ws.xr, logits, token_ids, rows, ws.logits, ws.selected, ws.weights, status, s);

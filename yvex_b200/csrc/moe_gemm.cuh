@@ -324,6 +324,7 @@ moe_grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, GemmParams p) {
     constexpr int kProducerWarps = Plan::kProducerWarps, kAStages = Plan::kAStages, kBStages = Plan::kBStages, kRawStages = Plan::kRawStages;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     if (smem_u32(smem_raw) & 1023u) {                           // uniform: nothing has been set up yet
+        pdl_wait();
         if (threadIdx.x == 0) raise(p.status, YVEX_B200_STATUS_TIMEOUT);
         return;
     }
@@ -356,6 +357,8 @@ moe_grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, GemmParams p) {
     tc_fence_after();
     const uint32_t tmem = sm->tmem_base;
     volatile int *abort = &sm->abort;
+    pdl_wait();                                                 // tile list, activations and sums come from the kernels before
+    pdl_trigger();
 
     const int ncb = *p.num_colblocks;
     constexpr int kRowsPerMat = kFused ? kTileM / 2 : kTileM;      // weight rows of one matrix in a tile
@@ -551,19 +554,19 @@ moe_grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, GemmParams p) {
                     else dscale[(sb_it % kScaleRing) * kTileM + row] = dd.x;
                     if (bad) raise(p.status, YVEX_B200_STATUS_NUMERIC);
                 }
-                // a chunk's words and table entries are read before the wait for its stage
+                // a chunk's words and table entries are read, and its first half converted, before the wait for its stage
+                // (2 % against converting all of it behind the wait; converting all of it before is no better)
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     typename Dec::Half half;
                     Dec::fetch(blk, c, h, tab, lane4, half);
+                    uint32_t v[8];
+                    Dec::convert(half, 0, v);
                     if (!mbar_wait_warp(&sm->a_empty[a.s], a.ph ^ 1u, abort)) goto done;
                     tc_fence_after();
-#pragma unroll
-                    for (int q = 0; q < 2; ++q) {
-                        uint32_t v[8];
-                        Dec::convert(half, q, v);
-                        tmem_st8(a_at + a.s * (kChunkK / 2) + 8u * (uint32_t)q, v);
-                    }
+                    tmem_st8(a_at + a.s * (kChunkK / 2), v);
+                    Dec::convert(half, 1, v);
+                    tmem_st8(a_at + a.s * (kChunkK / 2) + 8u, v);
                     tmem_st_wait();
                     tc_fence_before();
                     __syncwarp();

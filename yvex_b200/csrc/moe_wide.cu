@@ -24,6 +24,8 @@ namespace yb {
 // ---- pair list of the single-device layer ----------------------------------------------------------
 __global__ void wide_pairs_kernel(const int32_t *selected, const float *weights, uint64_t tokens, uint64_t topk, int experts,
                                   int *expert_of_pair, int *src_of_pair, float *weight_of_pair) {
+    pdl_wait();
+    pdl_trigger();
     const uint64_t routed = tokens * topk, total = routed + tokens;
     for (uint64_t p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; p < total; p += (uint64_t)gridDim.x * blockDim.x) {
         const bool r = p < routed;
@@ -45,6 +47,8 @@ __global__ void wide_list_kernel(const int32_t *ids, const float *weights, uint6
 
 // ---- permute ---------------------------------------------------------------------------------------
 __global__ void wide_count_kernel(const int *expert_of_pair, uint64_t pairs, int bins, int *counts, int *status) {
+    pdl_wait();
+    pdl_trigger();
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < pairs; i += (uint64_t)gridDim.x * blockDim.x) {
         const int e = expert_of_pair[i];
         if (e < 0 || e >= bins) raise(status, YVEX_B200_STATUS_ARGUMENT);
@@ -58,6 +62,8 @@ __global__ void wide_count_kernel(const int *expert_of_pair, uint64_t pairs, int
 // Lanes take 32 consecutive bins at a time; shuffle scans give each bin its first row and block.
 __global__ void wide_plan_kernel(const int *counts, int experts, uint64_t pairs, int *offsets, ColBlock *blocks_gu,
                                  ColBlock *blocks_down, int *num_blocks, int max_blocks, int tile_gu, int tile_down, int *status) {
+    pdl_wait();
+    pdl_trigger();
     ColBlock *blocks = blockIdx.x ? blocks_down : blocks_gu;
     const int tile_n = blockIdx.x ? tile_down : tile_gu, lane = threadIdx.x;
     const int per_group = kGroupRows / tile_n;                              // groups of <= kGroupRows token rows
@@ -98,6 +104,8 @@ __global__ void wide_plan_kernel(const int *counts, int experts, uint64_t pairs,
 
 // One CTA per bin: stable compaction of the pairs routed to it (ascending pair index).
 __global__ void wide_scatter_kernel(const int *expert_of_pair, uint64_t pairs, const int *offsets, int *perm, int *pos_of_pair) {
+    pdl_wait();
+    pdl_trigger();
     const int e = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     __shared__ int warp_count[32];
     __shared__ int base;
@@ -131,6 +139,8 @@ __global__ void wide_scatter_kernel(const int *expert_of_pair, uint64_t pairs, c
 __global__ void wide_gather_kernel(const __half *rows_h, const int *perm, const int *src_of_pair, const float *weight_of_pair,
                                    uint64_t pairs, uint64_t hidden, __half *act_h, float *weight_sorted, uint64_t src_pitch,
                                    int group, __half *act_sums, int *status) {
+    pdl_wait();
+    pdl_trigger();
     const uint32_t chunks = (uint32_t)(hidden / 8);           // 16-byte chunks per row
     for (uint64_t row = blockIdx.x; row < pairs; row += gridDim.x) {          // a CTA copies whole rows
         const int pair = perm[row];
@@ -197,6 +207,8 @@ __global__ void wide_list_payload_kernel(const uint8_t *payload, uint64_t pitch,
 // (inter is a multiple of 256, so rows start on warp boundaries of the flattened chunk index).
 __global__ void __launch_bounds__(256)
 wide_mid_sums_kernel(const __half *mid_h, uint64_t rows, uint64_t inter, int group, __half *sums) {
+    pdl_wait();
+    pdl_trigger();
     const uint64_t chunks = rows * (inter / 8), stride = (uint64_t)gridDim.x * blockDim.x;
     const uint32_t per_row = (uint32_t)(inter / 8);
     constexpr int kUnroll = 4;
@@ -233,6 +245,8 @@ __global__ void __launch_bounds__(128)
 wide_combine_kernel(const uint16_t *y, const uint16_t *y_shared, const int *pos, const int *pos_shared,
                     uint64_t tokens, uint64_t topk, uint64_t hidden, float *out, float *routed_out = nullptr,
                     float *shared_out = nullptr) {
+    pdl_wait();
+    pdl_trigger();
     const uint32_t chunks = (uint32_t)(hidden / 8), c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= chunks) return;
     for (uint64_t t = blockIdx.y; t < tokens; t += gridDim.y) {
@@ -395,7 +409,9 @@ static int launch_gemm(const GemmMaps &map, const GemmParams &p, cudaStream_t s)
     const size_t smem = GemmPlan<Dec>::kBytes;
     static SmemOptIn opt_in;
     if (opt_in.ensure(moe_grouped_gemm_kernel<Dec, kFused>, (int)smem) != OK) return ERR_BACKEND;
-    moe_grouped_gemm_kernel<Dec, kFused><<<g_gemm_ctas.load(std::memory_order_relaxed), GemmPlan<Dec>::kThreads, smem, s>>>(map, p);
+    if (launch_pdl(moe_grouped_gemm_kernel<Dec, kFused>, dim3((unsigned)g_gemm_ctas.load(std::memory_order_relaxed)), dim3(GemmPlan<Dec>::kThreads), smem, s, map, p) !=
+        cudaSuccess)
+        return ERR_BACKEND;
     return launch_status(1);
 }
 
@@ -457,14 +473,16 @@ static int run_pair_list(const MoeGeom &g, const MoeWeights &w, const PairWorksp
     const Geometry gg = geometry_of(g.gate_qtype), dg = geometry_of(g.down_qtype);
     const int bins = (int)g.experts + 1;
     cudaMemsetAsync(pw.counts, 0, (g.experts + 2) * 4, s);
-    wide_count_kernel<<<grid_for(pairs, 256, 4), 256, 0, s>>>(pw.expert_of_pair, pairs, bins, pw.counts, status);
-    wide_plan_kernel<<<2, 32, 0, s>>>(pw.counts, (int)g.experts, pairs, pw.offsets, pw.blocks, pw.blocks_down, pw.num_blocks,
+    // each launch of the chain with programmatic stream serialization: its latency runs under the kernel before
+    cudaError_t e = launch_pdl(wide_count_kernel, dim3(grid_for(pairs, 256, 4)), dim3(256), 0, s, pw.expert_of_pair, pairs, bins, pw.counts, status);
+    if (e == cudaSuccess) e = launch_pdl(wide_plan_kernel, dim3(2), dim3(32), 0, s, pw.counts, (int)g.experts, pairs, pw.offsets, pw.blocks, pw.blocks_down, pw.num_blocks,
                                       pw.max_blocks, gemm_tile_n(g.gate_qtype), gemm_tile_n(g.down_qtype), status);
-    wide_scatter_kernel<<<(unsigned)bins, 512, 0, s>>>(pw.expert_of_pair, pairs, pw.offsets, pw.perm, pw.pos_of_pair);
+    if (e == cudaSuccess) e = launch_pdl(wide_scatter_kernel, dim3((unsigned)bins), dim3(512), 0, s, pw.expert_of_pair, pairs, pw.offsets, pw.perm, pw.pos_of_pair);
     const auto sum_group = [](unsigned q) { return q == Q_Q4_K ? 32 : q == Q_Q2_K ? 16 : 0; };
-    wide_gather_kernel<<<grid_for(pairs, 1, 16), 128, 0, s>>>(rows_h, pw.perm, pw.src_of_pair, pw.weight_of_pair, pairs, g.hidden,
-                                                              pw.act_h, pw.weight_sorted, src_pitch, sum_group(g.gate_qtype),
-                                                              pw.act_sums, status);
+    if (e == cudaSuccess)
+        e = launch_pdl(wide_gather_kernel, dim3(grid_for(pairs, 1, 16)), dim3(128), 0, s, rows_h, pw.perm, pw.src_of_pair, pw.weight_of_pair, pairs, g.hidden,
+                       pw.act_h, pw.weight_sorted, src_pitch, sum_group(g.gate_qtype), pw.act_sums, status);
+    if (e != cudaSuccess) return ERR_BACKEND;
     if (home_bases)
         wide_dest_kernel<<<grid_for(pairs, 256, 4), 256, 0, s>>>(reinterpret_cast<const uint8_t *>(rows_h), src_pitch, g.hidden, pw.perm,
                                                                pairs, home_bases, home_world, home_pairs, pw.dest, status);
@@ -506,8 +524,8 @@ static int run_sorted_gemms(const MoeGeom &g, const MoeWeights &w, const PairWor
     mark_phase(3, s);
 
     const int group = sum_group(g.down_qtype);
-    if (group)
-        wide_mid_sums_kernel<<<grid_for(pairs * (g.inter / 8), 256, 8), 256, 0, s>>>(pw.mid_h, pairs, g.inter, group, pw.sums);
+    if (group && launch_pdl(wide_mid_sums_kernel, dim3(grid_for(pairs * (g.inter / 8), 256, 8)), dim3(256), 0, s, pw.mid_h, pairs, g.inter, group, pw.sums) != cudaSuccess)
+        return ERR_BACKEND;
     mark_phase(6, s);                                   // sums done (an extra probe point, outside the 0..5 sequence)
     GemmParams dn{};
     dn.row_bytes = (uint32_t)(g.inter / dg.elems * dg.bytes);
@@ -567,12 +585,14 @@ extern "C" int yvex_b200_moe_wide_parts(const yvex_b200_moe_geometry *geom, cons
         const uint64_t pairs = rows * (g.topk + 1), routed = rows * g.topk;
         pair_layout(g, pairs, base, &pw);
         pw.rebase(workspace);
-        wide_pairs_kernel<<<grid_for(pairs, 256, 4), 256, 0, s>>>(ws.selected, ws.weights, rows, g.topk, (int)g.experts,
-                                                                pw.expert_of_pair, pw.src_of_pair, pw.weight_of_pair);
+        if (launch_pdl(wide_pairs_kernel, dim3(grid_for(pairs, 256, 4)), dim3(256), 0, s, ws.selected, ws.weights, rows, g.topk, (int)g.experts, pw.expert_of_pair,
+                       pw.src_of_pair, pw.weight_of_pair) != cudaSuccess)
+            return ERR_BACKEND;
         rc = run_pair_list(g, *w, pw, ws.xr_h, pairs, status, s);
         if (rc != OK) return rc;
-        wide_combine_kernel<<<dim3((unsigned)((g.hidden / 8 + 127) / 128), (unsigned)grid_for(rows, 1, 16)), 128, 0, s>>>(
-            pw.y, pw.y, pw.pos_of_pair, pw.pos_of_pair + routed, rows, g.topk, g.hidden, out, routed_out, shared_out);
+        if (launch_pdl(wide_combine_kernel, dim3((unsigned)((g.hidden / 8 + 127) / 128), (unsigned)grid_for(rows, 1, 16)), dim3(128), 0, s, pw.y, pw.y,
+                       pw.pos_of_pair, pw.pos_of_pair + routed, rows, g.topk, g.hidden, out, routed_out, shared_out) != cudaSuccess)
+            return ERR_BACKEND;
         mark_phase(5, s);
         rc = launch_status(2);
     } else {
