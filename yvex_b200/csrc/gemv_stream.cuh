@@ -1121,17 +1121,24 @@ inline int stream_launch_t(StreamParams &p, const StreamShape &sh, int inputs, c
 
 struct StreamActivation { const float *up; const float *weight; float limit; };
 
+// Input rows one pass over a matrix serves (0: no shape fits), and its shape. Several input rows of ONE matrix: passes of up to
+// four rows that share each tile's decode, from two rows on (a pass costs 1.3 to 1.7 of a single row's) and where four rows'
+// planes leave room for a ring. Rows named by a table (x_rows) are one to a matrix: a pass takes consecutive ones.
+inline int pass_inputs(unsigned q, uint64_t width, uint64_t row_bytes, uint64_t count, uint64_t matrix_stride, const uint8_t *const *matrix_ptrs,
+                       const uint32_t *x_rows, const StreamActivation *act, StreamShape &sh) {
+    const bool shared = count > 1 && matrix_stride == 0 && !matrix_ptrs && !x_rows && !act;
+    if (shared && stream_shape(q, width, row_bytes, sh, kMaxInputs) && sh.consumers >= kMaxInputs) return kMaxInputs;
+    return stream_shape(q, width, row_bytes, sh) ? 1 : 0;
+}
+
 inline int stream_launch(unsigned q, const uint8_t *enc, uint64_t matrix_stride, uint64_t count, uint64_t rows, uint64_t width,
                          uint64_t row_bytes, const float *x, uint64_t x_stride, const float *additive, float *out,
                          uint64_t out_stride, int round_bf16, int *status, cudaStream_t stream,
                          const uint8_t *const *matrix_ptrs = nullptr, const uint32_t *x_rows = nullptr,
                          const StreamActivation *act = nullptr) {
-    // Several input rows of ONE matrix: passes of up to four rows that share each tile's decode, from two rows on (a pass
-    // costs 1.3 to 1.7 of a single row's) and where four rows' planes leave room for a ring.
     StreamShape sh;
-    const bool shared = count > 1 && matrix_stride == 0 && !matrix_ptrs && !act;
-    const int inputs = shared && stream_shape(q, width, row_bytes, sh, kMaxInputs) && sh.consumers >= kMaxInputs ? kMaxInputs : 1;
-    if (inputs == 1 && !stream_shape(q, width, row_bytes, sh)) return ERR_BOUNDS;
+    const int inputs = pass_inputs(q, width, row_bytes, count, matrix_stride, matrix_ptrs, x_rows, act, sh);
+    if (!inputs) return ERR_BOUNDS;
     StreamParams p{};
     p.inputs = (uint32_t)count;
     if (inputs > 1) count = (count + kMaxInputs - 1) / kMaxInputs;
