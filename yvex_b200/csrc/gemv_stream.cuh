@@ -125,9 +125,11 @@ __device__ __forceinline__ float comb(int a_hi, int a_lo, int b_hi, int b_lo) {
 // multiplied by zeros, and one decode serves every input. Lane t of a row ends up with the upper (t even) or lower digit
 // pair of input t >> 1; the group's scale is applied there, the halves meet once per tile. (With the single-row
 // arrangement - columns of zeros outside a lane's group - four rows in one pass were bound by 64 MMAs per 256 x 16 weights
-// and no faster than four passes.) 4096 x 4096, eight rows, a pass per row against this: Q8_0 30 / 17 us, Q4_K 27 / 17,
+// and no faster than four passes.) What a decoder takes off again (MXFP4's 16 per code, the minimum of Q4_K and Q2_K) a lane
+// takes off in its own digits, by the activation sums of its own digit pair: with the whole of it on the lower pair two large
+// sums met only at the end of a slice, and inputs with a mean lost up to a decimal digit (MXFP4 6e-6 against 1e-6). 4096 x 4096, eight rows, a pass per row against this: Q8_0 30 / 17 us, Q4_K 27 / 17,
 // Q2_K 32 / 18, MXFP4 30 / 25; IQ2_XXS 65536 x 2048 148 / 66.
-struct DenseB { uint32_t at, pair, sums, sums_pair; bool low; };      // planes and sums of this lane's input (of pair 0), to the next pair
+struct DenseB { uint32_t at, pair, sums, sums_pair; };      // planes and digit-pair sums of this lane's input (of pair 0), to the next pair
 
 template <int kIn> __device__ __forceinline__ void mma_dense(const uint32_t (&a)[4], const DenseB &b, int j, int (&c)[kIn / 2][4]) {
 #pragma unroll
@@ -214,7 +216,7 @@ struct StreamIq2 {
         hi = prmt(kPos, kNeg, sel >> 16);
     }
     template <int kIn, int> __device__ __forceinline__ static void dense(uint32_t row0, uint32_t row1, const DenseB &b, const Lane &l, float (&acc)[kIn / 2][2], int &bad) {
-        float blk[kIn / 2][2] = {};
+        float blk[2][kIn / 2][2] = {};                                          // the two halves of the superblock, as in unit()
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             uint32_t g0, s0, g1, s1, a[4];
@@ -227,14 +229,14 @@ struct StreamIq2 {
             const float f0 = (float)((s0 >> 27) | 1u), f1 = (float)((s1 >> 27) | 1u);
 #pragma unroll
             for (int p = 0; p < kIn / 2; ++p) {
-                blk[p][0] = fmaf(digit_pair(c[p][0], c[p][1]), f0, blk[p][0]);
-                blk[p][1] = fmaf(digit_pair(c[p][2], c[p][3]), f1, blk[p][1]);
+                blk[j >> 2][p][0] = fmaf(digit_pair(c[p][0], c[p][1]), f0, blk[j >> 2][p][0]);
+                blk[j >> 2][p][1] = fmaf(digit_pair(c[p][2], c[p][3]), f1, blk[j >> 2][p][1]);
             }
         }
         const float d0 = f16_bits_to_float((uint16_t)lds16(row0)), d1 = f16_bits_to_float((uint16_t)lds16(row1));
         bad |= (scale_bad(d0) ? 1 : 0) | (scale_bad(d1) ? 2 : 0);
 #pragma unroll
-        for (int p = 0; p < kIn / 2; ++p) { acc[p][0] = fmaf(blk[p][0], 0.125f * d0, acc[p][0]); acc[p][1] = fmaf(blk[p][1], 0.125f * d1, acc[p][1]); }
+        for (int p = 0; p < kIn / 2; ++p) { acc[p][0] = fmaf(blk[0][p][0] + blk[1][p][0], 0.125f * d0, acc[p][0]); acc[p][1] = fmaf(blk[0][p][1] + blk[1][p][1], 0.125f * d1, acc[p][1]); }
     }
 };
 
@@ -303,7 +305,7 @@ struct StreamQ4k {
         acc[1] += fmaf(d1, blk1, -n1 * min1);
     }
     template <int kIn, int> __device__ __forceinline__ static void dense(uint32_t row0, uint32_t row1, const DenseB &b, const Lane &l, float (&acc)[kIn / 2][2], int &bad) {
-        float blk[kIn / 2][2] = {}, mn[kIn / 2][2] = {};
+        float blk[2][kIn / 2][2] = {}, mn[2][kIn / 2][2] = {};
         const uint4 head0 = lds128(row0), head1 = lds128(row1);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -319,18 +321,20 @@ struct StreamQ4k {
 #pragma unroll
             for (int p = 0; p < kIn / 2; ++p) {
                 const float xs = ldsf(b.sums + p * b.sums_pair + 4 * j);
-                blk[p][0] = fmaf(digit_pair(c[p][0], c[p][1]), (float)sc0, blk[p][0]);
-                blk[p][1] = fmaf(digit_pair(c[p][2], c[p][3]), (float)sc1, blk[p][1]);
-                mn[p][0] = fmaf((float)q0, xs, mn[p][0]);
-                mn[p][1] = fmaf((float)q1, xs, mn[p][1]);
+                blk[j >> 2][p][0] = fmaf(digit_pair(c[p][0], c[p][1]), (float)sc0, blk[j >> 2][p][0]);
+                blk[j >> 2][p][1] = fmaf(digit_pair(c[p][2], c[p][3]), (float)sc1, blk[j >> 2][p][1]);
+                mn[j >> 2][p][0] = fmaf((float)q0, xs, mn[j >> 2][p][0]);
+                mn[j >> 2][p][1] = fmaf((float)q1, xs, mn[j >> 2][p][1]);
             }
         }
         const float d0 = f16_bits_to_float((uint16_t)head0.x), n0 = f16_bits_to_float((uint16_t)(head0.x >> 16));
         const float d1 = f16_bits_to_float((uint16_t)head1.x), n1 = f16_bits_to_float((uint16_t)(head1.x >> 16));
         bad |= (scale_bad(d0) || scale_bad(n0) ? 1 : 0) | (scale_bad(d1) || scale_bad(n1) ? 2 : 0);
-        const float m0 = b.low ? -n0 : 0.0f, m1 = b.low ? -n1 : 0.0f;           // the minimum term counts once, with the lower digits
 #pragma unroll
-        for (int p = 0; p < kIn / 2; ++p) { acc[p][0] += fmaf(d0, blk[p][0], m0 * mn[p][0]); acc[p][1] += fmaf(d1, blk[p][1], m1 * mn[p][1]); }
+        for (int p = 0; p < kIn / 2; ++p) {
+            acc[p][0] += fmaf(d0, blk[0][p][0], -n0 * mn[0][p][0]) + fmaf(d0, blk[1][p][0], -n0 * mn[1][p][0]);
+            acc[p][1] += fmaf(d1, blk[0][p][1], -n1 * mn[0][p][1]) + fmaf(d1, blk[1][p][1], -n1 * mn[1][p][1]);
+        }
     }
 };
 
@@ -391,7 +395,7 @@ struct StreamQ2k {
         acc[1] += fmaf(d1, blk1, -n1 * min1);
     }
     template <int kIn, int> __device__ __forceinline__ static void dense(uint32_t row0, uint32_t row1, const DenseB &b, const Lane &l, float (&acc)[kIn / 2][2], int &bad) {
-        float blk[kIn / 2][2] = {}, mn[kIn / 2][2] = {};
+        float blk[2][kIn / 2][2] = {}, mn[2][kIn / 2][2] = {};
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const uint32_t at = 16 + 32 * (j >> 2) + 8 * l.t;
@@ -403,20 +407,23 @@ struct StreamQ2k {
             mma_dense<kIn>(a, b, j, c);
 #pragma unroll
             for (int p = 0; p < kIn / 2; ++p) {
-                const float xa = ldsf(b.sums + p * b.sums_pair + 8 * j), xb = ldsf(b.sums + p * b.sums_pair + 8 * j + 4);
-                blk[p][0] += digit_pair(c[p][0], c[p][1]);
-                blk[p][1] += digit_pair(c[p][2], c[p][3]);
-                mn[p][0] = fmaf((float)((s0 >> 4) & 15u), xa, fmaf((float)(s0 >> 12), xb, mn[p][0]));
-                mn[p][1] = fmaf((float)((s1 >> 4) & 15u), xa, fmaf((float)(s1 >> 12), xb, mn[p][1]));
+                const uint2 xs = lds64(b.sums + p * b.sums_pair + 8 * j);
+                const float xa = __uint_as_float(xs.x), xb = __uint_as_float(xs.y);
+                blk[j & 1][p][0] += digit_pair(c[p][0], c[p][1]);
+                blk[j & 1][p][1] += digit_pair(c[p][2], c[p][3]);
+                mn[j & 1][p][0] = fmaf((float)((s0 >> 4) & 15u), xa, fmaf((float)(s0 >> 12), xb, mn[j & 1][p][0]));
+                mn[j & 1][p][1] = fmaf((float)((s1 >> 4) & 15u), xa, fmaf((float)(s1 >> 12), xb, mn[j & 1][p][1]));
             }
         }
         const uint32_t h0 = lds32(row0 + 80), h1 = lds32(row1 + 80);                 // d, dmin
         const float d0 = f16_bits_to_float((uint16_t)h0), n0 = f16_bits_to_float((uint16_t)(h0 >> 16));
         const float d1 = f16_bits_to_float((uint16_t)h1), n1 = f16_bits_to_float((uint16_t)(h1 >> 16));
         bad |= (scale_bad(d0) || scale_bad(n0) ? 1 : 0) | (scale_bad(d1) || scale_bad(n1) ? 2 : 0);
-        const float m0 = b.low ? -n0 : 0.0f, m1 = b.low ? -n1 : 0.0f;           // the minimum term counts once, with the lower digits
 #pragma unroll
-        for (int p = 0; p < kIn / 2; ++p) { acc[p][0] += fmaf(d0, blk[p][0], m0 * mn[p][0]); acc[p][1] += fmaf(d1, blk[p][1], m1 * mn[p][1]); }
+        for (int p = 0; p < kIn / 2; ++p) {
+            acc[p][0] += fmaf(d0, blk[0][p][0], -n0 * mn[0][p][0]) + fmaf(d0, blk[1][p][0], -n0 * mn[1][p][0]);
+            acc[p][1] += fmaf(d1, blk[0][p][1], -n1 * mn[0][p][1]) + fmaf(d1, blk[1][p][1], -n1 * mn[1][p][1]);
+        }
     }
 };
 
@@ -478,6 +485,7 @@ struct StreamQ80 {
         bad |= scale_bad(d) ? flag : 0;
     }
     template <int kIn, int> __device__ __forceinline__ static void dense(uint32_t row0, uint32_t row1, const DenseB &b, const Lane &l, float (&acc)[kIn / 2][2], int &bad) {
+        float odd[kIn / 2][2] = {};                                             // a second chain, for every other block
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             uint32_t a[4];
@@ -488,10 +496,13 @@ struct StreamQ80 {
             mma_dense<kIn>(a, b, j, c);
 #pragma unroll
             for (int p = 0; p < kIn / 2; ++p) {
-                acc[p][0] = fmaf(digit_pair(c[p][0], c[p][1]), d0, acc[p][0]);
-                acc[p][1] = fmaf(digit_pair(c[p][2], c[p][3]), d1, acc[p][1]);
+                float (&to)[2] = j & 1 ? odd[p] : acc[p];
+                to[0] = fmaf(digit_pair(c[p][0], c[p][1]), d0, to[0]);
+                to[1] = fmaf(digit_pair(c[p][2], c[p][3]), d1, to[1]);
             }
         }
+#pragma unroll
+        for (int p = 0; p < kIn / 2; ++p) { acc[p][0] += odd[p][0]; acc[p][1] += odd[p][1]; }
     }
 };
 
@@ -593,7 +604,7 @@ struct StreamMxfp4 {
             mma_dense<kIn>(a, b, j, c);
 #pragma unroll
             for (int p = 0; p < kIn / 2; ++p) {
-                const float off = b.low ? 16.0f * ldsf(b.sums + p * b.sums_pair + 4 * j) : 0.0f;        // 16 x the sum of the activation over this block
+                const float off = 16.0f * ldsf(b.sums + p * b.sums_pair + 4 * j);        // 16 x the sum of this digit pair over this block
                 acc[p][0] = fmaf(digit_pair(c[p][0], c[p][1]) - off, s0, acc[p][0]);
                 acc[p][1] = fmaf(digit_pair(c[p][2], c[p][3]) - off, s1, acc[p][1]);
             }
@@ -643,8 +654,17 @@ struct StreamCtl {
     int abort, layout_bad;
 };
 
-__host__ __device__ inline uint32_t stream_small_bytes(int K, int consumers, int depth, int units_per_slice, int groups, int inputs) {
-    return (uint32_t)(inputs * 4 * (K + (inputs > 1 ? kPlanePad : 0)) + 256 * units_per_slice + 128 + inputs * (K / 16) * 4 + 128 + inputs * (depth + 1) * consumers * groups * kTileRows * 4 + 256);
+constexpr int kSumPad = 4;               // floats between their digit pairs' sums: the four lanes of a quad read four of them at once
+
+// Activation sums: one per group of the row, or per input row and digit pair the sums that the qtype's decoder reads.
+__host__ __device__ inline uint32_t stream_sums_bytes(unsigned q, int K, int inputs) {
+    if (inputs == 1) return (uint32_t)(K / 16) * 4u;
+    const int group = q == Q_Q2_K ? 16 : q == Q_Q4_K || q == Q_MXFP4 ? 32 : 0;
+    return group ? (uint32_t)(inputs * 2 * (K / group + kSumPad)) * 4u : 0u;
+}
+__host__ __device__ inline uint32_t stream_small_bytes(unsigned q, int K, int consumers, int depth, int units_per_slice, int groups, int inputs) {
+    return (uint32_t)(inputs * 4 * (K + (inputs > 1 ? kPlanePad : 0)) + 256 * units_per_slice + 128 + 128 + inputs * (depth + 1) * consumers * groups * kTileRows * 4 + 256) +
+           stream_sums_bytes(q, K, inputs);
 }
 
 // The task list of one CTA, walked without divisions: tile `tile` of matrix `m`.
@@ -690,7 +710,7 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
         for (int i = 0; i < D; ++i) ctl.stage[i] = take(p.stage_bytes + 16);
         ctl.planes = take((uint32_t)(kIn * 4 * plane));
         ctl.zeros = take((uint32_t)(256 * p.units_per_slice + 16));
-        ctl.sums = take((uint32_t)(kIn * (p.K / 16)) * 4u);
+        ctl.sums = take(stream_sums_bytes(Dec::kQtype, p.K, kIn));
         ctl.red = take((uint32_t)(kIn * (D + 1) * consumers * kGroupsPerWarp * kTileRows) * 4u);
         ctl.table = tab;
         ctl.layout_bad = cur > end || (Dec::kTables && tab + kTableBytes > end);
@@ -900,10 +920,12 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
             const float to_q = ldexpf(1.0f, 27 - e);
             if (kIn == 1 ? threadIdx.x == 0 : x0 == 0) ctl.xscale[c.m & 7u][xin] = ldexpf(1.0f, e - 27);
             int8_t *pl = reinterpret_cast<int8_t *>(generic(ctl.planes)) + (size_t)xin * 4 * plane;
-            float *sm = reinterpret_cast<float *>(generic(ctl.sums)) + (size_t)xin * (p.K / 16);
+            const int per_pair = Dec::kSumGroup ? p.K / (Dec::kSumGroup ? Dec::kSumGroup : 1) + kSumPad : 0;      // kIn > 1: [input][upper, lower digit pair][group]
+            float *sm = reinterpret_cast<float *>(generic(ctl.sums)) + (size_t)(kIn > 1 ? xin * 2 * per_pair : 0);
             auto digits = [&](int k8, const float (&xv)[8]) {               // (whole warps: K / 8 is a multiple of 32)
                 uint32_t d[4][2] = {{0u, 0u}, {0u, 0u}, {0u, 0u}, {0u, 0u}};
                 float s = 0.0f;
+                int upper = 0, lower = 0;                                   // digit pairs are below 2^14: their sums are exact
 #pragma unroll
                 for (int i8 = 0; i8 < 8; ++i8) {
                     int q = isfinite(xv[i8]) ? __float2int_rn(xv[i8] * to_q) : 0;
@@ -913,6 +935,8 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
                     const int d1 = ((q + 64) & 127) - 64; q = (q - d1) >> 7;
                     const int d2 = ((q + 64) & 127) - 64; q = (q - d2) >> 7;
                     const int dig[4] = {q, d2, d1, d0};                     // plane 0 is the most significant
+                    upper += q * 128 + d2;
+                    lower += d1 * 128 + d0;
 #pragma unroll
                     for (int pi = 0; pi < 4; ++pi) d[pi][i8 >> 2] |= (uint32_t)(dig[pi] & 0xff) << (8 * (i8 & 3));
                 }
@@ -933,7 +957,17 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
                     for (int pi = 0; pi < 4; ++pi)
                         *reinterpret_cast<uint2 *>(pl + (size_t)pi * plane + 8 * k8) = make_uint2(d[pi][0], d[pi][1]);
                 }
-                if (Dec::kSumGroup == 32) {
+                if constexpr (kIn > 1 && Dec::kSumGroup) {
+#pragma unroll
+                    for (int o = 1; o < Dec::kSumGroup / 8; o *= 2) {
+                        upper += __shfl_xor_sync(0xffffffffu, upper, o);
+                        lower += __shfl_xor_sync(0xffffffffu, lower, o);
+                    }
+                    if (k8 % (Dec::kSumGroup / 8) == 0) {
+                        sm[k8 / (Dec::kSumGroup / 8)] = (float)upper;
+                        sm[per_pair + k8 / (Dec::kSumGroup / 8)] = (float)lower;
+                    }
+                } else if (Dec::kSumGroup == 32) {
                     s += __shfl_xor_sync(0xffffffffu, s, 1);
                     s += __shfl_xor_sync(0xffffffffu, s, 2);
                     if ((threadIdx.x & 3) == 0) sm[k8 >> 2] = s;
@@ -982,10 +1016,11 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
                         if constexpr (kIn == 1) {
                             Dec::template unit<decltype(odd)::value>(r0, r0 + second, b, l, sums + (uint32_t)(u * kSumsPerUnit * 4), acc[gi][0], bad[gi]);
                         } else {
-                            // column n = lane >> 2 of pair 0: digit plane n & 3 of input n >> 2; sums of the input this lane's results belong to
-                            const uint32_t n = (uint32_t)lane >> 2, k0 = (uint32_t)((unit0 + u) * Dec::kBlockK), per_input = (uint32_t)(p.K / 16) * 4u;
+                            // column n = lane >> 2 of pair 0: digit plane n & 3 of input n >> 2; lane t holds results of digit pair t & 1 of input t >> 1
+                            const uint32_t n = (uint32_t)lane >> 2, k0 = (uint32_t)((unit0 + u) * Dec::kBlockK);
+                            const uint32_t per_pair = Dec::kSumGroup ? (uint32_t)(p.K / (Dec::kSumGroup ? Dec::kSumGroup : 1) + kSumPad) * 4u : 0u;
                             const DenseB db{ctl.planes + n * (uint32_t)plane + k0 + 8u * (uint32_t)l.t, 8u * (uint32_t)plane,
-                                            sums + (uint32_t)(u * kSumsPerUnit * 4) + (uint32_t)(l.t >> 1) * per_input, 2u * per_input, (l.t & 1) != 0};
+                                            sums + (uint32_t)(u * kSumsPerUnit * 4) + (uint32_t)l.t * per_pair, 4u * per_pair};
                             Dec::template dense<kIn, 0>(r0, r0 + second, db, l, acc[gi], bad[gi]);
                         }
                     }
@@ -1057,7 +1092,7 @@ inline bool stream_shape(unsigned q, uint64_t width, uint64_t row_bytes, StreamS
             // every piece is rounded up to 128 bytes; with tables one piece may have to step over the table window,
             // which starts at most 64 KiB - 1 into the allocation (what lies before it stays usable)
             const uint32_t pieces = (uint32_t)sh.depth * (sh.stage_bytes + 16 + 128) +
-                                    stream_small_bytes((int)width, sh.consumers, sh.depth, sh.units_per_slice, sh.groups, inputs) + 5 * 128;
+                                    stream_small_bytes(q, (int)width, sh.consumers, sh.depth, sh.units_per_slice, sh.groups, inputs) + 5 * 128;
             uint32_t largest = sh.stage_bytes + 16;         // the piece that steps over leaves a gap of up to its own size
             for (uint32_t piece : {(uint32_t)(inputs * 4) * (uint32_t)(width + kPlanePad), (uint32_t)(inputs * (sh.depth + 1) * sh.consumers * sh.groups * kTileRows) * 4u})
                 largest = largest < piece ? piece : largest;
@@ -1073,7 +1108,7 @@ inline bool stream_shape(unsigned q, uint64_t width, uint64_t row_bytes, StreamS
                     for (int i = 0; i < sh.depth; ++i) take(sh.stage_bytes + 16);
                     take((uint32_t)(inputs * 4) * (uint32_t)(width + kPlanePad));
                     take((uint32_t)(256 * sh.units_per_slice + 16));
-                    take((uint32_t)(inputs * (int)(width / 16)) * 4u);
+                    take(stream_sums_bytes(q, (int)width, inputs));
                     take((uint32_t)(inputs * (sh.depth + 1) * sh.consumers * sh.groups * kTileRows) * 4u);
                     const uint32_t end = cur > tab + kTableBytes ? cur : tab + kTableBytes;
                     sh.smem_bytes = sh.smem_bytes > end - base ? sh.smem_bytes : end - base;
