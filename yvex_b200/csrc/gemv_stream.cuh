@@ -675,6 +675,138 @@ struct TaskCursor {
     __device__ __forceinline__ void next() { if (++tile == tiles_m) { tile = 0; ++m; } }
 };
 
+// The activation row of matrix m (kIn > 1: the rows of pass m) as four planes of signed base-128 digits, its scale and its sums;
+// every consumer warp calls it.
+template <class Dec, bool kBReg, int kIn>
+__device__ __forceinline__ void prepare_planes(StreamCtl &ctl, int K, int consumers, uint32_t m, uint32_t cur_x, uint32_t inputs, const float *x_base,
+                                               uint64_t x_stride, const float *x_up, const float *x_weight, float x_limit, int *status) {
+    // 8-value chunks of the input row per consumer thread: K / 8 over 32 x slices x row warps threads, at most the units per slice
+    constexpr int kXChunks = kIn > 1 ? 4 : kBReg ? 1 : 2;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, cthreads = 32 * consumers, plane = K + (kIn > 1 ? kPlanePad : 0);
+    auto generic = [](uint32_t a) { return __cvta_shared_to_generic(a); };
+    // every consumer has finished the previous matrix once it is past this barrier
+    asm volatile("bar.sync 1, %0;" ::"r"(cthreads) : "memory");
+    // kIn > 1: the warps are dealt to the pass's input rows (a remainder stays idle), rows past the last repeat it
+    const int xin = kIn == 1 ? 0 : warp % kIn, xthreads = kIn == 1 ? cthreads : 32 * (consumers / kIn);
+    const int x0 = kIn == 1 ? (int)threadIdx.x : warp / kIn < consumers / kIn ? 32 * (warp / kIn) + lane : K;
+    const uint32_t xrow = kIn == 1 ? cur_x : min(cur_x * kIn + (uint32_t)xin, inputs - 1u);
+    const float *x = x_base + (uint64_t)xrow * x_stride;
+    // One input row is read (and SwiGLU evaluated) once: a thread keeps its eight values, or sixteen at widths where a
+    // warp owns two units of one row group, from the search for the largest magnitude to the digits.
+    float mx = 0.0f;
+    bool badx = false;
+    const float *xu = kIn == 1 && x_up ? x_up + (uint64_t)cur_x * x_stride : nullptr;
+    const float xw = kIn == 1 && x_up ? __ldg(x_weight + m) : 1.0f;
+    float xs[kXChunks][8];
+    auto load8 = [&](int k8, float (&v)[8]) {
+        const float4 xa = __ldg(reinterpret_cast<const float4 *>(x + 8 * k8)), xb = __ldg(reinterpret_cast<const float4 *>(x + 8 * k8) + 1);
+        v[0] = xa.x; v[1] = xa.y; v[2] = xa.z; v[3] = xa.w; v[4] = xb.x; v[5] = xb.y; v[6] = xb.z; v[7] = xb.w;
+        if (xu) {
+            const float4 ua = __ldg(reinterpret_cast<const float4 *>(xu + 8 * k8)), ub = __ldg(reinterpret_cast<const float4 *>(xu + 8 * k8) + 1);
+            const float uv[8] = {ua.x, ua.y, ua.z, ua.w, ub.x, ub.y, ub.z, ub.w};
+#pragma unroll
+            for (int i8 = 0; i8 < 8; ++i8) v[i8] = swiglu_mid(v[i8], uv[i8], xw, x_limit, status);
+        }
+    };
+    auto magnitude = [&](const float (&v)[8]) {
+#pragma unroll
+        for (int i8 = 0; i8 < 8; ++i8) { badx |= !isfinite(v[i8]); mx = fmaxf(mx, fabsf(v[i8])); }
+    };
+#pragma unroll
+    for (int q = 0; q < kXChunks; ++q)
+        if (x0 + q * xthreads < K / 8) load8(x0 + q * xthreads, xs[q]);
+#pragma unroll
+    for (int q = 0; q < kXChunks; ++q)
+        if (x0 + q * xthreads < K / 8) magnitude(xs[q]);
+    if constexpr (kIn > 1) {                                        // (a quarter of the threads per row: the rest is read twice)
+        for (int k8 = x0 + kXChunks * xthreads; k8 < K / 8; k8 += xthreads) { float v[8]; load8(k8, v); magnitude(v); }
+    }
+    // (magnitudes order like their bit patterns; fmaxf has dropped any NaN)
+    mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));
+    if (lane == 0) ctl.warp_max[warp] = mx;
+    if (badx) raise(status, YVEX_B200_STATUS_NUMERIC);
+    asm volatile("bar.sync 1, %0;" ::"r"(cthreads) : "memory");
+    mx = __uint_as_float(__reduce_max_sync(0xffffffffu, lane < consumers && (kIn == 1 || (lane % kIn == xin && lane / kIn < consumers / kIn)) ? __float_as_uint(ctl.warp_max[lane]) : 0u));
+    // S = the power of two above the largest magnitude; q = rint(x / S * 2^27), |q| <= 2^27
+    int e = 0;
+    if (mx > 0.0f && isfinite(mx)) frexpf(mx, &e);
+    const float to_q = ldexpf(1.0f, 27 - e);
+    if (kIn == 1 ? threadIdx.x == 0 : x0 == 0) ctl.xscale[m & 7u][xin] = ldexpf(1.0f, e - 27);
+    int8_t *pl = reinterpret_cast<int8_t *>(generic(ctl.planes)) + (size_t)xin * 4 * plane;
+    const int per_pair = Dec::kSumGroup ? K / (Dec::kSumGroup ? Dec::kSumGroup : 1) + kSumPad : 0;      // kIn > 1: [input][upper, lower digit pair][group]
+    float *sm = reinterpret_cast<float *>(generic(ctl.sums)) + (size_t)(kIn > 1 ? xin * 2 * per_pair : 0);
+    auto digits = [&](int k8, const float (&xv)[8]) {               // (whole warps: K / 8 is a multiple of 32)
+        uint32_t d[4][2] = {{0u, 0u}, {0u, 0u}, {0u, 0u}, {0u, 0u}};
+        float s = 0.0f;
+        int upper = 0, lower = 0;                                   // digit pairs are below 2^14: their sums are exact
+#pragma unroll
+        for (int i8 = 0; i8 < 8; ++i8) {
+            int q = isfinite(xv[i8]) ? __float2int_rn(xv[i8] * to_q) : 0;
+            s += (float)q;
+            // balanced digits: d0..d2 in [-64, 63], the top digit takes what is left (|d3| <= 64)
+            const int d0 = ((q + 64) & 127) - 64; q = (q - d0) >> 7;
+            const int d1 = ((q + 64) & 127) - 64; q = (q - d1) >> 7;
+            const int d2 = ((q + 64) & 127) - 64; q = (q - d2) >> 7;
+            const int dig[4] = {q, d2, d1, d0};                     // plane 0 is the most significant
+            upper += q * 128 + d2;
+            lower += d1 * 128 + d0;
+#pragma unroll
+            for (int pi = 0; pi < 4; ++pi) d[pi][i8 >> 2] |= (uint32_t)(dig[pi] & 0xff) << (8 * (i8 & 3));
+        }
+        if (Dec::kInterleave) {
+            // lanes s and s + 2 of a quad hold weights 8 s .. and 16 + 8 s ..: lane s builds the 8-byte chunk 2 s
+            // (its own first word and the partner's, bytes alternating), lane s + 2 chunk 2 s + 1 (the second words)
+            const int sub = k8 & 3;
+#pragma unroll
+            for (int pi = 0; pi < 4; ++pi) {
+                const uint32_t got = __shfl_xor_sync(0xffffffffu, sub < 2 ? d[pi][1] : d[pi][0], 2);
+                const uint32_t lo = sub < 2 ? d[pi][0] : got, hi = sub < 2 ? got : d[pi][1];
+                const int chunk = sub < 2 ? 2 * sub : 2 * (sub - 2) + 1;
+                *reinterpret_cast<uint2 *>(pl + (size_t)pi * plane + 32 * (k8 >> 2) + 8 * chunk) =
+                    make_uint2(prmt(lo, hi, 0x5140u), prmt(lo, hi, 0x7362u));
+            }
+        } else {
+#pragma unroll
+            for (int pi = 0; pi < 4; ++pi)
+                *reinterpret_cast<uint2 *>(pl + (size_t)pi * plane + 8 * k8) = make_uint2(d[pi][0], d[pi][1]);
+        }
+        if constexpr (kIn > 1 && Dec::kSumGroup) {
+#pragma unroll
+            for (int o = 1; o < Dec::kSumGroup / 8; o *= 2) {
+                upper += __shfl_xor_sync(0xffffffffu, upper, o);
+                lower += __shfl_xor_sync(0xffffffffu, lower, o);
+            }
+            if (k8 % (Dec::kSumGroup / 8) == 0) {
+                sm[k8 / (Dec::kSumGroup / 8)] = (float)upper;
+                sm[per_pair + k8 / (Dec::kSumGroup / 8)] = (float)lower;
+            }
+        } else if (Dec::kSumGroup == 32) {
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            s += __shfl_xor_sync(0xffffffffu, s, 2);
+            if ((threadIdx.x & 3) == 0) sm[k8 >> 2] = s;
+        } else if (Dec::kSumGroup == 16) {
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            if ((threadIdx.x & 1) == 0) sm[k8 >> 1] = s;
+        }
+    };
+#pragma unroll
+    for (int q = 0; q < kXChunks; ++q)
+        if (x0 + q * xthreads < K / 8) digits(x0 + q * xthreads, xs[q]);
+    if constexpr (kIn > 1) {
+        for (int k8 = x0 + kXChunks * xthreads; k8 < K / 8; k8 += xthreads) { float v[8]; load8(k8, v); digits(k8, v); }
+    }
+    asm volatile("bar.sync 1, %0;" ::"r"(cthreads) : "memory");
+}
+// The same as a real call. Inlined, its registers cost the tile loop spills (MXFP4 4096 wide, one row: 56 bytes loaded a tile) and the
+// loop's schedule; as a call, and with a matrix's tiles in a loop of their own, 200 matrices of 4096 x 1536 / 1536 x 4096 take
+// MXFP4 208 / 202 us against 251 / 230, Q4_K 147 / 177 against 160 / 179, IQ2_XXS 185 / 171 against 195 / 179. Only the several-row
+// form of Q4_K and Q2_K, which keeps eight sums more, is 2 to 3 % faster with it inlined.
+template <class Dec, bool kBReg, int kIn>
+__device__ __noinline__ void prepare_planes_call(StreamCtl &ctl, int K, int consumers, uint32_t m, uint32_t cur_x, uint32_t inputs, const float *x_base,
+                                                 uint64_t x_stride, const float *x_up, const float *x_weight, float x_limit, int *status) {
+    prepare_planes<Dec, kBReg, kIn>(ctl, K, consumers, m, cur_x, inputs, x_base, x_stride, x_up, x_weight, x_limit, status);
+}
+
 // kBReg: the warp's whole K-slice is one unit, so its B fragments live in registers from one matrix change to the next.
 // kGroupsPerWarp: 16-row groups a consumer warp decodes per stage.
 // kRows: matrix rows in one MMA group: 16, or 8 where sixteen rows are too long for a ring (row g + 8 of a fragment then repeats row g).
@@ -845,9 +977,6 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
         }
     };
 
-    // 8-value chunks of the input row per consumer thread: K / 8 over 32 x slices x row warps threads, at most the units per slice
-    constexpr int kXChunks = kIn > 1 ? 4 : kBReg ? 1 : 2;
-
     // A warp whose wait ran out keeps walking the task list without touching data, so that it still
     // meets the other consumers at the named barriers of every matrix change and nobody waits for it.
     bool dead = false;
@@ -860,202 +989,95 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
     TaskCursor c;
     c.init(q0, tiles_m);
     uint32_t c_slot = 0, c_buf = 0, c_phase = 0;
-    for (uint32_t i = 0; i < n_local; ++i, c.next()) {
-        uint64_t row0;
-        const uint32_t nrows = rows_of(c, row0);
-        if (c.m != cur_m && cur_m != 0xffffffffu && p.x_rows && __ldg(p.x_rows + c.m) == cur_x) {
+    for (uint32_t i = 0; i < n_local;) {
+        if (cur_m != 0xffffffffu && p.x_rows && __ldg(p.x_rows + c.m) == cur_x) {
             // the next matrix reads the same input row: the planes, sums and B registers stand as they are
             if (threadIdx.x == 0) ctl.xscale[c.m & 7u][0] = ctl.xscale[cur_m & 7u][0];
-            cur_m = c.m;
-        }
-        if (c.m != cur_m) {
-            // a new matrix: its activation row becomes four planes of signed base-128 digits. Every
-            // consumer has finished the previous matrix once it is past this barrier.
-            asm volatile("bar.sync 1, %0;" ::"r"(cthreads) : "memory");
+        } else {
             cur_x = p.x_rows ? __ldg(p.x_rows + c.m) : c.m;
-            // kIn > 1: the warps are dealt to the pass's input rows (a remainder stays idle), rows past the last repeat it
-            const int xin = kIn == 1 ? 0 : warp % kIn, xthreads = kIn == 1 ? cthreads : 32 * (consumers / kIn);
-            const int x0 = kIn == 1 ? (int)threadIdx.x : warp / kIn < consumers / kIn ? 32 * (warp / kIn) + lane : p.K;
-            const uint32_t xrow = kIn == 1 ? cur_x : min(cur_x * kIn + (uint32_t)xin, p.inputs - 1u);
-            const float *x = p.x + (uint64_t)xrow * p.x_stride;
-            // One input row is read (and SwiGLU evaluated) once: a thread keeps its eight values, or sixteen at widths where a
-            // warp owns two units of one row group, from the search for the largest magnitude to the digits.
-            float mx = 0.0f;
-            bool badx = false;
-            const float *xu = kIn == 1 && p.x_up ? p.x_up + (uint64_t)cur_x * p.x_stride : nullptr;
-            const float xw = kIn == 1 && p.x_up ? __ldg(p.x_weight + c.m) : 1.0f;
-            float xs[kXChunks][8];
-            auto load8 = [&](int k8, float (&v)[8]) {
-                const float4 xa = __ldg(reinterpret_cast<const float4 *>(x + 8 * k8)), xb = __ldg(reinterpret_cast<const float4 *>(x + 8 * k8) + 1);
-                v[0] = xa.x; v[1] = xa.y; v[2] = xa.z; v[3] = xa.w; v[4] = xb.x; v[5] = xb.y; v[6] = xb.z; v[7] = xb.w;
-                if (xu) {
-                    const float4 ua = __ldg(reinterpret_cast<const float4 *>(xu + 8 * k8)), ub = __ldg(reinterpret_cast<const float4 *>(xu + 8 * k8) + 1);
-                    const float uv[8] = {ua.x, ua.y, ua.z, ua.w, ub.x, ub.y, ub.z, ub.w};
-#pragma unroll
-                    for (int i8 = 0; i8 < 8; ++i8) v[i8] = swiglu_mid(v[i8], uv[i8], xw, p.x_limit, p.status);
-                }
-            };
-            auto magnitude = [&](const float (&v)[8]) {
-#pragma unroll
-                for (int i8 = 0; i8 < 8; ++i8) { badx |= !isfinite(v[i8]); mx = fmaxf(mx, fabsf(v[i8])); }
-            };
-#pragma unroll
-            for (int q = 0; q < kXChunks; ++q)
-                if (x0 + q * xthreads < p.K / 8) load8(x0 + q * xthreads, xs[q]);
-#pragma unroll
-            for (int q = 0; q < kXChunks; ++q)
-                if (x0 + q * xthreads < p.K / 8) magnitude(xs[q]);
-            if constexpr (kIn > 1) {                                        // (a quarter of the threads per row: the rest is read twice)
-                for (int k8 = x0 + kXChunks * xthreads; k8 < p.K / 8; k8 += xthreads) { float v[8]; load8(k8, v); magnitude(v); }
-            }
-            // (magnitudes order like their bit patterns; fmaxf has dropped any NaN)
-            mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));
-            if (lane == 0) ctl.warp_max[warp] = mx;
-            if (badx) raise(p.status, YVEX_B200_STATUS_NUMERIC);
-            asm volatile("bar.sync 1, %0;" ::"r"(cthreads) : "memory");
-            mx = __uint_as_float(__reduce_max_sync(0xffffffffu, lane < consumers && (kIn == 1 || (lane % kIn == xin && lane / kIn < consumers / kIn)) ? __float_as_uint(ctl.warp_max[lane]) : 0u));
-            // S = the power of two above the largest magnitude; q = rint(x / S * 2^27), |q| <= 2^27
-            int e = 0;
-            if (mx > 0.0f && isfinite(mx)) frexpf(mx, &e);
-            const float to_q = ldexpf(1.0f, 27 - e);
-            if (kIn == 1 ? threadIdx.x == 0 : x0 == 0) ctl.xscale[c.m & 7u][xin] = ldexpf(1.0f, e - 27);
-            int8_t *pl = reinterpret_cast<int8_t *>(generic(ctl.planes)) + (size_t)xin * 4 * plane;
-            const int per_pair = Dec::kSumGroup ? p.K / (Dec::kSumGroup ? Dec::kSumGroup : 1) + kSumPad : 0;      // kIn > 1: [input][upper, lower digit pair][group]
-            float *sm = reinterpret_cast<float *>(generic(ctl.sums)) + (size_t)(kIn > 1 ? xin * 2 * per_pair : 0);
-            auto digits = [&](int k8, const float (&xv)[8]) {               // (whole warps: K / 8 is a multiple of 32)
-                uint32_t d[4][2] = {{0u, 0u}, {0u, 0u}, {0u, 0u}, {0u, 0u}};
-                float s = 0.0f;
-                int upper = 0, lower = 0;                                   // digit pairs are below 2^14: their sums are exact
-#pragma unroll
-                for (int i8 = 0; i8 < 8; ++i8) {
-                    int q = isfinite(xv[i8]) ? __float2int_rn(xv[i8] * to_q) : 0;
-                    s += (float)q;
-                    // balanced digits: d0..d2 in [-64, 63], the top digit takes what is left (|d3| <= 64)
-                    const int d0 = ((q + 64) & 127) - 64; q = (q - d0) >> 7;
-                    const int d1 = ((q + 64) & 127) - 64; q = (q - d1) >> 7;
-                    const int d2 = ((q + 64) & 127) - 64; q = (q - d2) >> 7;
-                    const int dig[4] = {q, d2, d1, d0};                     // plane 0 is the most significant
-                    upper += q * 128 + d2;
-                    lower += d1 * 128 + d0;
-#pragma unroll
-                    for (int pi = 0; pi < 4; ++pi) d[pi][i8 >> 2] |= (uint32_t)(dig[pi] & 0xff) << (8 * (i8 & 3));
-                }
-                if (Dec::kInterleave) {
-                    // lanes s and s + 2 of a quad hold weights 8 s .. and 16 + 8 s ..: lane s builds the 8-byte chunk 2 s
-                    // (its own first word and the partner's, bytes alternating), lane s + 2 chunk 2 s + 1 (the second words)
-                    const int sub = k8 & 3;
-#pragma unroll
-                    for (int pi = 0; pi < 4; ++pi) {
-                        const uint32_t got = __shfl_xor_sync(0xffffffffu, sub < 2 ? d[pi][1] : d[pi][0], 2);
-                        const uint32_t lo = sub < 2 ? d[pi][0] : got, hi = sub < 2 ? got : d[pi][1];
-                        const int chunk = sub < 2 ? 2 * sub : 2 * (sub - 2) + 1;
-                        *reinterpret_cast<uint2 *>(pl + (size_t)pi * plane + 32 * (k8 >> 2) + 8 * chunk) =
-                            make_uint2(prmt(lo, hi, 0x5140u), prmt(lo, hi, 0x7362u));
-                    }
-                } else {
-#pragma unroll
-                    for (int pi = 0; pi < 4; ++pi)
-                        *reinterpret_cast<uint2 *>(pl + (size_t)pi * plane + 8 * k8) = make_uint2(d[pi][0], d[pi][1]);
-                }
-                if constexpr (kIn > 1 && Dec::kSumGroup) {
-#pragma unroll
-                    for (int o = 1; o < Dec::kSumGroup / 8; o *= 2) {
-                        upper += __shfl_xor_sync(0xffffffffu, upper, o);
-                        lower += __shfl_xor_sync(0xffffffffu, lower, o);
-                    }
-                    if (k8 % (Dec::kSumGroup / 8) == 0) {
-                        sm[k8 / (Dec::kSumGroup / 8)] = (float)upper;
-                        sm[per_pair + k8 / (Dec::kSumGroup / 8)] = (float)lower;
-                    }
-                } else if (Dec::kSumGroup == 32) {
-                    s += __shfl_xor_sync(0xffffffffu, s, 1);
-                    s += __shfl_xor_sync(0xffffffffu, s, 2);
-                    if ((threadIdx.x & 3) == 0) sm[k8 >> 2] = s;
-                } else if (Dec::kSumGroup == 16) {
-                    s += __shfl_xor_sync(0xffffffffu, s, 1);
-                    if ((threadIdx.x & 1) == 0) sm[k8 >> 1] = s;
-                }
-            };
-#pragma unroll
-            for (int q = 0; q < kXChunks; ++q)
-                if (x0 + q * xthreads < p.K / 8) digits(x0 + q * xthreads, xs[q]);
-            if constexpr (kIn > 1) {
-                for (int k8 = x0 + kXChunks * xthreads; k8 < p.K / 8; k8 += xthreads) { float v[8]; load8(k8, v); digits(k8, v); }
-            }
-            asm volatile("bar.sync 1, %0;" ::"r"(cthreads) : "memory");
+            constexpr bool kInline = kIn > 1 && (Dec::kQtype == Q_Q4_K || Dec::kQtype == Q_Q2_K);
+            constexpr auto prepare = kInline ? prepare_planes<Dec, kBReg, kIn> : prepare_planes_call<Dec, kBReg, kIn>;
+            prepare(ctl, p.K, consumers, c.m, cur_x, p.inputs, p.x, p.x_stride, p.x_up, p.x_weight, p.x_limit, p.status);
             asm volatile("" : "+r"(b_hi), "+r"(b_lo), "+r"(sums));      // reads of the new planes stay behind the barrier
             if (kBReg) load_b(breg, 0);
-            cur_m = c.m;
         }
-        // stage i % D with phase (i / D) & 1 and result buffer i % (D + 1), kept as counters (no divisions in this loop)
-        const uint32_t slot = c_slot, buf = c_buf;
-        if (!dead && !mbar_wait_warp<kTryWaitHintNs>(&ctl.full[slot], c_phase, &ctl.abort)) dead = true;
-        if (++c_slot == (uint32_t)D) { c_slot = 0; c_phase ^= 1u; }
-        if (++c_buf == (uint32_t)(D + 1)) c_buf = 0;
-        float acc[kGroupsPerWarp][kIn > 1 ? kIn / 2 : 1][2];               // [group][input pair][row]
-        int bad[kGroupsPerWarp];
+        cur_m = c.m;
+        // the tiles of the matrix, in a loop of their own (prepare_planes_call says why)
+        do {
+            uint64_t row0;
+            const uint32_t nrows = rows_of(c, row0);
+            // stage i % D with phase (i / D) & 1 and result buffer i % (D + 1), kept as counters (no divisions in this loop)
+            const uint32_t slot = c_slot, buf = c_buf;
+            if (!dead && !mbar_wait_warp<kTryWaitHintNs>(&ctl.full[slot], c_phase, &ctl.abort)) dead = true;
+            if (++c_slot == (uint32_t)D) { c_slot = 0; c_phase ^= 1u; }
+            if (++c_buf == (uint32_t)(D + 1)) c_buf = 0;
+            float acc[kGroupsPerWarp][kIn > 1 ? kIn / 2 : 1][2];               // [group][input pair][row]
+            int bad[kGroupsPerWarp];
 #pragma unroll
-        for (int gi = 0; gi < kGroupsPerWarp; ++gi) {
-            bad[gi] = 0;
+            for (int gi = 0; gi < kGroupsPerWarp; ++gi) {
+                bad[gi] = 0;
 #pragma unroll
-            for (int pr = 0; pr < (kIn > 1 ? kIn / 2 : 1); ++pr) acc[gi][pr][0] = acc[gi][pr][1] = 0.0f;
-        }
-        const uint32_t first = warp_rows * (uint32_t)rw;                     // this warp's first row within the tile
-        if (!dead && first < nrows) {
-            uint32_t base = ctl.stage[slot] + (first + (uint32_t)l.g) * row_bytes + (uint32_t)(unit0 * Dec::kBlockBytes);
-            asm volatile("" : "+r"(base));                              // reads of the stage stay behind the wait above
-            for (int u = 0; u < my_units; ++u) {
-                BUnit bmem;
-                if (!kBReg && kIn == 1) load_b(bmem, u);
-                const BUnit &b = kBReg ? breg : bmem;
-                auto groups = [&](auto odd) {
-#pragma unroll
-                    for (int gi = 0; gi < kGroupsPerWarp; ++gi) {
-                        // groups past a ragged tile's last row decode stale bytes; their results are never stored
-                        const uint32_t r0 = base + (uint32_t)(kRows * gi) * row_bytes + (uint32_t)(u * Dec::kBlockBytes);
-                        if constexpr (kIn == 1) {
-                            Dec::template unit<decltype(odd)::value>(r0, r0 + second, b, l, sums + (uint32_t)(u * kSumsPerUnit * 4), acc[gi][0], bad[gi]);
-                        } else {
-                            // column n = lane >> 2 of pair 0: digit plane n & 3 of input n >> 2; lane t holds results of digit pair t & 1 of input t >> 1
-                            const uint32_t n = (uint32_t)lane >> 2, k0 = (uint32_t)((unit0 + u) * Dec::kBlockK);
-                            const uint32_t per_pair = Dec::kSumGroup ? (uint32_t)(p.K / (Dec::kSumGroup ? Dec::kSumGroup : 1) + kSumPad) * 4u : 0u;
-                            const DenseB db{ctl.planes + n * (uint32_t)plane + k0 + 8u * (uint32_t)l.t, 8u * (uint32_t)plane,
-                                            sums + (uint32_t)(u * kSumsPerUnit * 4) + (uint32_t)l.t * per_pair, 4u * per_pair};
-                            Dec::template dense<kIn, 0>(r0, r0 + second, db, l, acc[gi], bad[gi]);
-                        }
-                    }
-                };
-                if (Dec::kParity && ((unit0 + u) & 1)) groups(std::integral_constant<int, 1>{});
-                else groups(std::integral_constant<int, 0>{});
+                for (int pr = 0; pr < (kIn > 1 ? kIn / 2 : 1); ++pr) acc[gi][pr][0] = acc[gi][pr][1] = 0.0f;
             }
-        }
-        // this warp is done with the stage
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&ctl.empty[slot]);
-        float *red = red_all + ((size_t)buf * kIn * consumers + warp) * warp_rows;           // [input][warp][rows]
+            const uint32_t first = warp_rows * (uint32_t)rw;                     // this warp's first row within the tile
+            if (!dead && first < nrows) {
+                uint32_t base = ctl.stage[slot] + (first + (uint32_t)l.g) * row_bytes + (uint32_t)(unit0 * Dec::kBlockBytes);
+                asm volatile("" : "+r"(base));                              // reads of the stage stay behind the wait above
+                for (int u = 0; u < my_units; ++u) {
+                    BUnit bmem;
+                    if (!kBReg && kIn == 1) load_b(bmem, u);
+                    const BUnit &b = kBReg ? breg : bmem;
+                    auto groups = [&](auto odd) {
 #pragma unroll
-        for (int gi = 0; gi < kGroupsPerWarp; ++gi) {
-            if constexpr (kIn == 1) {
-                float a0 = acc[gi][0][0], a1 = acc[gi][0][1];
-                a0 += __shfl_xor_sync(0xffffffffu, a0, 1); a0 += __shfl_xor_sync(0xffffffffu, a0, 2);
-                a1 += __shfl_xor_sync(0xffffffffu, a1, 1); a1 += __shfl_xor_sync(0xffffffffu, a1, 2);
-                float *to = red + (uint32_t)(kRows * gi) + (uint32_t)l.g;
-                if (l.t == 0) { to[0] = a0; if (whole) to[8] = a1; }
-            } else {
-#pragma unroll
-                for (int pr = 0; pr < kIn / 2; ++pr) {
-                    const float a0 = fmaf(acc[gi][pr][0], 16384.0f, __shfl_xor_sync(0xffffffffu, acc[gi][pr][0], 1));
-                    const float a1 = fmaf(acc[gi][pr][1], 16384.0f, __shfl_xor_sync(0xffffffffu, acc[gi][pr][1], 1));
-                    float *to = red + (size_t)(2 * pr + (l.t >> 1)) * consumers * warp_rows + (uint32_t)(kRows * gi) + (uint32_t)l.g;
-                    if ((l.t & 1) == 0) { to[0] = a0; if (whole) to[8] = a1; }
+                        for (int gi = 0; gi < kGroupsPerWarp; ++gi) {
+                            // groups past a ragged tile's last row decode stale bytes; their results are never stored
+                            const uint32_t r0 = base + (uint32_t)(kRows * gi) * row_bytes + (uint32_t)(u * Dec::kBlockBytes);
+                            if constexpr (kIn == 1) {
+                                Dec::template unit<decltype(odd)::value>(r0, r0 + second, b, l, sums + (uint32_t)(u * kSumsPerUnit * 4), acc[gi][0], bad[gi]);
+                            } else {
+                                // column n = lane >> 2 of pair 0: digit plane n & 3 of input n >> 2; lane t holds results of digit pair t & 1 of input t >> 1
+                                const uint32_t n = (uint32_t)lane >> 2, k0 = (uint32_t)((unit0 + u) * Dec::kBlockK);
+                                const uint32_t per_pair = Dec::kSumGroup ? (uint32_t)(p.K / (Dec::kSumGroup ? Dec::kSumGroup : 1) + kSumPad) * 4u : 0u;
+                                const DenseB db{ctl.planes + n * (uint32_t)plane + k0 + 8u * (uint32_t)l.t, 8u * (uint32_t)plane,
+                                                sums + (uint32_t)(u * kSumsPerUnit * 4) + (uint32_t)l.t * per_pair, 4u * per_pair};
+                                Dec::template dense<kIn, 0>(r0, r0 + second, db, l, acc[gi], bad[gi]);
+                            }
+                        }
+                    };
+                    if (Dec::kParity && ((unit0 + u) & 1)) groups(std::integral_constant<int, 1>{});
+                    else groups(std::integral_constant<int, 0>{});
                 }
             }
-            // a malformed block scale only counts for rows that exist
-            const uint32_t r_lo = first + (uint32_t)(kRows * gi) + (uint32_t)l.g, r_hi = r_lo + (whole ? 8u : 0u);
-            if (((bad[gi] & 1) && r_lo < nrows) || ((bad[gi] & 2) && r_hi < nrows)) raise(p.status, YVEX_B200_STATUS_NUMERIC);
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&ctl.red_full[buf]);
+            // this warp is done with the stage
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ctl.empty[slot]);
+            float *red = red_all + ((size_t)buf * kIn * consumers + warp) * warp_rows;           // [input][warp][rows]
+#pragma unroll
+            for (int gi = 0; gi < kGroupsPerWarp; ++gi) {
+                if constexpr (kIn == 1) {
+                    float a0 = acc[gi][0][0], a1 = acc[gi][0][1];
+                    a0 += __shfl_xor_sync(0xffffffffu, a0, 1); a0 += __shfl_xor_sync(0xffffffffu, a0, 2);
+                    a1 += __shfl_xor_sync(0xffffffffu, a1, 1); a1 += __shfl_xor_sync(0xffffffffu, a1, 2);
+                    float *to = red + (uint32_t)(kRows * gi) + (uint32_t)l.g;
+                    if (l.t == 0) { to[0] = a0; if (whole) to[8] = a1; }
+                } else {
+#pragma unroll
+                    for (int pr = 0; pr < kIn / 2; ++pr) {
+                        const float a0 = fmaf(acc[gi][pr][0], 16384.0f, __shfl_xor_sync(0xffffffffu, acc[gi][pr][0], 1));
+                        const float a1 = fmaf(acc[gi][pr][1], 16384.0f, __shfl_xor_sync(0xffffffffu, acc[gi][pr][1], 1));
+                        float *to = red + (size_t)(2 * pr + (l.t >> 1)) * consumers * warp_rows + (uint32_t)(kRows * gi) + (uint32_t)l.g;
+                        if ((l.t & 1) == 0) { to[0] = a0; if (whole) to[8] = a1; }
+                    }
+                }
+                // a malformed block scale only counts for rows that exist
+                const uint32_t r_lo = first + (uint32_t)(kRows * gi) + (uint32_t)l.g, r_hi = r_lo + (whole ? 8u : 0u);
+                if (((bad[gi] & 1) && r_lo < nrows) || ((bad[gi] & 2) && r_hi < nrows)) raise(p.status, YVEX_B200_STATUS_NUMERIC);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ctl.red_full[buf]);
+            ++i;
+            c.next();
+        } while (i < n_local && c.m == cur_m);
     }
 }
 
