@@ -518,10 +518,12 @@ def test_gqa_decode_slices_and_block_edges(L, dim, group, sessions, kv, visible,
 
 
 @pytest.mark.parametrize("qtype", [synth.F32, synth.F16, synth.BF16])
-@pytest.mark.parametrize("rows,width,inputs", [(2048, 256, 2), (2051, 1000, 3), (2050, 512, 8), (9473, 264, 9), (2049, 8192, 17), (2048, 16, 4)])
+@pytest.mark.parametrize("rows,width,inputs", [(2048, 256, 2), (2051, 1000, 3), (2050, 512, 8), (9473, 264, 9), (2049, 8192, 17), (2048, 16, 4),
+                                               (4099, 1000, 2), (8195, 264, 4), (14211, 2056, 8), (14209, 4096, 5), (2047, 512, 9)])
 def test_gemv_scalar_qtypes_several_inputs(L, qtype, rows, width, inputs):
     """Four matrix rows per warp and two, four or eight inputs per pass: ragged rows, widths below a warp's chunk and a width
-    whose eight rows do not fit beside each other, against 64 bits (f32 sums of `width` products: 1e-6), with an additive row."""
+    whose eight rows do not fit beside each other, against 64 bits (f32 sums of `width` products: 1e-6), with an additive row
+    and with bf16 results (the f32 result rounded)."""
     import torch
     gen = torch.Generator(device="cuda")
     gen.manual_seed(rows + inputs)
@@ -530,9 +532,33 @@ def test_gemv_scalar_qtypes_several_inputs(L, qtype, rows, width, inputs):
     y = L.gemv(qtype, w.view(torch.uint8).reshape(-1), rows, width, x, st)
     assert st.read() == 0
     assert rel_l2(y.cpu().numpy(), (x.double() @ w.double().T).cpu().numpy()) <= 1e-6
+    add = torch.randn((inputs, rows), device="cuda", generator=gen)
+    plus = L.gemv(qtype, w.view(torch.uint8).reshape(-1), rows, width, x, st, additive=add)
+    assert torch.equal(plus, y + add)
+    assert torch.equal(L.gemv(qtype, w.view(torch.uint8).reshape(-1), rows, width, x, st, additive=add, round_bf16=True), plus.to(torch.bfloat16).float())
+    assert st.read() == 0
     x[inputs - 1, width - 1] = float("inf")
     L.gemv(qtype, w.view(torch.uint8).reshape(-1), rows, width, x, st)
     assert st.read() == 1
+
+
+@pytest.mark.parametrize("qtype", [synth.F32, synth.F16, synth.BF16])
+@pytest.mark.parametrize("width,inputs", [(1024, 4), (2048, 8), (4096, 2), (4096, 8), (8192, 4)])
+def test_gemv_scalar_several_inputs_lose_no_precision(L, qtype, width, inputs):
+    """Rows that share a pass are as close to 64 bits as the same rows one call each: f32 sums of the same products in chains
+    that are no longer. 2 % is what the sampled error of 16384 and more results varies by."""
+    import torch
+    rows, st = 16384, L.Status()
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(width)
+    w = (torch.randn((rows, width), device="cuda", generator=gen) * 0.02).to({synth.F32: torch.float32, synth.F16: torch.float16, synth.BF16: torch.bfloat16}[qtype])
+    x, enc = torch.randn((inputs, width), device="cuda", generator=gen), w.view(torch.uint8).reshape(-1)
+    y = L.gemv(qtype, enc, rows, width, x, st).double()
+    one = torch.stack([L.gemv(qtype, enc, rows, width, x[i], st)[0] for i in range(inputs)]).double()
+    want = x.double() @ w.double().T
+    assert st.read() == 0
+    error, alone = (float((v - want).norm() / want.norm()) for v in (y, one))
+    assert error <= 1.02 * alone, (error, alone)
 
 
 @pytest.mark.parametrize("qtype", [synth.IQ2_XXS, synth.Q4_K, synth.Q8_0, synth.Q2_K, synth.MXFP4])

@@ -179,15 +179,17 @@ __global__ void __launch_bounds__(512) gemv_dense_kernel(const uint8_t *enc, uin
 // Several input rows (a verification or micro-batch step): the matrix is streamed once for up to eight of them instead of once
 // for each. A warp takes four matrix rows, so that an activation read from shared memory is used four times (with one
 // row per warp the reads of eight inputs would hold the kernel to about 1 TB/s), and a chunk's activations stand
-// as 16-byte halves in separate arrays, so that neighbouring lanes read neighbouring slots. Bound by DRAM up to four inputs and
-// by the multiply-adds from eight on. 129280 x 4096 BF16: 207 us for four rows and 295 for eight, where a pass per row took
-// 163 us each; 4096 x 4096: 27 against 56 us for eight.
+// as 16-byte halves in separate arrays, so that neighbouring lanes read neighbouring slots. Sums: a lane takes its products in
+// fours, summed on their own, and adds those in two chains (the halves of a chunk; F32: every other chunk), so that the longest
+// chain is no longer than in gemv_dense_kernel; with eight inputs, whose two chains would not fit in registers, in eights
+// and one chain. (One chain of all products lost precision: 2.2e-7 of the result against 1.2e-7 at 4096 BF16 weights.)
 template <unsigned kQ, int kIn>
 __global__ void __launch_bounds__(512) gemv_dense_multi_kernel(const uint8_t *enc, uint64_t rows, uint64_t width, uint64_t row_bytes,
                                                                const float *input, uint32_t input_rows, const float *additive, float *out,
                                                                int round_bf16, int *status) {
     extern __shared__ __align__(16) float dense_x[];
-    constexpr int kPer = kQ == Q_F32 ? 4 : 8, kHalves = kPer / 4, kRows = 4;
+    // a step of a lane is two groups of four products: the halves of a 16-byte chunk, or (F32) two chunks
+    constexpr int kHalves = kQ == Q_F32 ? 1 : 2, kRows = 4, kChunks = 2 / kHalves, kChains = kIn == 8 ? 1 : 2;
     const uint32_t in0 = blockIdx.y * kIn, here = min((uint32_t)kIn, input_rows - in0), chunks = (uint32_t)(row_bytes / 16);
     float4 *xs = reinterpret_cast<float4 *>(dense_x);                       // [half][input][chunk]
     bool bad = false;
@@ -203,45 +205,69 @@ __global__ void __launch_bounds__(512) gemv_dense_multi_kernel(const uint8_t *en
         const uint4 *rp[kRows];                                             // rows past the end repeat the last one
 #pragma unroll
         for (int r = 0; r < kRows; ++r) rp[r] = reinterpret_cast<const uint4 *>(enc + (r0 + r < rows ? r0 + r : rows - 1) * row_bytes);
-        float acc[kRows][kIn];
+        float acc[kChains][kRows][kIn];
 #pragma unroll
         for (int r = 0; r < kRows; ++r)
 #pragma unroll
-            for (int i = 0; i < kIn; ++i) acc[r][i] = 0.0f;
-        uint4 next[kRows];
+            for (int i = 0; i < kIn; ++i) acc[0][r][i] = acc[kChains - 1][r][i] = 0.0f;
+        uint4 next[kChunks][kRows];
+        auto load = [&](uint32_t c) {                                       // (chunks past the row's end are zeros against the step's first activations)
 #pragma unroll
-        for (int r = 0; r < kRows; ++r) next[r] = (uint32_t)lane < chunks ? __ldcs(rp[r] + lane) : make_uint4(0, 0, 0, 0);
-        for (uint32_t c = lane; c < chunks; c += 32) {
-            uint4 v[kRows];
+            for (int u = 0; u < kChunks; ++u)
 #pragma unroll
-            for (int r = 0; r < kRows; ++r) v[r] = next[r];
-            if (c + 32 < chunks) {
+                for (int r = 0; r < kRows; ++r) next[u][r] = c + 32 * u < chunks ? __ldcs(rp[r] + c + 32 * u) : make_uint4(0, 0, 0, 0);
+        };
+        load((uint32_t)lane);
+        for (uint32_t c = lane; c < chunks; c += 32 * kChunks) {
+            uint4 v[kChunks][kRows];
 #pragma unroll
-                for (int r = 0; r < kRows; ++r) next[r] = __ldcs(rp[r] + c + 32);
-            }
+            for (int u = 0; u < kChunks; ++u)
 #pragma unroll
-            for (int h = 0; h < kHalves; ++h) {
-                float w[kRows][4];
+                for (int r = 0; r < kRows; ++r) v[u][r] = next[u][r];
+            if (c + 32 * kChunks < chunks) load(c + 32 * kChunks);
+            // group g of the step: four weights of each row, and where its activations stand
+            auto weights = [&](int g, float (&w)[kRows][4]) {
 #pragma unroll
                 for (int r = 0; r < kRows; ++r) {
-                    const uint32_t a = h ? v[r].z : v[r].x, b = h ? v[r].w : v[r].y;
+                    const uint4 x = v[kChunks == 2 ? g : 0][r];
+                    const uint32_t a = g ? x.z : x.x, b = g ? x.w : x.y;
                     if (kQ == Q_F32) {
-                        w[r][0] = __uint_as_float(v[r].x); w[r][1] = __uint_as_float(v[r].y); w[r][2] = __uint_as_float(v[r].z); w[r][3] = __uint_as_float(v[r].w);
+                        w[r][0] = __uint_as_float(x.x); w[r][1] = __uint_as_float(x.y); w[r][2] = __uint_as_float(x.z); w[r][3] = __uint_as_float(x.w);
                     } else if (kQ == Q_BF16) {
                         w[r][0] = __uint_as_float(a << 16); w[r][1] = __uint_as_float(a & 0xffff0000u);
                         w[r][2] = __uint_as_float(b << 16); w[r][3] = __uint_as_float(b & 0xffff0000u);
                     } else {
-                        const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&a)), g = __half22float2(*reinterpret_cast<const __half2 *>(&b));
-                        w[r][0] = f.x; w[r][1] = f.y; w[r][2] = g.x; w[r][3] = g.y;
+                        const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&a)), h = __half22float2(*reinterpret_cast<const __half2 *>(&b));
+                        w[r][0] = f.x; w[r][1] = f.y; w[r][2] = h.x; w[r][3] = h.y;
                     }
                 }
+            };
+            const float4 *xg[2] = {xs + c, kChunks == 2 ? xs + (c + 32 < chunks ? c + 32 : c) : xs + kIn * chunks + c};
+            auto dot4 = [](const float (&w)[4], const float4 &x) { return fmaf(w[3], x.w, fmaf(w[2], x.z, fmaf(w[1], x.y, w[0] * x.x))); };
+            if constexpr (kChains == 2) {
+#pragma unroll
+                for (int g = 0; g < 2; ++g) {
+                    float w[kRows][4];
+                    weights(g, w);
+#pragma unroll
+                    for (int i = 0; i < kIn; ++i) {
+                        const float4 x = xg[g][i * chunks];
+#pragma unroll
+                        for (int r = 0; r < kRows; ++r) acc[g][r][i] += dot4(w[r], x);
+                    }
+                }
+            } else {
+                float w0[kRows][4], w1[kRows][4];
+                weights(0, w0);
+                weights(1, w1);
 #pragma unroll
                 for (int i = 0; i < kIn; ++i) {
-                    const float4 x = xs[(h * kIn + i) * chunks + c];
+                    const float4 x0 = xg[0][i * chunks], x1 = xg[1][i * chunks];
 #pragma unroll
                     for (int r = 0; r < kRows; ++r) {
-                        acc[r][i] = fmaf(w[r][0], x.x, acc[r][i]); acc[r][i] = fmaf(w[r][1], x.y, acc[r][i]);
-                        acc[r][i] = fmaf(w[r][2], x.z, acc[r][i]); acc[r][i] = fmaf(w[r][3], x.w, acc[r][i]);
+                        float t = dot4(w0[r], x0);
+                        t = fmaf(w1[r][0], x1.x, t); t = fmaf(w1[r][1], x1.y, t); t = fmaf(w1[r][2], x1.z, t); t = fmaf(w1[r][3], x1.w, t);
+                        acc[0][r][i] += t;
                     }
                 }
             }
@@ -250,7 +276,9 @@ __global__ void __launch_bounds__(512) gemv_dense_multi_kernel(const uint8_t *en
         for (int r = 0; r < kRows; ++r)
 #pragma unroll
             for (int i = 0; i < kIn; ++i) {
-                float sum = warp_sum(acc[r][i]);
+                float sum = acc[0][r][i];
+                if (kChains == 2) sum += acc[kChains - 1][r][i];
+                sum = warp_sum(sum);
                 if (lane == 0 && r0 + r < rows && (uint32_t)i < here) {
                     const uint64_t job = (uint64_t)(in0 + i) * rows + r0 + r;
                     if (additive) sum += additive[job];
@@ -264,9 +292,7 @@ __global__ void __launch_bounds__(512) gemv_dense_multi_kernel(const uint8_t *en
 
 template <unsigned kQ>
 static int gemv_dense_multi_launch(const uint8_t *enc, uint64_t rows, uint64_t width, uint64_t row_bytes, const float *input, uint64_t input_rows,
-                                   const float *additive, float *out, int round_bf16, int *status, cudaStream_t s) {
-    // eight inputs where their rows fit beside each other in shared memory, else four (48 KB of row at most: 192 KB)
-    const int in = input_rows <= 2 ? 2 : input_rows <= 4 || width * 32 > 200 * 1024 ? 4 : 8;
+                                   const float *additive, float *out, int round_bf16, int *status, cudaStream_t s, int in) {
     const size_t smem = (size_t)in * width * 4;
     static SmemOptIn opt_in[3];
     auto *kernel = in == 2 ? gemv_dense_multi_kernel<kQ, 2> : in == 4 ? gemv_dense_multi_kernel<kQ, 4> : gemv_dense_multi_kernel<kQ, 8>;
@@ -283,13 +309,21 @@ static bool gemv_dense_eligible(unsigned q, uint64_t width, uint64_t row_bytes, 
            ((reinterpret_cast<uintptr_t>(enc) | reinterpret_cast<uintptr_t>(input)) & 15u) == 0 && (width * 4) % 16 == 0;
 }
 
+// Input rows a pass over the matrix serves.
+static int dense_pass_inputs(uint64_t rows, uint64_t width, uint64_t input_rows) {
+    // (below 2048 rows there are too few four-row warps for the chip, and the matrix comes from L2 anyway)
+    if (input_rows == 1 || rows < 2048) return 1;
+    // eight inputs where their rows fit beside each other in shared memory, else four (48 KB of row at most: 192 KB)
+    return input_rows <= 2 ? 2 : input_rows <= 4 || width * 32 > 200 * 1024 ? 4 : 8;
+}
+
 static int gemv_dense_launch(unsigned q, const uint8_t *enc, uint64_t rows, uint64_t width, uint64_t row_bytes, const float *input,
                              uint64_t input_rows, const float *additive, float *out, int round_bf16, int *status, cudaStream_t s) {
-    // (below 2048 rows there are too few four-row warps for the chip, and the matrix comes from L2 anyway)
-    if (input_rows > 1 && rows >= 2048) {
-        if (q == Q_F32) return gemv_dense_multi_launch<Q_F32>(enc, rows, width, row_bytes, input, input_rows, additive, out, round_bf16, status, s);
-        if (q == Q_F16) return gemv_dense_multi_launch<Q_F16>(enc, rows, width, row_bytes, input, input_rows, additive, out, round_bf16, status, s);
-        return gemv_dense_multi_launch<Q_BF16>(enc, rows, width, row_bytes, input, input_rows, additive, out, round_bf16, status, s);
+    const int in = dense_pass_inputs(rows, width, input_rows);
+    if (in > 1) {
+        if (q == Q_F32) return gemv_dense_multi_launch<Q_F32>(enc, rows, width, row_bytes, input, input_rows, additive, out, round_bf16, status, s, in);
+        if (q == Q_F16) return gemv_dense_multi_launch<Q_F16>(enc, rows, width, row_bytes, input, input_rows, additive, out, round_bf16, status, s, in);
+        return gemv_dense_multi_launch<Q_BF16>(enc, rows, width, row_bytes, input, input_rows, additive, out, round_bf16, status, s, in);
     }
     const uint64_t want = (rows + 15) / 16, cap = (uint64_t)kSmCount * 4;
     const dim3 grid((unsigned)(want < cap ? want : cap), (unsigned)input_rows);
