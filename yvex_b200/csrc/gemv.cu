@@ -309,12 +309,20 @@ static bool gemv_dense_eligible(unsigned q, uint64_t width, uint64_t row_bytes, 
            ((reinterpret_cast<uintptr_t>(enc) | reinterpret_cast<uintptr_t>(input)) & 15u) == 0 && (width * 4) % 16 == 0;
 }
 
-// Input rows a pass over the matrix serves.
+// Input rows a pass over the matrix serves (1: a pass per row). A matrix of few rows is all latency: it wants many CTAs, so passes
+// of fewer inputs side by side; a large one wants to be read once. Measured (us, passes of 1 / 2 / 4 / 8 inputs):
+//   BF16  2048 x 1024   2 rows 4.0 / 4.3 / 5 / 9     4 rows 6.5 / 4.5 / 5.3 / 10   8 rows 11 / 5.3 / 5.4 / 11
+//   BF16  4096 x 4096   2 rows 17 / 9.1 / 11 / 19    4 rows 30 / 12.2 / 13 / 20    8 rows 53 / 22 / 18 / 23
+//   BF16  8192 x 2048   2 rows 16 / 7.6 / 10 / 17    4 rows 29 / 13 / 11 / 18      8 rows 55 / 24 / 19 / 20
+//   BF16 32768 x 4096   2 rows 90 / 59 / 62 / 86     4 rows 174 / 107 / 63 / 88    8 rows 344 / 208 / 113 / 92
+// (F32 alike; below 2048 rows one row per pass is within a tenth up to four rows). Eight pay where their reads of shared memory
+// are a small part, from about 2048 weights a row. One costs 1.7 passes of four there, so that nine to twelve rows take fours, and 1.4 from 4096 on.
 static int dense_pass_inputs(uint64_t rows, uint64_t width, uint64_t input_rows) {
-    // (below 2048 rows there are too few four-row warps for the chip, and the matrix comes from L2 anyway)
-    if (input_rows == 1 || rows < 2048) return 1;
-    // eight inputs where their rows fit beside each other in shared memory, else four (48 KB of row at most: 192 KB)
-    return input_rows <= 2 ? 2 : input_rows <= 4 || width * 32 > 200 * 1024 ? 4 : 8;
+    if (input_rows == 1 || rows < 2048 || (input_rows == 2 && rows < 4096)) return 1;
+    if (input_rows == 2 || (input_rows <= 4 && rows < 8192) || (input_rows <= 8 && rows < 4096)) return 2;
+    const uint64_t fours = (input_rows + 3) / 4, eights = (input_rows + 7) / 8;
+    // (eight rows of activations beside each other in shared memory: 200 KB; four of the widest row, 48 KB, always fit)
+    return rows >= 96ull * kSmCount && width >= 2048 && width * 32 <= 200 * 1024 && (width < 4096 ? 17 : 14) * eights < 10 * fours ? 8 : 4;
 }
 
 static int gemv_dense_launch(unsigned q, const uint8_t *enc, uint64_t rows, uint64_t width, uint64_t row_bytes, const float *input,
