@@ -562,10 +562,11 @@ def test_gemv_scalar_several_inputs_lose_no_precision(L, qtype, width, inputs):
 
 
 @pytest.mark.parametrize("qtype", [synth.IQ2_XXS, synth.Q4_K, synth.Q8_0, synth.Q2_K, synth.MXFP4])
-@pytest.mark.parametrize("rows,width,inputs", [(17, 512, 2), (33, 1536, 3), (300, 4096, 8), (5, 7168, 5), (64, 1024, 4), (40, 256, 6), (16, 8192, 9)])
+@pytest.mark.parametrize("rows,width,inputs", [(17, 512, 2), (33, 1536, 3), (300, 4096, 8), (5, 7168, 5), (64, 1024, 4), (40, 256, 6), (16, 8192, 9),
+                                               (65539, 512, 8), (32777, 1536, 7), (16411, 4096, 6), (9001, 5120, 9)])
 def test_gemv_block_qtypes_several_inputs(L, qtype, rows, width, inputs):
-    """Passes of four input rows against one call per row: full and ragged passes, ragged tiles, rows and planes of every
-    slicing, widths whose planes leave no room for four rows (those take one row per pass). Exact integer products and the
+    """Several input rows against one call per row: small matrices and widths whose planes leave no room for four rows (a pass per
+    row), large ones in passes of four, full and ragged passes, ragged tiles, rows and planes of every slicing. Exact integer products and the
     same f32 steps: 1e-6 covers another slicing of K. One non-finite value in the last row is refused."""
     import torch
     if qtype == synth.MXFP4 and width % 512:
@@ -574,7 +575,8 @@ def test_gemv_block_qtypes_several_inputs(L, qtype, rows, width, inputs):
     gen = torch.Generator(device="cuda")
     gen.manual_seed(inputs)
     x, add, st = torch.randn((inputs, width), device="cuda", generator=gen), torch.randn((inputs, rows), device="cuda", generator=gen), L.Status()
-    x *= torch.logspace(-3, 3, inputs, device="cuda")[:, None]           # every row needs its own scale
+    scale = torch.logspace(-3, 3, inputs, device="cuda")[:, None]        # every row needs its own
+    x, add = x * scale, add * scale
     y = L.gemv(qtype, w, rows, width, x, st, additive=add)
     one = torch.stack([L.gemv(qtype, w, rows, width, x[i], st, additive=add[i])[0] for i in range(inputs)])
     assert st.read() == 0
@@ -591,9 +593,9 @@ def test_gemv_block_qtypes_several_inputs(L, qtype, rows, width, inputs):
 def test_gemv_several_inputs_lose_no_precision(L, qtype, width, mean):
     """Rows that share a decode are as close to 64 bits over the decoded weights as the same rows one call each, inputs with a
     mean included (the minimum terms of Q4_K and Q2_K and MXFP4's offset then cancel large sums). Both are f32 sums of the same
-    exact products in another order; 5 % is what the sampled error of 8 x 1024 results varies by, 2e-8 the f32 result itself."""
+    exact products in another order; 5 % is what the sampled error of that many results varies by, 2e-8 the f32 result itself."""
     import torch
-    rows, inputs = 1024, 8
+    rows, inputs = 16395, 7
     w = dev(synth.random_blocks(qtype, rows, width, width))
     gen = torch.Generator(device="cuda")
     gen.manual_seed(width)

@@ -35,8 +35,16 @@ def test_only_consecutive_rows_of_one_matrix_share_a_decode(ask, name):
     matrices and SwiGLU inputs are one row to a pass, whatever the width."""
     widths = range(512, 8193, 512)
     forms = [(count, stride, ptrs, rows, act) for count in (1, 2, 5, 62) for stride in (0, 4096) for ptrs in (0, 1) for rows in (0, 1) for act in (0, 1)]
-    asked = [(BLOCK[name], w, *f) for w in widths for f in forms]
+    asked = [(BLOCK[name], 65536, w, *f) for w in widths for f in forms]
     for q, per_pass in zip(asked, ask(asked)):
-        count, stride, ptrs, rows, act = q[2:]
+        count, stride, ptrs, rows, act = q[3:]
         assert per_pass in ((1, 4) if count > 1 and not (stride or ptrs or rows or act) else (1,)), (q, per_pass)
-    assert 4 in ask([(BLOCK[name], 2048, 8, 0, 0, 0, 0)])
+    assert ask([(BLOCK[name], 65536, 2048, 8, 0, 0, 0, 0)]) == [4]
+
+
+@pytest.mark.parametrize("name", BLOCK)
+def test_small_matrices_take_a_pass_per_row(ask, name):
+    """Two rows of a matrix that one round of tiles covers, and any few rows of a small one, are faster alone; a matrix of many
+    rounds shares its decode whatever the count from four rows on (rows of up to 4096 weights: more may not fit)."""
+    assert set(ask([(BLOCK[name], rows, width, n, 0, 0, 0, 0) for rows in (1, 17, 256, 512) for width in (512, 1024, 2048, 4096) for n in (2, 3, 4, 5)])) == {1}
+    assert set(ask([(BLOCK[name], 65536, width, n, 0, 0, 0, 0) for width in (1024, 2048, 4096) for n in (4, 8, 12, 16)])) == {4}

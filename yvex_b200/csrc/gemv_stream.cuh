@@ -1178,14 +1178,32 @@ inline int stream_launch_t(StreamParams &p, const StreamShape &sh, int inputs, c
 
 struct StreamActivation { const float *up; const float *weight; float limit; };
 
-// Input rows one pass over a matrix serves (0: no shape fits), and its shape. Several input rows of ONE matrix: passes of up to
-// four rows that share each tile's decode, from two rows on (a pass costs 1.3 to 1.7 of a single row's) and where four rows'
-// planes leave room for a ring. Rows named by a table (x_rows) are one to a matrix: a pass takes consecutive ones.
-inline int pass_inputs(unsigned q, uint64_t width, uint64_t row_bytes, uint64_t count, uint64_t matrix_stride, const uint8_t *const *matrix_ptrs,
-                       const uint32_t *x_rows, const StreamActivation *act, StreamShape &sh) {
-    const bool shared = count > 1 && matrix_stride == 0 && !matrix_ptrs && !x_rows && !act;
-    if (shared && stream_shape(q, width, row_bytes, sh, kMaxInputs) && sh.consumers >= kMaxInputs) return kMaxInputs;
-    return stream_shape(q, width, row_bytes, sh) ? 1 : 0;
+// 16-row groups x 256-weight units that a warp of the busiest CTA decodes.
+inline uint64_t stream_rounds(const StreamShape &sh, uint64_t rows, uint64_t matrices) {
+    const uint64_t tile_rows = (uint64_t)sh.group_rows * sh.groups * sh.row_warps, tiles = matrices * ((rows + tile_rows - 1) / tile_rows);
+    return (tiles + kSmCount - 1) / kSmCount * (uint64_t)(sh.groups * sh.units_per_slice);
+}
+
+// Input rows one pass over a matrix serves (0: no shape fits), and its shape. Several input rows of ONE matrix may run in passes of
+// up to four that share each tile's decode, where four rows' planes leave room for a ring. Rows named by a table (x_rows) are one
+// to a matrix: a pass takes consecutive ones. Sharing costs more per group and unit and prepares four rows' digits with a
+// quarter of the warps each, so it pays when the busiest warp's work falls by enough: one row's rounds >= cost x shared rounds +
+// fixed + 2 x width / 4096, with cost and fixed fitted per qtype to 2 .. 16 rows of twenty matrix sizes (us, a pass per row / shared):
+//   4096 x 4096, 2 rows: IQ2_XXS 11 / 12, Q4_K 10 / 12, MXFP4 11 / 16.5     8 rows: IQ2_XXS 24 / 17, Q4_K 22 / 19, MXFP4 27 / 25
+//   512 x 2048, 8 rows: Q4_K 6.0 / 8.6, Q8_0 7.1 / 10.6                       16384 x 4096, 8 rows: IQ2_XXS 73 / 43, Q4_K 79 / 47, MXFP4 88 / 65
+// Rows of a multiple of 128 bytes put the eight rows of an MXFP4 fragment on the same banks; one or two slices are few warps.
+inline int pass_inputs(unsigned q, uint64_t rows, uint64_t width, uint64_t row_bytes, uint64_t count, uint64_t matrix_stride,
+                       const uint8_t *const *matrix_ptrs, const uint32_t *x_rows, const StreamActivation *act, StreamShape &sh) {
+    if (!stream_shape(q, width, row_bytes, sh)) return 0;
+    StreamShape several;
+    if (count < 2 || matrix_stride || matrix_ptrs || x_rows || act || !stream_shape(q, width, row_bytes, several, kMaxInputs) || several.consumers < kMaxInputs)
+        return 1;
+    unsigned cost10 = q == Q_Q8_0 ? 16 : q == Q_IQ2_XXS ? 17 : q == Q_Q2_K ? 20 : q == Q_Q4_K ? 24 : row_bytes % 128 == 0 ? 26 : 17;
+    if (several.slices <= 2) cost10 = 32;
+    const uint64_t one = stream_rounds(sh, rows, count), shared = stream_rounds(several, rows, (count + kMaxInputs - 1) / kMaxInputs);
+    if (10 * one < cost10 * shared + (q == Q_Q2_K ? 20 : 5) + 20 * width / 4096) return 1;
+    sh = several;
+    return kMaxInputs;
 }
 
 inline int stream_launch(unsigned q, const uint8_t *enc, uint64_t matrix_stride, uint64_t count, uint64_t rows, uint64_t width,
@@ -1194,7 +1212,7 @@ inline int stream_launch(unsigned q, const uint8_t *enc, uint64_t matrix_stride,
                          const uint8_t *const *matrix_ptrs = nullptr, const uint32_t *x_rows = nullptr,
                          const StreamActivation *act = nullptr) {
     StreamShape sh;
-    const int inputs = pass_inputs(q, width, row_bytes, count, matrix_stride, matrix_ptrs, x_rows, act, sh);
+    const int inputs = pass_inputs(q, rows, width, row_bytes, count, matrix_stride, matrix_ptrs, x_rows, act, sh);
     if (!inputs) return ERR_BOUNDS;
     StreamParams p{};
     p.inputs = (uint32_t)count;
