@@ -161,3 +161,16 @@ def test_expert_parallel_entry_refuses_bad_arguments_before_touching_nccl(lib):
     assert B._lib.yvex_moe_ep_open(C.byref(ep), None, ident, 2, 0, 1000, C.byref(err)) == B.INVALID_ARG and not ep.value
     assert B._lib.yvex_moe_ep_execute_rows(None, None, None, None, None, C.byref(err)) == B.INVALID_ARG
     assert B._lib.yvex_moe_ep_close(C.byref(ep), C.byref(err)) == B.OK
+
+
+def test_attention_workspace_is_monotone_and_bounded(lib):
+    """A workspace sized for a context serves every prefix of it, and slices never ask for more than three waves of CTAs where one
+    slice per group is less: what the fixed 8 MiB array took with one slice per group, it takes at every length."""
+    for dim, group in ((64, 1), (64, 4), (128, 2), (128, 4), (256, 1), (256, 4)):
+        wave = 148 * (4 if dim == 64 else 3)
+        for groups in list(range(1, 700, 7)) + [444, 592, 1000, 1776, 1777, 5000]:
+            need = [int(lib.lib.yvex_b200_attention_workspace_bytes(1, groups * group, groups, dim, c))
+                    for c in (1, 63, 64, 65, 100, 128, 129, 300, 700, 1500, 4000, 16000, 60000, 1 << 20)]
+            one = groups * group * (dim + 2) * 4
+            assert need[0] == one and need == sorted(need)
+            assert need[-1] <= max(one, 3 * wave * group * (dim + 2) * 4) and 3 * wave * group * (dim + 2) * 4 <= 8 << 20

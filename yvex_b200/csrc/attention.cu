@@ -228,9 +228,16 @@ __global__ void __launch_bounds__(D) gqa_merge_kernel(const float *__restrict__ 
         if (threadIdx.x == 0) denominator = gl;
     }
     __syncthreads();
-    float acc = 0.0f;
-#pragma unroll 8
-    for (int s = 0; s < splits; ++s) acc += p[s * pitch + 2 + d] * factor[s];
+    float acc = splits == 1 ? p[2 + d] * factor[0] : 0.0f;
+    // (eight loads at a time whatever the count: a loop for the remainder waits for one load after the other, and twelve slices
+    // of 1 x 8 heads x 700 keys took 6.3 us where eight or sixteen took 5.8)
+    for (int s0 = 0; s0 < splits && splits > 1; s0 += 8) {
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = s0 + i < splits ? p[(s0 + i) * pitch + 2 + d] : 0.0f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc += v[i] * factor[s0 + i];
+    }
     const float o = acc / denominator;
     if (!(denominator > 0.0f) || !isfinite(o)) raise(status, YVEX_B200_STATUS_NUMERIC);
     out[(sk * G + h) * D + d] = o;
@@ -360,18 +367,28 @@ __global__ void __launch_bounds__(32 * kSinkWarps) attention_sink_kernel(const f
     }
 }
 
-static int pick_splits(uint64_t groups, uint64_t visible) {
-    // Enough CTAs to fill 148 SMs a few times over with at least 64 keys per slice (one block per warp: a short context is
-    // all latency; 1500 keys x 8 heads at 256 keys per slice are 48 CTAs of four serial blocks per warp); among those with at least 256 keys prefer a count that makes
-    // groups * splits a whole number of waves (a multiple of the SM count). The count never falls when `visible` grows, so a
-    // workspace sized for the whole context serves every prefix.
-    const uint64_t want = ((uint64_t)kSmCount * 4 + groups - 1) / groups;
-    const uint64_t most = (visible + 63) / 64, cap = (visible + 255) / 256;
-    uint64_t s = want < most ? want : most;
-    s = s < 1 ? 1 : s > kMaxSplits ? kMaxSplits : s;
-    for (uint64_t t = s; t <= s + 40 && t <= cap && t <= kMaxSplits; ++t)
-        if ((groups * t) % kSmCount == 0) { s = t; break; }
-    return (int)s;
+static int pick_splits(uint64_t groups, uint64_t visible, uint64_t head_dim) {
+    // The slices of a call run in waves of as many CTAs as fit the chip (registers: four per SM at 64 dims, three at 128 and 256),
+    // and a wave that is not full costs as much as a full one. Few groups: as many slices as one wave holds, down to 64 keys
+    // (a block per warp). Many: the count within three waves whose last is fullest, 4 % charged per slice for its merge, down to
+    // 128 keys. (us, this / 64-key slices up to four CTAs an SM, in any number of waves: 32 groups of four heads x 128, 1500 keys 11 / 15;
+    // 128 groups x 700 13 / 17; 8 groups x 60000 54 / 69; 64 groups of one head x 256, 1500 keys 31 / 40. 162 shapes: 2 % over the best count, 15 % before.)
+    // The count never falls when `visible` grows, so a workspace sized for the whole context serves every prefix, and
+    // beyond one slice per group it stays within three waves.
+    const uint64_t wave = (uint64_t)kSmCount * (head_dim == 64 ? 4 : 3);
+    uint64_t s = 1, most = (visible + 127) / 128;
+    if (2 * groups <= wave) {
+        s = wave / groups;
+        most = (visible + 63) / 64;
+    } else {
+        uint64_t least = ~0ull;
+        for (uint64_t t = 1; t == 1 || (t <= kMaxSplits && groups * t <= 3 * wave); ++t) {
+            const uint64_t cost = (groups * t + wave - 1) / wave * wave * 100 / (groups * t) + 4 * t;
+            if (cost < least) { least = cost; s = t; }
+        }
+    }
+    s = s < most ? s : most;
+    return (int)(s < kMaxSplits ? s : kMaxSplits);
 }
 
 template <int D>
@@ -396,7 +413,7 @@ using namespace yb;
 extern "C" uint64_t yvex_b200_attention_workspace_bytes(uint64_t sessions, uint64_t q_heads, uint64_t kv_heads,
                                                         uint64_t head_dim, uint64_t context) {
     if (!kv_heads) return 0;
-    int splits = pick_splits(sessions * kv_heads, context);
+    int splits = pick_splits(sessions * kv_heads, context, head_dim);
     return sessions * q_heads * (uint64_t)splits * (head_dim + 2) * sizeof(float);
 }
 
@@ -410,7 +427,7 @@ extern "C" int yvex_b200_attention_gqa_decode(const void *q, const void *k, cons
     if (q_heads % kv_heads) return ERR_INVALID_ARG;
     if (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 15u) return ERR_INVALID_ARG;
     const uint64_t group = q_heads / kv_heads, visible = position + 1;
-    const int splits = pick_splits(sessions * kv_heads, visible);
+    const int splits = pick_splits(sessions * kv_heads, visible, head_dim);
     const uint64_t need = sessions * q_heads * (uint64_t)splits * (head_dim + 2) * sizeof(float);
     if (!workspace || workspace_bytes < need) return ERR_NOMEM;
     const uint16_t *qq = (const uint16_t *)q, *kk = (const uint16_t *)k, *vv = (const uint16_t *)v;
