@@ -368,27 +368,21 @@ __global__ void __launch_bounds__(32 * kSinkWarps) attention_sink_kernel(const f
 }
 
 static int pick_splits(uint64_t groups, uint64_t visible, uint64_t head_dim) {
-    // The slices of a call run in waves of as many CTAs as fit the chip (registers: four per SM at 64 dims, three at 128 and 256),
-    // and a wave that is not full costs as much as a full one. Few groups: as many slices as one wave holds, down to 64 keys
-    // (a block per warp). Many: the count within three waves whose last is fullest, 4 % charged per slice for its merge, down to
-    // 128 keys. (us, this / 64-key slices up to four CTAs an SM, in any number of waves: 32 groups of four heads x 128, 1500 keys 11 / 15;
-    // 128 groups x 700 13 / 17; 8 groups x 60000 54 / 69; 64 groups of one head x 256, 1500 keys 31 / 40. 162 shapes: 2 % over the best count, 15 % before.)
-    // The count never falls when `visible` grows, so a workspace sized for the whole context serves every prefix, and
-    // beyond one slice per group it stays within three waves.
-    const uint64_t wave = (uint64_t)kSmCount * (head_dim == 64 ? 4 : 3);
-    uint64_t s = 1, most = (visible + 127) / 128;
-    if (2 * groups <= wave) {
-        s = wave / groups;
-        most = (visible + 63) / 64;
-    } else {
-        uint64_t least = ~0ull;
-        for (uint64_t t = 1; t == 1 || (t <= kMaxSplits && groups * t <= 3 * wave); ++t) {
-            const uint64_t cost = (groups * t + wave - 1) / wave * wave * 100 / (groups * t) + 4 * t;
-            if (cost < least) { least = cost; s = t; }
-        }
-    }
-    s = s < most ? s : most;
-    return (int)(s < kMaxSplits ? s : kMaxSplits);
+    // Enough CTAs to fill 148 SMs a few times over with at least 256 keys per slice; among those prefer a count that makes
+    // groups * slices a whole number of waves (a multiple of the SM count). Short contexts are all latency: they are cut down to
+    // 64 keys (a block per warp) as long as every slice fits the chip at once - registers leave room for four CTAs per SM
+    // at 64 dims, three at 128 and 256 -, since one CTA more costs a second wave (64 groups of one head x 256, 1500 keys: 6 slices
+    // 30 us, 10 slices 40; 8 x 128, 1500 keys: 6 slices 9.4, 24 slices 8.1). Fewer and longer slices than this would be faster
+    // at some lengths, but f32 sums over a slice lose precision with its length (64 keys 1.5e-6, 1024 2.1e-6, 10923 6.7e-6).
+    // The count never falls when `visible` grows, so a workspace sized for the whole context serves every prefix.
+    const uint64_t want = ((uint64_t)kSmCount * 4 + groups - 1) / groups, cap = (visible + 255) / 256;
+    const uint64_t wave = (uint64_t)kSmCount * (head_dim == 64 ? 4 : 3), fine = wave / groups, finest = (visible + 63) / 64;
+    uint64_t s = want < cap ? want : cap;
+    for (uint64_t t = s; t <= s + 40 && t <= cap && t <= kMaxSplits; ++t)
+        if ((groups * t) % kSmCount == 0) { s = t; break; }
+    const uint64_t shortened = fine < finest ? fine : finest;
+    s = s > shortened ? s : shortened;
+    return (int)(s < 1 ? 1 : s > kMaxSplits ? kMaxSplits : s);
 }
 
 template <int D>
