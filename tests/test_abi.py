@@ -163,6 +163,14 @@ def test_expert_parallel_entry_refuses_bad_arguments_before_touching_nccl(lib):
     assert B._lib.yvex_moe_ep_close(C.byref(ep), C.byref(err)) == B.OK
 
 
+def test_kernels_write_out_no_mathematics():
+    """Divisions, roots and exponentials are CUDA's own functions: no approximate instruction refined by hand."""
+    csrc = os.path.join(ROOT, "yvex_b200", "csrc")
+    for f in sorted(os.listdir(csrc)):
+        text = open(os.path.join(csrc, f)).read()
+        assert not re.search(r"\b(rcp|div|sqrt|rsqrt|ex2|lg2|sin|cos|tanh)\.(approx|full|r[nzmp])\b", text), f
+
+
 def test_attention_workspace_is_monotone_and_bounded(lib):
     """A workspace sized for a context serves every prefix of it, and slices of fewer than 256 keys are only made while all of
     them fit the chip at once."""

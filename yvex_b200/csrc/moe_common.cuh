@@ -18,19 +18,6 @@ __device__ __forceinline__ float swiglu_product(float g, float u, float route_we
     const float silu = (g >= 0.0f ? g : g * t) / (1.0f + t);
     return silu * u * route_weight;
 }
-// The same without the route weight, for a tile end that is bound by issue slots: the denominator lies in [1, 2], so the
-// quotient is a hardware reciprocal and one Newton correction of the residual - accurate to the last bit or its
-// neighbour - instead of the general division with its range checks.
-__device__ __forceinline__ float swiglu_product_bounded(float g, float u, float limit) {
-    g = fminf(g, limit);
-    u = fmaxf(-limit, fminf(u, limit));
-    const float t = expf(-fabsf(g)), num = g >= 0.0f ? g : g * t, den = 1.0f + t;
-    float r;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(den));
-    r = fmaf(r, fmaf(-den, r, 1.0f), r);
-    const float q = num * r;
-    return fmaf(r, fmaf(-den, q, num), q) * u;
-}
 __device__ __forceinline__ float swiglu_mid(float g, float u, float route_weight, float limit, int *status) {
     const float mid = swiglu_product(g, u, route_weight, limit);
     if (!isfinite(mid)) raise(status, YVEX_B200_STATUS_NUMERIC);

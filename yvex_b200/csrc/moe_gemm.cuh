@@ -688,7 +688,7 @@ moe_grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, GemmParams p) {
                     for (int b = 0; b < 4; ++b) wv[b] = __shfl_sync(0xffffffffu, wl, 8 * b + 2 * rr + (odd ? 1 : 0));
 #pragma unroll
                     for (int m = 0; m < 16; ++m)                        // g[m] = silu(gate) * up
-                        g[m] = swiglu_product_bounded(g[2 * m], g[2 * m + 1], p.limit);
+                        g[m] = swiglu_product(g[2 * m], g[2 * m + 1], 1.0f, p.limit);
 #pragma unroll
                     for (int b = 0; b < 4; ++b) {
                         float *r = g + 4 * b;
