@@ -178,7 +178,10 @@ uint64_t yvex_b200_moe_wide_workspace_bytes(const yvex_b200_moe_geometry *g, uin
  * qtypes or a weight pack that does not start on a 16-byte boundary send it to the row kernels
  * (same results, far slower). Lets a caller report or refuse the slow path instead of meeting it. */
 int yvex_b200_moe_wide_uses_gemm(const yvex_b200_moe_geometry *g, const yvex_b200_moe_weights *w);
-/* Token columns of one grouped-GEMM tile for a weight qtype (0: the qtype has no GEMM decoder). */
+/* Most token columns of one grouped-GEMM tile for a weight qtype (0: the qtype has no GEMM decoder). An expert's rows are cut
+ * into tiles of equal width, a multiple of YVEX_B200_MOE_TILE_STEP columns, so the rows a run in one piece multiplies for
+ * padding are those up to the next multiple. */
+#define YVEX_B200_MOE_TILE_STEP 16
 uint64_t yvex_b200_moe_wide_tile_columns(unsigned int qtype);
 int yvex_b200_moe_wide(const yvex_b200_moe_geometry *g, const yvex_b200_moe_weights *w,
                        const float *x, const float *logits, const uint32_t *token_ids,

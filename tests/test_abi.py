@@ -163,6 +163,16 @@ def test_expert_parallel_entry_refuses_bad_arguments_before_touching_nccl(lib):
     assert B._lib.yvex_moe_ep_close(C.byref(ep), C.byref(err)) == B.OK
 
 
+def test_tile_columns_are_those_of_the_grouped_gemm(lib):
+    """Most columns of a tile: what the kernel's plan gives each qtype room for, and a multiple of the step tiles grow by."""
+    text = open(os.path.join(ROOT, "yvex_b200", "csrc", "moe_gemm.cuh")).read()
+    affine, plain = map(int, re.search(r"kTileN = kHasMin \? (\d+) : (\d+);", text).groups())
+    columns = {q: int(lib.lib.yvex_b200_moe_wide_tile_columns(q)) for q in (0, 1, 8, 10, 12, 16, 30, 39, 43)}
+    assert columns == {16: plain, 12: affine, 10: affine, 0: 0, 1: 0, 8: 0, 30: 0, 39: 0, 43: 0}
+    step = int(re.search(r"#define YVEX_B200_MOE_TILE_STEP (\d+)", open(os.path.join(ROOT, "include", "yvex_b200_kernels.h")).read()).group(1))
+    assert plain % step == 0 and affine % step == 0
+
+
 def test_kernels_write_out_no_mathematics():
     """Divisions, roots and exponentials are CUDA's own functions: no approximate instruction refined by hand."""
     csrc = os.path.join(ROOT, "yvex_b200", "csrc")

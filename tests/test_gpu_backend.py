@@ -508,6 +508,8 @@ def test_execute_rows_wide_copy_pipeline_is_bit_identical(B):
     assert (out.view(np.uint32) == whole.reshape(T, H).view(np.uint32)).all()
     assert res.unique_experts == res2.unique_experts == E
     assert res.worklists.tensor_core_eligible_pairs == T * k and res.worklists.narrow_pairs == 0
+    # an expert's tiles are equally wide, multiples of 16 columns: the last one's padding is all there is
+    assert res.worklists.tail_rows == sum(-int(n) % 16 for n in np.bincount(sel.ravel().astype(np.int64), minlength=E))
     assert be.close() == B.OK
 
 

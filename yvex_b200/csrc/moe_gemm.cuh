@@ -53,6 +53,8 @@
 
 namespace yb {
 
+constexpr int kTileStep = YVEX_B200_MOE_TILE_STEP;               // columns a group's last tile is padded to
+static_assert(kTileStep == 16, "the N of tcgen05.mma kind::f16 at M = 128 is a multiple of 16");
 constexpr int kTileM = 128, kBoxN = 64, kMinTileN = 128, kChunkK = 64;
 constexpr uint32_t kBoxBytes = kBoxN * kChunkK * 2;          // activations arrive in boxes of 64 rows: a ragged tile fetches what it needs
 constexpr uint32_t kMinTileBytes = kTileM * 64;               // 8 KiB: A' or B' of the min term, 32 fp16 per row, 64-byte swizzle

@@ -82,9 +82,9 @@ __global__ void wide_plan_kernel(const int *counts, int experts, uint64_t pairs,
         const int row0 = off + row_end - count, blk0 = nb + blk_end - nblocks;
         if (e <= experts) {
             if (blockIdx.x == 0) offsets[e] = row0;
-            // an expert's rows in blocks of equal width (rounded up to the MMA's 16 columns): the tensor time follows the width,
+            // an expert's rows in blocks of equal width (rounded up to the MMA's columns): the tensor time follows the width,
             // while a full block beside a nearly empty one would decode the same weights for both
-            const int width = nblocks ? ((count + nblocks - 1) / nblocks + 15) & ~15 : 0;
+            const int width = nblocks ? ((count + nblocks - 1) / nblocks + kTileStep - 1) / kTileStep * kTileStep : 0;
             for (int b = 0; b < nblocks; ++b) {
                 const int first = blk0 + b - b % per_group;
                 const int in_group = min(per_group, nblocks - (b - b % per_group));
@@ -609,8 +609,7 @@ extern "C" int yvex_b200_moe_wide_uses_gemm(const yvex_b200_moe_geometry *g, con
 }
 
 extern "C" uint64_t yvex_b200_moe_wide_tile_columns(unsigned int qtype) {
-    // the width the worklist counts its tails in; a tile takes at most as many columns (224 or 128, in blocks of equal width)
-    return gemm_qtype(qtype) ? qtype == Q_IQ2_XXS ? 256 : 128 : 0;
+    return gemm_qtype(qtype) ? (uint64_t)gemm_tile_n(qtype) : 0;
 }
 
 extern "C" uint64_t yvex_b200_moe_wide_workspace_bytes(const yvex_b200_moe_geometry *g, uint64_t rows) {
@@ -1138,7 +1137,7 @@ extern "C" int yvex_b200_expert_worklist(const int32_t *selected, uint64_t rows,
     ColBlock *b1 = reinterpret_cast<ColBlock *>(take((uint64_t)max_blocks * sizeof(ColBlock)));
     cudaMemsetAsync(counts, 0, (experts + 2) * 4, s);
     wide_count_kernel<<<grid_for(pairs, 256, 4), 256, 0, s>>>(selected, pairs, (int)experts + 1, counts, status);
-    wide_plan_kernel<<<2, 32, 0, s>>>(counts, (int)experts, pairs, offsets, b0, b1, num_blocks, max_blocks, 256, 128, status);
+    wide_plan_kernel<<<2, 32, 0, s>>>(counts, (int)experts, pairs, offsets, b0, b1, num_blocks, max_blocks, kMinTileN, kMinTileN, status);      // (only the offsets are read)
     worklist_observe_kernel<<<1, 32, 0, s>>>(counts, offsets, (int)experts, pairs, rows, tensor_core_minimum, admitted_width, provenance,
                                              observation, expert_ids, bucket_offsets, bucket_populations, status);
     int launches = 3;

@@ -213,11 +213,12 @@ static int rows_layer(rows_run *r, const char **message) {
 
 /* The worklist summary of the batch (src/backend/cuda/moe.c:1710-1726), built on the device from the
  * router's selection. The wide path sends every pair through the tensor-core GEMM tiles; the narrow
- * path has no admission threshold, which the reference's summary counts as narrow pairs. */
+ * path has no admission threshold, which the reference's summary counts as narrow pairs. Tail rows are the columns that
+ * the GEMM pads an expert's rows with. */
 static int rows_worklist(rows_run *r, const char **message) {
     *message = "device layer refused the expert worklist geometry";
     return yvex_b200_expert_worklist((const int32_t *)r->ws_sel, r->rows, r->g.topk, r->g.experts, r->wide && r->tensor_path ? 1ull : 0ull,
-                                     r->wide && r->tensor_path ? yvex_b200_moe_wide_tile_columns(r->g.gate_qtype) : 1ull, r->provenance, NULL,
+                                     r->wide && r->tensor_path ? (unsigned long long)YVEX_B200_MOE_TILE_STEP : 1ull, r->provenance, NULL,
                                      NULL, NULL, NULL, NULL, NULL, r->dev_obs, r->ws_kernel, r->kernel_ws, r->backend->status_word,
                                      r->backend->stream);
 }
