@@ -173,6 +173,15 @@ def test_tile_columns_are_those_of_the_grouped_gemm(lib):
     assert plain % step == 0 and affine % step == 0
 
 
+@pytest.mark.parametrize("shortcut", [True, False])
+def test_stream_handle_with_and_without_the_private_shortcut(lib, monkeypatch, shortcut):
+    """The raw handle comes from torch's shortcut where there is one and from the stream object elsewhere."""
+    from types import SimpleNamespace as N
+    private = N(_cuda_getCurrentRawStream=lambda device: 100 + device) if shortcut else N()
+    monkeypatch.setattr(lib, "_module", N(_C=private, cuda=N(current_device=lambda: 3, current_stream=lambda: N(cuda_stream=7))))
+    assert lib._stream() == (103 if shortcut else 7)
+
+
 def test_kernels_write_out_no_mathematics():
     """Divisions, roots and exponentials are CUDA's own functions: no approximate instruction refined by hand."""
     csrc = os.path.join(ROOT, "yvex_b200", "csrc")
