@@ -127,8 +127,9 @@ __device__ __forceinline__ float comb(int a_hi, int a_lo, int b_hi, int b_lo) {
 // arrangement - columns of zeros outside a lane's group - four rows in one pass were bound by 64 MMAs per 256 x 16 weights
 // and no faster than four passes.) What a decoder takes off again (MXFP4's 16 per code, the minimum of Q4_K and Q2_K) a lane
 // takes off in its own digits, by the activation sums of its own digit pair: with the whole of it on the lower pair two large
-// sums met only at the end of a slice, and inputs with a mean lost up to a decimal digit (MXFP4 6e-6 against 1e-6). 4096 x 4096, eight rows, a pass per row against this: Q8_0 30 / 17 us, Q4_K 27 / 17,
-// Q2_K 32 / 18, MXFP4 30 / 25; IQ2_XXS 65536 x 2048 148 / 66.
+// sums met only at the end of a slice, and inputs with a mean lost precision (MXFP4 4096 wide 1.8e-6 against 7.5e-7 alone).
+// Eight rows, a pass per row against this, us: 4096 x 4096 IQ2_XXS 24 / 17, Q2_K 29 / 18.5, Q4_K 22 / 18.5, Q8_0 28 / 18, MXFP4 27 / 25;
+// 65536 x 2048 IQ2_XXS 145 / 66, Q2_K 126 / 69, Q4_K 140 / 75, Q8_0 313 / 146, MXFP4 170 / 78.
 struct DenseB { uint32_t at, pair, sums, sums_pair; };      // planes and digit-pair sums of this lane's input (of pair 0), to the next pair
 
 template <int kIn> __device__ __forceinline__ void mma_dense(const uint32_t (&a)[4], const DenseB &b, int j, int (&c)[kIn / 2][4]) {
@@ -146,6 +147,7 @@ __device__ __forceinline__ float digit_pair(int hi, int lo) { return (float)(hi 
 //   unit(...)               adds this lane's share of the dot products of rows g and g + 8 with the
 //                           activation over one unit to acc[0] / acc[1] (in units of 2^-27 * x scale);
 //                           bad bit 0 / 1: a malformed block scale in row g / g + 8
+//   dense(...)              the same for kIn input rows that share the decode: acc[p] holds the lane's digit pair of input 2 p + (t >> 1)
 struct StreamIq2 {
     static constexpr unsigned kQtype = Q_IQ2_XXS;
     static constexpr int kBlockBytes = 66, kBlockK = 256;
@@ -155,6 +157,7 @@ struct StreamIq2 {
     static constexpr bool kParity = false;               // unit<1> for odd units of a row, unit<0> for even ones
     static constexpr int kRowPad = 0;                    // bytes between the rows of a stage (0: the tile arrives as one copy)
 
+    static constexpr uint32_t kPos = 8u | (25u << 8) | (43u << 16), kNeg = 0xf8u | (0xe7u << 8) | (0xd5u << 16);      // magnitudes by digit, and their negatives
     __device__ __forceinline__ static void group(uint32_t a, uint32_t &grids, uint32_t &ss) {
         // a group starts on a 2-byte boundary: three aligned words, funnel-shifted when it sits mid-word
         const uint32_t sh = (a & 2u) * 8u, w = a & ~3u;
@@ -164,7 +167,6 @@ struct StreamIq2 {
     }
     // One subgroup of 8 weights -> two registers of signed bytes.
     template <int J> __device__ __forceinline__ static void sub(uint32_t grids, uint32_t ss, const Lane &l, uint32_t &lo, uint32_t &hi) {
-        constexpr uint32_t kPos = 8u | (25u << 8) | (43u << 16), kNeg = 0xf8u | (0xe7u << 8) | (0xd5u << 16);
         const uint32_t na = prmt(grids, l.nib_base, 0x7604u | ((uint32_t)J << 4));
         const uint32_t sa = prmt(shr_mul<7 * J>(ss), l.sgn_base, 0x7604u);
         uint32_t nib, sgn;
@@ -210,12 +212,11 @@ struct StreamIq2 {
         acc[1] = fmaf(blk1, 0.125f * f1, acc[1]);
     }
     __device__ __forceinline__ static void sub_of(uint32_t grids, uint32_t ss, const Lane &l, uint32_t &lo, uint32_t &hi) {
-        constexpr uint32_t kPos = 8u | (25u << 8) | (43u << 16), kNeg = 0xf8u | (0xe7u << 8) | (0xd5u << 16);
         const uint32_t sel = lds32(prmt(grids, l.nib_base, 0x7604u | ((uint32_t)l.t << 4))) | lds32(prmt(ss >> (7 * l.t), l.sgn_base, 0x7604u));
         lo = prmt(kPos, kNeg, sel);
         hi = prmt(kPos, kNeg, sel >> 16);
     }
-    template <int kIn, int> __device__ __forceinline__ static void dense(uint32_t row0, uint32_t row1, const DenseB &b, const Lane &l, float (&acc)[kIn / 2][2], int &bad) {
+    template <int kIn> __device__ __forceinline__ static void dense(uint32_t row0, uint32_t row1, const DenseB &b, const Lane &l, float (&acc)[kIn / 2][2], int &bad) {
         float blk[2][kIn / 2][2] = {};                                          // the two halves of the superblock, as in unit()
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -304,7 +305,7 @@ struct StreamQ4k {
         acc[0] += fmaf(d0, blk0, -n0 * min0);
         acc[1] += fmaf(d1, blk1, -n1 * min1);
     }
-    template <int kIn, int> __device__ __forceinline__ static void dense(uint32_t row0, uint32_t row1, const DenseB &b, const Lane &l, float (&acc)[kIn / 2][2], int &bad) {
+    template <int kIn> __device__ __forceinline__ static void dense(uint32_t row0, uint32_t row1, const DenseB &b, const Lane &l, float (&acc)[kIn / 2][2], int &bad) {
         float blk[2][kIn / 2][2] = {}, mn[2][kIn / 2][2] = {};
         const uint4 head0 = lds128(row0), head1 = lds128(row1);
 #pragma unroll
@@ -394,7 +395,7 @@ struct StreamQ2k {
         acc[0] += fmaf(d0, blk0, -n0 * min0);
         acc[1] += fmaf(d1, blk1, -n1 * min1);
     }
-    template <int kIn, int> __device__ __forceinline__ static void dense(uint32_t row0, uint32_t row1, const DenseB &b, const Lane &l, float (&acc)[kIn / 2][2], int &bad) {
+    template <int kIn> __device__ __forceinline__ static void dense(uint32_t row0, uint32_t row1, const DenseB &b, const Lane &l, float (&acc)[kIn / 2][2], int &bad) {
         float blk[2][kIn / 2][2] = {}, mn[2][kIn / 2][2] = {};
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -484,7 +485,7 @@ struct StreamQ80 {
         d = f16_bits_to_float((uint16_t)lds16(block));
         bad |= scale_bad(d) ? flag : 0;
     }
-    template <int kIn, int> __device__ __forceinline__ static void dense(uint32_t row0, uint32_t row1, const DenseB &b, const Lane &l, float (&acc)[kIn / 2][2], int &bad) {
+    template <int kIn> __device__ __forceinline__ static void dense(uint32_t row0, uint32_t row1, const DenseB &b, const Lane &l, float (&acc)[kIn / 2][2], int &bad) {
         float odd[kIn / 2][2] = {};                                             // a second chain, for every other block
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -593,7 +594,7 @@ struct StreamMxfp4 {
         bad |= e == 255u ? flag : 0;
         scale = __uint_as_float(e ? e << 23 : 0x00400000u) * 0.5f;
     }
-    template <int kIn, int> __device__ __forceinline__ static void dense(uint32_t row0, uint32_t row1, const DenseB &b, const Lane &l, float (&acc)[kIn / 2][2], int &bad) {
+    template <int kIn> __device__ __forceinline__ static void dense(uint32_t row0, uint32_t row1, const DenseB &b, const Lane &l, float (&acc)[kIn / 2][2], int &bad) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             uint32_t a[4];
@@ -1040,7 +1041,7 @@ __global__ void __launch_bounds__(32 * (kMaxConsumers + 1), 1) gemv_stream_kerne
                                 const uint32_t per_pair = Dec::kSumGroup ? (uint32_t)(p.K / (Dec::kSumGroup ? Dec::kSumGroup : 1) + kSumPad) * 4u : 0u;
                                 const DenseB db{ctl.planes + n * (uint32_t)plane + k0 + 8u * (uint32_t)l.t, 8u * (uint32_t)plane,
                                                 sums + (uint32_t)(u * kSumsPerUnit * 4) + (uint32_t)l.t * per_pair, 4u * per_pair};
-                                Dec::template dense<kIn, 0>(r0, r0 + second, db, l, acc[gi], bad[gi]);
+                                Dec::template dense<kIn>(r0, r0 + second, db, l, acc[gi], bad[gi]);
                             }
                         }
                     };
