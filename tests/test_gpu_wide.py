@@ -350,3 +350,89 @@ def test_grouped_gemm_tile_edges(L, gate, down, hidden, inter):
         rows = (ids == e).nonzero()[:, 0]
         if rows.numel():
             assert rel_l2(y[rows].float().cpu().numpy(), want[rows].cpu().numpy()) <= 1e-3, (e, rows.numel())
+
+
+@pytest.mark.parametrize("hidden,inter", [(6400, 512), (8192, 256)])
+def test_decode_layer_with_long_q8_0_rows(L, hidden, inter):
+    """Q8_0 rows of more than about 6 K weights go through the decode layer's gate and up launch in groups of eight (rows of down
+    are at most 4096): against 64 bits over the decoded weights with the layer's bf16 roundings."""
+    import torch
+    from yvex_b200.workloads import device_blocks
+    E, k, T = 3, 2, 5
+    spec = synth.MoELayerSpec(hidden, E, k, inter, gate_qtype=synth.Q8_0, down_qtype=synth.Q8_0)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(hidden)
+    shapes = dict(gate=(inter, hidden), up=(inter, hidden), down=(hidden, inter))
+    t = {n: device_blocks(torch, synth.Q8_0, E * r, w, gen, "cuda") for n, (r, w) in shapes.items()}
+    t.update({"shared_" + n: device_blocks(torch, synth.Q8_0, r, w, gen, "cuda") for n, (r, w) in shapes.items()})
+    x, logits, st = torch.randn((T, hidden), device="cuda", generator=gen), torch.randn((T, E), device="cuda", generator=gen), L.Status()
+    out, sel, wts = L.moe_layer(L.geometry_of(spec), L.weights_of(t), x, st, logits=logits)
+    assert st.read() == 0
+    rows = x.to(torch.bfloat16).double()
+
+    def expert(e, row, weight):
+        part = lambda n: L.dequant_rows(synth.Q8_0, (t["shared_" + n] if e < 0 else t[n].reshape(E, -1)[e]).contiguous(), *shapes[n], st).double()  # noqa: E731
+        g, u = part("gate") @ row, part("up") @ row
+        g, u = g.clamp(max=spec.limit), u.clamp(-spec.limit, spec.limit)
+        mid = (g * torch.sigmoid(g) * u * weight).to(torch.bfloat16).double()
+        return (part("down") @ mid).to(torch.bfloat16).float()
+
+    for r in range(T):
+        routed = torch.zeros(hidden, device="cuda")
+        for p in range(k):
+            routed += expert(int(sel[r, p]), rows[r], float(wts[r, p]))
+        want = (routed + expert(-1, rows[r], 1.0)).to(torch.bfloat16).float()
+        assert rel_l2(out[r].cpu().numpy(), want.cpu().numpy()) <= 1e-3
+
+
+def test_calls_launched_programmatically_replay_from_a_graph(L):
+    """The wide layer, attention and a matvec of several rows captured together: a replay on other inputs in the same buffers gives
+    what the calls give, bit for bit (captured programmatic launches keep their order)."""
+    import torch
+    from yvex_b200.workloads import device_blocks
+    H, I, E, k, T = 512, 256, 8, 2, 300
+    spec = synth.MoELayerSpec(H, E, k, I, down_qtype=synth.Q2_K)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(5)
+    q = {n: spec.gate_qtype if n != "down" else spec.down_qtype for n in ("gate", "up", "down")}
+    shapes = dict(gate=(I, H), up=(I, H), down=(H, I))
+    t = {n: device_blocks(torch, q[n], E * r, w, gen, "cuda") for n, (r, w) in shapes.items()}
+    t.update({"shared_" + n: device_blocks(torch, q[n], r, w, gen, "cuda") for n, (r, w) in shapes.items()})
+    t["router"] = 0.02 * torch.randn((E, H), device="cuda", generator=gen)
+    geometry, weights, st = L.geometry_of(spec), L.weights_of(t), L.Status()
+    x, out = torch.empty((T, H), device="cuda"), torch.empty((T, H), device="cuda")
+    sel, wts = torch.empty((T, k), dtype=torch.int32, device="cuda"), torch.empty((T, k), device="cuda")
+    ws = torch.empty(L.moe_workspace_bytes(geometry, T, True), dtype=torch.uint8, device="cuda")
+    qa, key, val = (torch.empty(s, dtype=torch.bfloat16, device="cuda") for s in ((2, 8, 128), (2, 2, 700, 128), (2, 2, 700, 128)))
+    aws = torch.empty(int(L.lib.yvex_b200_attention_workspace_bytes(2, 8, 2, 128, 700)), dtype=torch.uint8, device="cuda")
+    att = torch.empty((2, 8, 128), device="cuda")
+    head = device_blocks(torch, synth.Q4_K, 32768, H, gen, "cuda")
+    y = torch.empty((8, 32768), device="cuda")
+
+    def fill():
+        x.normal_(generator=gen)
+        for v in (qa, key, val):
+            v.normal_(generator=gen)
+
+    def calls():
+        L.moe_layer(geometry, weights, x, st, wide=True, workspace=ws, out=out, selected=sel, wts=wts)
+        L.attention_gqa_decode(qa, key, val, 650, 128 ** -0.5, st, workspace=aws, out=att)
+        L.gemv(synth.Q4_K, head, 32768, H, out[:8], st, out=y)
+        return [v.clone() for v in (out, sel, wts, att, y)]
+
+    fill()
+    calls()                                             # attributes of the kernels are set by their first launch
+    stream = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        calls()
+    for _ in range(2):
+        fill()
+        want = calls()
+        for v in (out, sel, wts, att, y):
+            v.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert st.read() == 0
+        assert all(torch.equal(a, b) for a, b in zip(want, (out, sel, wts, att, y)))
