@@ -36,9 +36,9 @@ UNIT = "tokens/s"
 
 # DRAM bytes (read + write) per launch of the dominant kernel, from the ncu captures summarised under
 # profiles/ (dram__bytes_read.sum + dram__bytes_write.sum, one capture per workload).
-TRAFFIC = {"c1": 4389376, "c2": 22777600, "c4": 2160352104,
-           "c3_gate_up_gemm": 361532672, "c3_down_gemm": 367173120,
-           "c5_gate_up_gemm": 10006566912, "c5_down_gemm": 5925237760}
+TRAFFIC = {"c1": 4471552, "c2": 22857728, "c4": 2160996096,
+           "c3_gate_up_gemm": 361430016, "c3_down_gemm": 362665216,
+           "c5_gate_up_gemm": 4683632128, "c5_down_gemm": 4917250304}
 
 
 def measured_peaks():

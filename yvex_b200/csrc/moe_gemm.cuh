@@ -114,14 +114,16 @@ struct RingAt {
 };
 
 // ---- per-qtype decoders -----------------------------------------------------------------------------
-// A decoder sees one superblock of one weight row as 32-bit words in shared memory, starting at the
-// 4-byte aligned address at or below the block (`mis` = bytes skipped, 0 or 2). kBoxBytes is the
-// width of the TMA box that fetches it: the block plus the most its start can lie above a 16-byte
-// boundary (block sizes are multiples of 2, 4 or 16 bytes), rounded up to 16.
-//   kParts     threads per row: each decodes 64 / kParts weights of a 64-K chunk
-//   store      weights k = 64*c + (64/kParts)*part .. -> 16-byte fp16 chunks of the A tile row
+// A decoder sees one superblock of one weight row in its slot of a raw stage. kBoxBytes is the pitch of the slots and the
+// width of the TMA box that fetches one: the block plus the most its start can lie above a 16-byte boundary
+// (block sizes are multiples of 2, 4 or 16 bytes), rounded up to 16 and, for Q2_K, to a pitch without bank conflicts.
+// Two threads share a row: thread h decodes weights 64 c + 32 h .. + 31 of 64-K chunk c.
+//   open       the block that starts `off` bytes into its slot; what of it is wanted in registers
+//   fetch      the words, table entries and integer scale of half h of chunk c (read before the wait for the chunk's stage)
+//   convert    sixteen of its weights (q = 0, 1) as eight words of two fp16
 //   scales     {d, dmin} of the block, and whether they are acceptable
 //   mins       this thread's share of the A' row (affine qtypes)
+//   kTableBytes, kMinSlots   shared-memory tables the decoder reads; K slots of the min term's MMA (0: none)
 // prmt.b32 with a run-time selector. (__byte_perm masks the selector with 0x7777 first; the decoders'
 // selectors never have bit 3 of a nibble set, and the instruction reads only the low 16 bits.)
 __device__ __forceinline__ uint32_t prmt_raw(uint32_t a, uint32_t b, uint32_t sel) {
@@ -664,10 +666,10 @@ moe_grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, GemmParams p) {
                 // blocks (intermediates x columns) with shuffles: lane (a, r, parity) ends up with
                 // intermediates 4a..4a+3 of column 8b + 2r + parity, multiplies by that column's route
                 // weight and stores them as one 8-byte vector.
-                // Shuffles share the shared-memory pipe with the producers' table lookups and tile stores,
-                // which keep it busy, so a shuffle takes long to come back. The tile end is therefore
-                // written in ROUNDS of independent shuffles (all swaps; all first transpose steps; all
-                // second steps) rather than block by block with three dependent shuffles each.
+                // A shuffle takes tens of cycles to come back (its pipe also serves the producers' reads), and
+                // nothing of a tile end hides behind the two accumulators. It is therefore written in ROUNDS of
+                // independent shuffles (all swaps; all first transpose steps; all second steps) rather than block
+                // by block with three dependent shuffles each.
                 const bool odd = lane & 1, o2 = lane & 2, o4 = lane & 4;
                 const int rr = (lane >> 1) & 3;
                 const uint64_t m0 = (uint64_t)mt * kRowsPerMat + 16 * quarter + 4 * (lane >> 3);
@@ -720,7 +722,7 @@ moe_grouped_gemm_kernel(const __grid_constant__ GemmMaps maps, GemmParams p) {
                 }
                 if (bad) raise(p.status, YVEX_B200_STATUS_NUMERIC);
             } else {
-                // store: out[(row0 + n)][mt*128 + row]. A thread holds 64 token columns of ONE weight row, so a
+                // store: out[(row0 + n)][mt*128 + row]. A thread holds 64 (affine qtypes: 32) token columns of ONE weight row, so a
                 // direct store is one instruction per column and 2 bytes per lane. Instead every aligned
                 // group of four lanes transposes 4 x 4 blocks with shuffles: lane 4a+j ends up with weight
                 // rows 4a..4a+3 of token column 4b+j and stores them as one 8-byte vector (a quarter of

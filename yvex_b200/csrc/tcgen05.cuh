@@ -15,8 +15,8 @@ constexpr uint64_t kWaitLimitNs = 2000000000ull;
 constexpr uint32_t kSpinLimit = 1u << 30;
 // Optional suspend-time hint of a try_wait (how long one poll may keep the thread suspended before it
 // reports "not yet"). A streaming kernel whose consumers wait on copies for microseconds gives it so that
-// its waiting warps leave the issue slots alone; the grouped GEMM, whose two-stage rings turn every
-// cycle of wake-up latency into pipeline time, polls without it (measured: 3 % faster).
+// its waiting warps leave the issue slots alone; the grouped GEMM, whose short rings (two A stages
+// for IQ2_XXS, four for the affine types) turn wake-up latency into pipeline time, polls without it (measured: 3 % faster).
 constexpr uint32_t kTryWaitHintNs = 2000u;
 
 __device__ __forceinline__ uint64_t global_ns() {
