@@ -44,7 +44,8 @@ def test_only_consecutive_rows_of_one_matrix_share_a_decode(ask, name):
 
 @pytest.mark.parametrize("name", BLOCK)
 def test_small_matrices_take_a_pass_per_row(ask, name):
-    """Two rows of a matrix that one round of tiles covers, and any few rows of a small one, are faster alone; a matrix of many
-    rounds shares its decode whatever the count from four rows on (rows of up to 4096 weights: more may not fit)."""
-    assert set(ask([(BLOCK[name], rows, width, n, 0, 0, 0, 0) for rows in (1, 17, 256, 512) for width in (512, 1024, 2048, 4096) for n in (2, 3, 4, 5)])) == {1}
+    """A few rows of a small matrix are faster alone (MXFP4, whose decode is dear: at widths whose shared form meets bank conflicts);
+    a matrix of many rounds shares its decode whatever the count from four rows on (rows of up to 4096 weights: more may not fit)."""
+    widths = (512, 4096) if name == "MXFP4" else (512, 1024, 2048, 4096)
+    assert set(ask([(BLOCK[name], rows, width, n, 0, 0, 0, 0) for rows in (1, 17, 256, 512) for width in widths for n in (2, 3, 4, 5)])) == {1}
     assert set(ask([(BLOCK[name], 65536, width, n, 0, 0, 0, 0) for width in (1024, 2048, 4096) for n in (4, 8, 12, 16)])) == {4}

@@ -1189,7 +1189,7 @@ inline uint64_t stream_rounds(const StreamShape &sh, uint64_t rows, uint64_t mat
 // up to four that share each tile's decode, where four rows' planes leave room for a ring. Rows named by a table (x_rows) are one
 // to a matrix: a pass takes consecutive ones. Sharing costs more per group and unit and prepares four rows' digits with a
 // quarter of the warps each, so it pays when the busiest warp's work falls by enough: one row's rounds >= cost x shared rounds +
-// fixed + 2 x width / 4096, with cost and fixed fitted per qtype to 2 .. 16 rows of twenty matrix sizes (us, a pass per row / shared):
+// fixed + wide x width / 4096, the three fitted per qtype to 2 .. 16 rows of twenty matrix sizes (us, a pass per row / shared):
 //   4096 x 4096, 2 rows: IQ2_XXS 11 / 12, Q4_K 10 / 12, MXFP4 11 / 16.5     8 rows: IQ2_XXS 24 / 17, Q4_K 22 / 19, MXFP4 27 / 25
 //   512 x 2048, 8 rows: Q4_K 6.0 / 8.6, Q8_0 7.1 / 10.6                       16384 x 4096, 8 rows: IQ2_XXS 73 / 43, Q4_K 79 / 47, MXFP4 88 / 65
 // Rows of a multiple of 128 bytes put the eight rows of an MXFP4 fragment on the same banks; one or two slices are few warps.
@@ -1199,10 +1199,16 @@ inline int pass_inputs(unsigned q, uint64_t rows, uint64_t width, uint64_t row_b
     StreamShape several;
     if (count < 2 || matrix_stride || matrix_ptrs || x_rows || act || !stream_shape(q, width, row_bytes, several, kMaxInputs) || several.consumers < kMaxInputs)
         return 1;
-    unsigned cost10 = q == Q_Q8_0 ? 16 : q == Q_IQ2_XXS ? 17 : q == Q_Q2_K ? 20 : q == Q_Q4_K ? 24 : row_bytes % 128 == 0 ? 26 : 17;
-    if (several.slices <= 2) cost10 = 32;
+    struct Price { int cost, fixed, wide; };                // tenths
+    const Price price = several.slices <= 2 ? Price{q == Q_IQ2_XXS ? 17 : q == Q_Q8_0 ? 26 : 32, 5, 20}
+                        : q == Q_IQ2_XXS    ? Price{15, 5, 20}
+                        : q == Q_Q4_K       ? Price{22, -5, 30}
+                        : q == Q_Q8_0       ? Price{17, 10, 5}
+                        : q == Q_Q2_K       ? Price{20, 20, 20}
+                        : row_bytes % 128   ? Price{14, -10, 30}
+                                            : Price{28, 25, 0};
     const uint64_t one = stream_rounds(sh, rows, count), shared = stream_rounds(several, rows, (count + kMaxInputs - 1) / kMaxInputs);
-    if (10 * one < cost10 * shared + (q == Q_Q2_K ? 20 : 5) + 20 * width / 4096) return 1;
+    if (10 * (int64_t)one < price.cost * (int64_t)shared + price.fixed + price.wide * (int64_t)width / 4096) return 1;
     sh = several;
     return kMaxInputs;
 }
