@@ -38,7 +38,7 @@ UNIT = "tokens/s"
 # profiles/ (dram__bytes_read.sum + dram__bytes_write.sum, one capture per workload).
 TRAFFIC = {"c1": 4471552, "c2": 22857728, "c4": 2160996096,
            "c3_gate_up_gemm": 361430016, "c3_down_gemm": 362665216,
-           "c5_gate_up_gemm": 4683632128, "c5_down_gemm": 4917250304}
+           "c5_gate_up_gemm": 4667365376, "c5_down_gemm": 4887192320}
 
 
 def measured_peaks():
