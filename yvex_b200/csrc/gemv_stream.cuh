@@ -1190,8 +1190,8 @@ inline uint64_t stream_rounds(const StreamShape &sh, uint64_t rows, uint64_t mat
 // to a matrix: a pass takes consecutive ones. Sharing costs more per group and unit and prepares four rows' digits with a
 // quarter of the warps each, so it pays when the busiest warp's work falls by enough: one row's rounds >= cost x shared rounds +
 // fixed + wide x width / 4096, the three fitted per qtype to 2 .. 16 rows of twenty matrix sizes (us, a pass per row / shared):
-//   4096 x 4096, 2 rows: IQ2_XXS 11 / 12, Q4_K 10 / 12, MXFP4 11 / 16.5     8 rows: IQ2_XXS 24 / 17, Q4_K 22 / 19, MXFP4 27 / 25
-//   512 x 2048, 8 rows: Q4_K 6.0 / 8.6, Q8_0 7.1 / 10.6                       16384 x 4096, 8 rows: IQ2_XXS 73 / 43, Q4_K 79 / 47, MXFP4 88 / 65
+//   4096 x 4096, 2 rows: IQ2_XXS 10.5 / 11.5, Q4_K 10.2 / 12.2, MXFP4 11.6 / 16.6     8 rows: IQ2_XXS 24 / 17, Q4_K 22 / 18.5, MXFP4 27 / 25
+//   512 x 2048, 8 rows: Q4_K 5.9 / 8.2, Q8_0 7.3 / 10.7                              16384 x 4096, 8 rows: IQ2_XXS 74 / 43, Q4_K 78 / 47, MXFP4 90 / 66
 // Rows of a multiple of 128 bytes put the eight rows of an MXFP4 fragment on the same banks; one or two slices are few warps.
 inline int pass_inputs(unsigned q, uint64_t rows, uint64_t width, uint64_t row_bytes, uint64_t count, uint64_t matrix_stride,
                        const uint8_t *const *matrix_ptrs, const uint32_t *x_rows, const StreamActivation *act, StreamShape &sh) {
